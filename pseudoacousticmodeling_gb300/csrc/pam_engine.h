@@ -42,7 +42,7 @@ struct pam_engine {
     int check_numeric();                 // PAM_E_NUMERIC (with a message) if that bit is set
     int seis_own_shots = 0, seis_own_nrec = 0;
     std::vector<float> wavelet;
-    float* d_wavelet = nullptr;          // [nt], the persistent path's source samples
+    float* d_wavelet = nullptr;          // [nt], the persistent tiles' source samples
 
     // step-level interface
     int step_shots = 0, next_step = 0;
@@ -138,13 +138,29 @@ struct pam_engine {
     bool autotune = true;
     int seg_height(int nshots) const;
     int tune_segments(int nshots, cudaStream_t s);
-    // The persistent path of small Cerjan runs (step_persistent_kernel): the
-    // segment height to use for this batch, 0 for the graph path
-    int persist_capacity = -1;
     // set by pam_adjoint_gradient: the exact job's data are the adjoint source
     bool adjoint_source_given = false;
-    int persistent_height(int nshots);
-    int launch_persistent(int nshots, int H, float* d_seis, int k0, int k1, cudaStream_t s);
+    // Small runs as persistent tiles (pam_tile.cu): the plan of a batch size, or
+    // nullptr for the one-step launches; tile_begin makes the buffers and lists
+    // of a plan ready, tile_forward runs steps k0 .. k1-1 from the state that
+    // the run's earlier launches left (before the first: d_u[0], d_u[1])
+    struct TilePlan {
+        bool usable = false;
+        int T = 0, TZ = 0, TX = 0, nty = 0, ntx = 0, R = 0;
+        int group = 0;                   // shots per launch
+    };
+    std::map<int, TilePlan> tile_plans;
+    const TilePlan* tile_plan(int nshots);
+    int tile_begin(const TilePlan& p, cudaStream_t s);
+    int tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s);
+    float* d_tile[2] = {nullptr, nullptr};   // [B][stride] the second published state of the tiles
+    unsigned* d_tile_bar = nullptr;
+    int* d_tile_beg = nullptr;           // receivers by tile (tile_begin)
+    int2* d_tile_ent = nullptr;
+    std::vector<int> h_rz, h_rx;
+    bool tile_lists_stale = true;
+    int tile_lists_TZ = 0, tile_lists_TX = 0;
+    int tile_set = 0;                    // which published state is the current one
     // The same for the fused adjoint + gradient kernel of the exact gradient
     // (fewer resident warps per SM than the stepping kernel, so its own
     // height); the stepping kernel's until tuned.

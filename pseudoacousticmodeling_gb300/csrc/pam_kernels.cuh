@@ -28,7 +28,6 @@
 // the other shots.  The arithmetic runs on packed two-wide FP32 instructions
 // (FFMA2 / FADD2 / FMUL2).
 #pragma once
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -198,6 +197,47 @@ __device__ __forceinline__ float sd_ratio(float num, float den) {
 #endif
 }
 
+// The update of a cell pair from its derivatives: 2 U(t) - U(t-1) (base) plus
+// kappa times the operator, in the reference's written order.  k is kappa,
+// e2 = 1 + 2 eps, m1 = -2 (eps - delta), m2 = 2 (1 + delta), ca / sa the cosine
+// and sine of the tilt (VTI and TTI operands are unused otherwise).
+template <int APPROX>
+__device__ __forceinline__ float2 update_pair(float2 k, float2 base, float2 pxx, float2 pzz, float2 px, float2 pz,
+                                              float2 pxz, float2 e2, float2 m1, float2 m2, float2 ca, float2 sa) {
+    if (APPROX == kAcoustic) return pfma2(k, padd2(pxx, pzz), base);
+    float2 sx_ = px, sz_ = pz;
+    if (APPROX == kTTI) {
+        sx_ = pfma2(px, ca, neg2(pmul2(pz, sa)));
+        sz_ = pfma2(px, sa, pmul2(pz, ca));
+    }
+    // Sd of cpp/Modeling.cu:605-611 (VTI) and :719-727 (TTI), switched
+    // on where |den| > 1e-12: the reference's products in its
+    // written order, its sums contracted as the compiler does
+    const float2 px2 = pmul2(sx_, sx_), pz2 = pmul2(sz_, sz_);
+    const float2 num = pmul2(pmul2(m1, px2), pz2);
+    float2 den;
+    if (APPROX == kVTI) {
+        // (1 + 2 eps) (px px px px) + (pz pz pz pz) + 2 (1 + delta) (px px) (pz pz)
+        const float2 p4x = pmul2(pmul2(px2, sx_), sx_), p4z = pmul2(pmul2(pz2, sz_), sz_);
+        den = pfma2(pmul2(m2, px2), pz2, pfma2(e2, p4x, p4z));
+    } else {
+        // (1 + 2 eps) xr2 xr2 + zr2 zr2 + 2 (1 + delta) xr2 zr2
+        den = pfma2(pmul2(m2, px2), pz2, pfma2(pmul2(e2, px2), px2, pmul2(pz2, pz2)));
+    }
+    const float2 sd = make_float2(sd_ratio(num.x, den.x), sd_ratio(num.y, den.y));
+    if (APPROX == kVTI) {
+        const float2 ax = pmul2(k, padd2(e2, sd));
+        const float2 az = pmul2(k, padd2(make_float2(1.f, 1.f), sd));
+        return pfma2(az, pzz, pfma2(ax, pxx, base));   // the pxx term first, as written
+    }
+    const float2 c2 = pmul2(ca, ca), s2 = pmul2(sa, sa);
+    const float2 ax = pmul2(k, padd2(pfma2(e2, c2, s2), sd));
+    const float2 az = pmul2(k, padd2(pfma2(e2, s2, c2), sd));
+    // -2 eps kappa sin(2 theta) pxz = (1 - e2) kappa 2 s c pxz
+    const float2 hs = pmul2(fsub2(make_float2(1.f, 1.f), e2), pmul2(k, pmul2(padd2(sa, sa), ca)));
+    return pfma2(hs, pxz, pfma2(az, pzz, pfma2(ax, pxx, base)));   // in written order
+}
+
 template <int APPROX>
 __host__ __device__ constexpr int step_min_blocks() { return APPROX == kTTI ? 3 : 4; }
 
@@ -210,10 +250,9 @@ __host__ __device__ constexpr int interior_unroll() { return APPROX == kAcoustic
 template <int V>
 struct IntTag { static constexpr int value = V; };
 
-// One time step of this thread's warp (its shot, tile and segment): the
-// body of step_kernel, also run once per step by step_persistent_kernel.
+// One time step of each warp's shot, tile and segment.
 template <int APPROX, int BC>
-__device__ __forceinline__ void step_body(const StepArgs& a)
+__global__ void __launch_bounds__(128, step_min_blocks<APPROX>()) step_kernel(const StepArgs a)
 {
     constexpr int NA = ring_arrays<APPROX>();
     constexpr bool XH = fetched_halo<APPROX>();
@@ -457,51 +496,13 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
                 const float2 czq = make_float2(cz, cz);
                 if (damp) p = pmul2(pmul2(p, cxq), czq);   // damping of U(t-1) deferred to this read
                 const float2 base = fsub2(padd2(uc, uc), p);   // 2 U(t) - U(t-1)
-                float2 o;
-                if (APPROX == kAcoustic) {
-                    o = pfma2(k, padd2(pxx2[q], pzz2[q]), base);
-                } else {
-                    const float2 px = px2v[q], pz = pz2v[q];
-                    const float2 pxxe = pxx2[q], pzze = pzz2[q];
-                    const float2 e2 = q == 0 ? lo2(e4) : hi2(e4);   // 1 + 2 eps
-                    const float2 m1 = q == 0 ? lo2(n4) : hi2(n4);   // -2 (eps - delta)
-                    const float2 m2 = q == 0 ? lo2(b4) : hi2(b4);   // 2 (1 + delta)
-                    float2 sx_ = px, sz_ = pz, ca, sa;
-                    if (APPROX == kTTI) {
-                        ca = q == 0 ? lo2(c4) : hi2(c4);
-                        sa = q == 0 ? lo2(s4) : hi2(s4);
-                        sx_ = pfma2(px, ca, neg2(pmul2(pz, sa)));
-                        sz_ = pfma2(px, sa, pmul2(pz, ca));
-                    }
-                    // Sd of cpp/Modeling.cu:605-611 (VTI) and :719-727 (TTI), switched
-                    // on where |den| > 1e-12: the reference's products in its
-                    // written order, its sums contracted as the compiler does
-                    const float2 px2 = pmul2(sx_, sx_), pz2 = pmul2(sz_, sz_);
-                    const float2 num = pmul2(pmul2(m1, px2), pz2);
-                    float2 den;
-                    if (APPROX == kVTI) {
-                        // (1 + 2 eps) (px px px px) + (pz pz pz pz) + 2 (1 + delta) (px px) (pz pz)
-                        const float2 p4x = pmul2(pmul2(px2, sx_), sx_), p4z = pmul2(pmul2(pz2, sz_), sz_);
-                        den = pfma2(pmul2(m2, px2), pz2, pfma2(e2, p4x, p4z));
-                    } else {
-                        // (1 + 2 eps) xr2 xr2 + zr2 zr2 + 2 (1 + delta) xr2 zr2
-                        den = pfma2(pmul2(m2, px2), pz2, pfma2(pmul2(e2, px2), px2, pmul2(pz2, pz2)));
-                    }
-                    const float2 sd = make_float2(sd_ratio(num.x, den.x), sd_ratio(num.y, den.y));
-                    if (APPROX == kVTI) {
-                        const float2 ax = pmul2(k, padd2(e2, sd));
-                        const float2 az = pmul2(k, padd2(make_float2(1.f, 1.f), sd));
-                        o = pfma2(az, pzze, pfma2(ax, pxxe, base));   // the pxx term first, as written
-                    } else {
-                        const float2 c2 = pmul2(ca, ca), s2 = pmul2(sa, sa);
-                        const float2 ax = pmul2(k, padd2(pfma2(e2, c2, s2), sd));
-                        const float2 az = pmul2(k, padd2(pfma2(e2, s2, c2), sd));
-                        // -2 eps kappa sin(2 theta) pxz = (1 - e2) kappa 2 s c pxz
-                        const float2 hs = pmul2(fsub2(make_float2(1.f, 1.f), e2),
-                                                     pmul2(k, pmul2(padd2(sa, sa), ca)));
-                        o = pfma2(hs, pxz2[q], pfma2(az, pzze, pfma2(ax, pxxe, base)));   // in written order
-                    }
-                }
+                const float2 z2 = make_float2(0.f, 0.f);
+                float2 o = update_pair<APPROX>(k, base, pxx2[q], pzz2[q], px2v[q], pz2v[q], pxz2[q],
+                                               APPROX == kAcoustic ? z2 : q == 0 ? lo2(e4) : hi2(e4),
+                                               APPROX == kAcoustic ? z2 : q == 0 ? lo2(n4) : hi2(n4),
+                                               APPROX == kAcoustic ? z2 : q == 0 ? lo2(b4) : hi2(b4),
+                                               APPROX != kTTI ? z2 : q == 0 ? lo2(c4) : hi2(c4),
+                                               APPROX != kTTI ? z2 : q == 0 ? lo2(s4) : hi2(s4));
                 if (damp) o = pmul2(pmul2(o, cxq), czq);
                 outp[q] = o;
             }
@@ -551,12 +552,6 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     if (edge) march(IntTag<1>{}, IntTag<1>{});
     else march(IntTag<0>{}, IntTag<interior_unroll<APPROX>()>{});
     cp_async_wait<0>();
-}
-
-template <int APPROX, int BC>
-__global__ void __launch_bounds__(128, step_min_blocks<APPROX>()) step_kernel(const StepArgs a)
-{
-    step_body<APPROX, BC>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -907,8 +902,9 @@ static __global__ void __launch_bounds__(1024) cpml_z_pair_kernel(const CpmlArgs
 // Receiver recording (cpp/Modeling.cu:488-497): seis[b][t][r] = D * U(t) at
 // the receiver cell, D the Cerjan factor there (1 for CPML and the interior).
 
-__device__ __forceinline__ void record_sample(const RecordArgs& a, long long i)
+static __global__ void record_kernel(const RecordArgs a)
 {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)a.nrec * a.B) return;
     const int r = (int)(i % a.nrec);
     const int b = (int)(i / a.nrec);
@@ -926,49 +922,6 @@ __device__ __forceinline__ void record_sample(const RecordArgs& a, long long i)
     *PAM_CHK(&a.seis[((long long)b * a.nt_data + a.it) * a.nrec + r], a.seis, (long long)a.B * a.nt_data * a.nrec * 4,
              4, 42) = v;
     if (!isfinite(v)) atomicOr(a.status, 1);   // an unstable scheme overflows the fields
-}
-
-static __global__ void record_kernel(const RecordArgs a)
-{
-    record_sample(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// The forward time loop of a small batch in one cooperative launch: steps
-// k0 .. k1-1, each the warps' step_body, the recording of U(k) by the first
-// nrec * B threads of the grid, and a grid-wide barrier (a cooperative launch
-// keeps every block resident, so each barrier is reached by all of them).
-// For runs whose steps are so short that one CUDA-graph launch per kernel
-// and step dominates (the single-shot plain case: about 3 us of a 5.7 us
-// step); larger batches keep the graph of one-step launches.
-struct PersistArgs {
-    StepArgs base;                  // cur / nxt / src_amp set per step
-    float* u[2];                    // the two field buffers: U(k) in u[k & 1]
-    const float* __restrict__ wavelet;   // [nt]
-    RecordArgs rec;                 // it set per step; seis == nullptr: no recording
-    int nt, itlag, k0, k1;
-};
-
-template <int APPROX, int BC>
-__global__ void __launch_bounds__(128, step_min_blocks<APPROX>()) step_persistent_kernel(const PersistArgs p)
-{
-    namespace cg = cooperative_groups;
-    cg::grid_group grid = cg::this_grid();
-    const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (int k = p.k0; k < p.k1; k++) {
-        StepArgs a = p.base;
-        a.cur = p.u[k & 1];
-        a.nxt = p.u[(k + 1) & 1];
-        a.prev = nullptr;
-        a.src_amp = k + 1 < p.nt ? p.wavelet[k + 1] : 0.0f;
-        if (k >= p.itlag && p.rec.seis) {
-            RecordArgs r = p.rec;
-            r.cur = a.cur;
-            r.it = k - p.itlag;
-            record_sample(r, gtid);
-        }
-        step_body<APPROX, BC>(a);
-        grid.sync();
-    }
 }
 
 // Writes the first wavelet sample at each shot's source cell (the injection

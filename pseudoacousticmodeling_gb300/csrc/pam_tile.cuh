@@ -1,0 +1,408 @@
+// Time loops of small batches as persistent tiles (sm_103a).
+//
+// A small grid's step costs far less than the latency of starting it: a graph
+// of one-step launches takes 6 us a step for one 301 x 501 shot, and one
+// cooperative launch with a grid-wide barrier after every step 2.8 us, most
+// of it the barrier and the reload of the field from L2.  Here one block per
+// SM owns a tile of one shot for the whole launch and keeps it on chip with a
+// halo 4 T cells wide.  It advances T steps between barriers, each on a region
+// 4 cells smaller on every side than the one before (the stencil's reach), so
+// that the last one ends on the tile itself; then it publishes the tile's two
+// fields, waits for the other blocks and reads the halo back from L2.  The
+// halo cells are computed by several blocks, from the same values by the same
+// operations, so the results are those of the one-step kernels bit for bit.
+//
+// A thread owns one quad of columns and R rows of the tile with its halo:
+// U(t) and U(t-1) of those cells stay in its registers, and two copies of U in
+// shared memory (one read, one written, one block barrier per step) give it
+// the four rows above and below and the quads left and right.  What a thread
+// needs for its cells - addresses, masks, damping factors, kappa - is worked
+// out once per launch: the step loop itself is bound by the latency of its
+// arithmetic and by instruction issue.
+//
+// A larger T saves barriers (about 2 us each with the exchange) and costs
+// halo cells; tile_plan() on the host weighs the two for the grid at hand.
+// Measured per step, tiles against the graph of one-step launches (and the
+// one-barrier-per-step persistent kernel): acoustic 301 x 501 1.4 against 5.7
+// (2.8) us, 501 x 1101 2.2 against 5.9; VTI 501 x 1101 3.5 against 7.1 (6.3);
+// TTI 381 x 681 3.1 against 7.3.  At 1.4 us a step the 301 x 501 tile spends
+// about 0.65 us a step in the exchange and issues 28% of the cycles.
+#pragma once
+#include "pam_kernels.cuh"
+
+namespace pam {
+
+constexpr int kTileThreads = 512;       // at most
+constexpr int kTilePitch = 32;          // quads per row of a shared copy (more than a tile with its halo has)
+constexpr int kTileMaxT = 8;
+// polls of a grid barrier before it is given up (a poll takes about half a
+// microsecond): all blocks are resident, so this is never reached
+constexpr int kTileSpin = 1 << 21;
+
+// model arrays of an approximation: kappa, 1 + 2 eps, -2 (eps - delta),
+// 2 (1 + delta), cos, sin
+template <int APPROX>
+__host__ __device__ constexpr int tile_models() { return APPROX == kAcoustic ? 1 : (APPROX == kVTI ? 4 : 6); }
+
+struct TileShape {
+    int T;              // steps between barriers
+    int TZ, TX;         // cells of a tile (TX a multiple of 4)
+    int nty, ntx;       // tiles of one shot
+    int R;              // rows per thread
+    int nrg, EXq;       // row groups and quads of a tile with its halo
+};
+
+__host__ __device__ inline int tile_threads(const TileShape& g) { return (g.nrg * g.EXq + 31) / 32 * 32; }
+// two copies of U (for TTI a third array, of its z derivative) with four guard
+// rows above and below; the models of each thread's cells (the acoustic kappa stays in registers)
+__host__ __device__ inline size_t tile_smem_bytes(const TileShape& g, int models) {
+    const int copies = models == tile_models<kTTI>() ? 3 : 2;
+    return (size_t)copies * (g.nrg * g.R + 8) * kTilePitch * 16 +
+           (models > 1 ? (size_t)models * g.R * tile_threads(g) * 16 : 0);
+}
+
+struct TileArgs {
+    StepArgs s;                          // grid, models, Cerjan factors, sources (no fields)
+    TileShape g;
+    float* ex[2][2];                     // published state [set][0: U(k), 1: U(k-1)], [B][nz][P]
+    int set0;                            // set that holds the state before step k0
+    int shot0;                           // first shot of this launch
+    const float* __restrict__ wavelet;   // [nt]
+    RecordArgs rec;                      // seis == nullptr: no recording
+    const int* __restrict__ rec_beg;     // [tiles (per shot) + 1] receivers of each tile ...
+    const int2* __restrict__ rec_ent;    // ... as (row << 16 | column, receiver)
+    int nt, itlag, k0, k1;
+    unsigned* bar;                       // barrier counter, zero at the launch
+    int* status;                         // bit 1 set when a barrier was given up
+};
+
+// Grid-wide barrier of resident blocks: each block's writes before it are
+// visible (through L2) to every block after it.  `want` = blocks x barriers so
+// far.  False when it was given up.
+__device__ __forceinline__ bool tile_barrier(unsigned* bar, unsigned want, int* status, int* flag) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        int left = kTileSpin;
+        unsigned v;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+        } while ((int)(v - want) < 0 && --left > 0);
+        *flag = left > 0;
+        if (left == 0) atomicOr(status, 2);
+    }
+    __syncthreads();
+    return *flag != 0;
+}
+
+// A quad of row z, column x (a multiple of 4) of a pitched array; zero outside
+// [0, nz) x [0, P).  Fields are read past L1, which other SMs' writes do not reach.
+__device__ __forceinline__ float4 tile_fetch(const float* src, int z, int x, int nz, int P,
+                                             [[maybe_unused]] const void* base, [[maybe_unused]] long long bytes) {
+    if (z < 0 || z >= nz || x < 0 || x >= P) return make_float4(0.f, 0.f, 0.f, 0.f);
+    return __ldcg(reinterpret_cast<const float4*>(PAM_CHK(src + (long long)z * P + x, base, bytes, 16, 100)));
+}
+
+// What a thread owns, worked out once per launch.
+template <int R>
+struct TileCells {
+    int z, x;                // first row, first column
+    int at;                  // quad index in a shared copy
+    int need;                // smallest region halo that holds one of its cells
+    unsigned valid, mine;    // rows of the update region; rows of the block's own tile
+    bool tail, damp;         // columns past the update region; any damped cell
+    float4 cx;               // damping factors (1 outside the border)
+    float cz[R];
+};
+
+template <int R>
+__device__ __forceinline__ TileCells<R> tile_cells(const StepArgs& a, const TileShape& g, int tile) {
+    const int z0 = 4 + (tile / g.ntx) * g.TZ, x0 = 4 + (tile % g.ntx) * g.TX;
+    const int z1 = min(z0 + g.TZ, a.nz - 4), x1 = min(x0 + g.TX, a.nx - 4);
+    const int rg = threadIdx.x / g.EXq, q = threadIdx.x - rg * g.EXq;
+    TileCells<R> c;
+    c.z = z0 - 4 * g.T + rg * R;
+    c.x = x0 - 4 * g.T + 4 * q;
+    c.at = (4 + min(rg, g.nrg - 1) * R) * kTilePitch + q;
+    c.need = 1 << 20;
+    c.valid = c.mine = 0;
+    auto factor = [&](int i, int len) {
+        float f = 1.0f;
+        if (a.cerjan && i >= 0 && i < a.N) f = a.cerjan[i];
+        if (a.cerjan && i >= len - a.N && i < len) f = f * a.cerjan[len - 1 - i];
+        return f;
+    };
+    const bool xin = rg < g.nrg && c.x >= 4 && c.x < a.nx - 4;
+    const int hx = max(x0 - c.x, c.x >= x1 ? c.x - x1 + 4 : 0);
+    c.damp = c.x < a.N || c.x + 4 > a.nx - a.N;
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const int z = c.z + j;
+        if (xin && z >= 4 && z < a.nz - 4) {
+            c.valid |= 1u << j;
+            c.need = min(c.need, max(max(max(z0 - z, z - z1 + 1), hx), 0));
+            if (z >= z0 && z < z1 && c.x >= x0 && c.x < x1) c.mine |= 1u << j;
+        }
+        c.cz[j] = factor(z, a.nz);
+        c.damp = c.damp || z < a.N || z >= a.nz - a.N;
+    }
+    c.damp = c.damp && a.cerjan;
+    c.cx = make_float4(factor(c.x, a.nx), factor(c.x + 1, a.nx), factor(c.x + 2, a.nx), factor(c.x + 3, a.nx));
+    c.tail = c.x + 4 > a.nx - 4;
+    return c;
+}
+
+// One step of a thread's cells: out[j] = U(k+1) from cur[j] = U(k), old[j] =
+// U(k-1) and the neighbours' U(k) in the shared copy A.  model(i, j) gives row
+// j of model array i.  For TTI every thread that holds cells of the block
+// calls it (Z passes the z derivatives on, with a barrier), and out is left
+// alone where the thread is not active.
+template <int APPROX, int R, class Model>
+__device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>& t, const float4* __restrict__ A,
+                                          float4* __restrict__ Z, bool active, const float4 (&cur)[R],
+                                          const float4 (&old)[R], Model model, float4 (&out)[R]) {
+    const float4* const col = A + t.at;
+    float4 w[R + 8];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        w[j] = col[(j - 4) * kTilePitch];
+        w[R + 4 + j] = col[(R + j) * kTilePitch];
+    }
+#pragma unroll
+    for (int j = 0; j < R; j++) w[j + 4] = cur[j];
+    // the z derivatives; for the TTI cross derivative (the x derivative of the
+    // z derivative) they go to the neighbouring quads through shared memory
+    float2 pzv[R][2];
+    if (APPROX != kAcoustic) {
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            pzv[j][0] = d1_pair_ref(lo2(w[j + 5]), lo2(w[j + 3]), lo2(w[j + 6]), lo2(w[j + 2]), lo2(w[j + 7]), lo2(w[j + 1]),
+                                    lo2(w[j + 8]), lo2(w[j]), a.inv_dz);
+            pzv[j][1] = d1_pair_ref(hi2(w[j + 5]), hi2(w[j + 3]), hi2(w[j + 6]), hi2(w[j + 2]), hi2(w[j + 7]), hi2(w[j + 1]),
+                                    hi2(w[j + 8]), hi2(w[j]), a.inv_dz);
+            if (APPROX == kTTI && t.valid)
+                Z[t.at + j * kTilePitch] = make_float4(pzv[j][0].x, pzv[j][0].y, pzv[j][1].x, pzv[j][1].y);
+        }
+    }
+    if (APPROX == kTTI) __syncthreads();
+    if (!active) return;
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const float4 c = cur[j], l = col[j * kTilePitch - 1], r = col[j * kTilePitch + 1];
+        const float4 kap = model(0, j);
+        const float2 P0 = lo2(l), P1 = hi2(l), P2 = lo2(c), P3 = hi2(c), P4 = lo2(r), P5 = hi2(r);
+        const float2 O0 = make_float2(l.y, l.z), O1 = make_float2(l.w, c.x), O2 = make_float2(c.y, c.z);
+        const float2 O3 = make_float2(c.w, r.x), O4 = make_float2(r.y, r.z);
+        float2 pxx[2], pzz[2], px[2], pz[2], pxz[2];
+        px[0] = px[1] = pz[0] = pz[1] = pxz[0] = pxz[1] = make_float2(0.f, 0.f);
+        pxx[0] = d2_pair(P2, O2, O1, P3, P1, O3, O0, P4, P0, a.inv_dx2);
+        pxx[1] = d2_pair(P3, O3, O2, P4, P2, O4, O1, P5, P1, a.inv_dx2);
+        pzz[0] = d2_pair(lo2(c), lo2(w[j + 5]), lo2(w[j + 3]), lo2(w[j + 6]), lo2(w[j + 2]), lo2(w[j + 7]), lo2(w[j + 1]),
+                         lo2(w[j + 8]), lo2(w[j]), a.inv_dz2);
+        pzz[1] = d2_pair(hi2(c), hi2(w[j + 5]), hi2(w[j + 3]), hi2(w[j + 6]), hi2(w[j + 2]), hi2(w[j + 7]), hi2(w[j + 1]),
+                         hi2(w[j + 8]), hi2(w[j]), a.inv_dz2);
+        if (APPROX != kAcoustic) {
+            px[0] = d1_pair_ref(O2, O1, P3, P1, O3, O0, P4, P0, a.inv_dx);
+            px[1] = d1_pair_ref(O3, O2, P4, P2, O4, O1, P5, P1, a.inv_dx);
+            pz[0] = pzv[j][0];
+            pz[1] = pzv[j][1];
+        }
+        if (APPROX == kTTI) {
+            const float4 zl = Z[t.at + j * kTilePitch - 1], zr = Z[t.at + j * kTilePitch + 1];
+            const float2 V0 = lo2(zl), V1 = hi2(zl), V4 = lo2(zr), V5 = hi2(zr);
+            const float2 W0 = make_float2(zl.y, zl.z), W1 = make_float2(zl.w, pz[0].x);
+            const float2 W2 = make_float2(pz[0].y, pz[1].x), W3 = make_float2(pz[1].y, zr.x);
+            const float2 W4 = make_float2(zr.y, zr.z);
+            pxz[0] = d1_pair(W2, W1, pz[1], V1, W3, W0, V4, V0, a.cx1);
+            pxz[1] = d1_pair(W3, W2, V4, pz[0], W4, W1, V5, V1, a.cx1);
+        }
+        float4 e4 = kap, n4 = kap, b4 = kap, c4 = kap, s4 = kap;
+        if (APPROX != kAcoustic) { e4 = model(1, j); n4 = model(2, j); b4 = model(3, j); }
+        if (APPROX == kTTI) { c4 = model(4, j); s4 = model(5, j); }
+        float2 o[2];
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const float2 uc = m ? hi2(c) : lo2(c), cxm = m ? hi2(t.cx) : lo2(t.cx);
+            float2 u1 = m ? hi2(old[j]) : lo2(old[j]);
+            if (t.damp) u1 = pmul2(pmul2(u1, cxm), bc2(t.cz[j]));   // damping of U(t-1) deferred to this read
+            const float2 base = fsub2(padd2(uc, uc), u1);
+            float2 v = update_pair<APPROX>(m ? hi2(kap) : lo2(kap), base, pxx[m], pzz[m], px[m], pz[m], pxz[m],
+                                           m ? hi2(e4) : lo2(e4), m ? hi2(n4) : lo2(n4), m ? hi2(b4) : lo2(b4),
+                                           m ? hi2(c4) : lo2(c4), m ? hi2(s4) : lo2(s4));
+            if (t.damp) v = pmul2(pmul2(v, cxm), bc2(t.cz[j]));
+            o[m] = v;
+        }
+        out[j] = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+    }
+    // cells off the update region stay zero
+    if (t.valid != (1u << R) - 1u)
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (!(t.valid >> j & 1u)) out[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t.tail)
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            if (t.x + 1 >= a.nx - 4) out[j].y = 0.f;
+            if (t.x + 2 >= a.nx - 4) out[j].z = 0.f;
+            if (t.x + 3 >= a.nx - 4) out[j].w = 0.f;
+        }
+}
+
+// Forward time loop, steps k0 .. k1-1, of the shots shot0 .. (one block per
+// tile of each): see the head of the file.
+template <int APPROX, int R>
+__global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const TileArgs t)
+{
+    extern __shared__ float4 tsm[];
+    __shared__ int alive;
+    const StepArgs& a = t.s;
+    const TileShape& g = t.g;
+    const int ntiles = g.nty * g.ntx;
+    const int shot = t.shot0 + blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    const TileCells<R> own = tile_cells<R>(a, g, tile);
+    const int copy = (g.nrg * R + 8) * kTilePitch;
+    float4* A = tsm;                       // U(k)
+    float4* B = tsm + copy;                // U(k+1)
+    constexpr int ncopy = APPROX == kTTI ? 3 : 2;
+    float4* const Z = tsm + 2 * copy;      // TTI: z derivative of U(k)
+    float4* const M = tsm + ncopy * copy + tid;
+    const long long so = (long long)shot * a.shot_stride;
+    [[maybe_unused]] const long long fbytes = (long long)a.B * a.shot_stride * 4;
+    [[maybe_unused]] const long long mbytes = (long long)a.nz * a.P * 4;
+
+    // the state and the models of the thread's cells
+    float4 cur[R], old[R], kap[R];
+    {
+        for (int i = tid; i < ncopy * copy; i += nthr) tsm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* const in0 = t.set0 ? t.ex[1][0] : t.ex[0][0];
+        const float* const in1 = t.set0 ? t.ex[1][1] : t.ex[0][1];
+        const float* const mod[6] = {a.kap, a.e2, a.m1, a.m2, a.cth, a.sth};
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const bool v = own.valid >> j & 1u;
+            const int z = v ? own.z + j : -1;
+            cur[j] = tile_fetch(in0 + so, z, own.x, a.nz, a.P, in0, fbytes);
+            old[j] = tile_fetch(in1 + so, z, own.x, a.nz, a.P, in1, fbytes);
+            kap[j] = tile_fetch(a.kap, z, own.x, a.nz, a.P, a.kap, mbytes);
+            if (APPROX != kAcoustic)
+#pragma unroll
+                for (int i = 0; i < tile_models<APPROX>(); i++)
+                    M[(i * R + j) * nthr] = tile_fetch(mod[i], z, own.x, a.nz, a.P, mod[i], mbytes);
+        }
+        __syncthreads();
+        if (own.valid)
+#pragma unroll
+            for (int j = 0; j < R; j++) A[own.at + j * kTilePitch] = cur[j];
+    }
+    auto model = [&](int i, int j) { return APPROX == kAcoustic ? kap[j] : M[(i * R + j) * nthr]; };
+
+    // the source, if it is one of the thread's cells
+    const int sz = *PAM_CHK(&a.src_z[shot], a.src_z, a.B * 4, 4, 101);
+    const int sx = *PAM_CHK(&a.src_x[shot], a.src_x, a.B * 4, 4, 101);
+    const int srow = sz - own.z;
+    const bool has_src = own.valid && srow >= 0 && srow < R && (own.valid >> srow & 1u) && sx >= own.x && sx < own.x + 4 &&
+                         sx < a.nx - 4;
+    // the first of the receivers that the thread records: place and damping
+    // factors, x then z, as in the one-step kernels' recording
+    const int rl = t.rec.per_shot ? shot * ntiles + tile : tile;
+    const int rb = t.rec.seis ? t.rec_beg[rl] : 0, re = t.rec.seis ? t.rec_beg[rl + 1] : 0;
+    const int ez0 = 4 + (tile / g.ntx) * g.TZ - 4 * g.T - 4, ex0 = 4 + (tile % g.ntx) * g.TX - 4 * g.T;
+    [[maybe_unused]] const long long sbytes = (long long)a.B * t.rec.nt_data * t.rec.nrec * 4;
+    float* const seis = t.rec.seis + (long long)shot * t.rec.nt_data * t.rec.nrec;
+    auto place = [&](int2 e, int& off, float& fx, float& fz) {
+        const int z = e.x >> 16, x = e.x & 0xffff;
+        off = (z - ez0) * (4 * kTilePitch) + x - ex0;
+        fx = x < a.N ? a.cerjan[x] : x >= a.nx - a.N ? a.cerjan[a.nx - 1 - x] : 1.0f;
+        fz = z < a.N ? a.cerjan[z] : z >= a.nz - a.N ? a.cerjan[a.nz - 1 - z] : 1.0f;
+    };
+    auto sample = [&](int it, int r, int off, float fx, float fz) {
+        const float v = reinterpret_cast<const float*>(A)[off] * fx * fz;
+        *PAM_CHK(&seis[(long long)it * t.rec.nrec + r], t.rec.seis, sbytes, 4, 102) = v;
+        if (!isfinite(v)) atomicOr(t.status, 1);
+    };
+    int roff = 0, rr = -1;
+    float rfx = 1.0f, rfz = 1.0f;
+    if (rb + tid < re) {
+        const int2 e = t.rec_ent[rb + tid];
+        rr = e.y;
+        place(e, roff, rfx, rfz);
+    }
+    __syncthreads();
+
+    int k = t.k0, set = t.set0;
+    unsigned want = 0;
+    float amp = k + 1 < t.nt ? t.wavelet[k + 1] : 0.0f;
+    while (k < t.k1) {
+        const int nsub = min(g.T, t.k1 - k);
+        for (int s = 0; s < nsub; s++, k++) {
+            const float next_amp = k + 2 < t.nt ? t.wavelet[k + 2] : 0.0f;
+            if (k >= t.itlag) {
+                if (rr >= 0) sample(k - t.itlag, rr, roff, rfx, rfz);
+                for (int i = rb + tid + nthr; i < re; i += nthr) {
+                    const int2 e = t.rec_ent[i];
+                    int off;
+                    float fx, fz;
+                    place(e, off, fx, fz);
+                    sample(k - t.itlag, e.y, off, fx, fz);
+                }
+            }
+            // a region of halo 4 (nsub - 1 - s) around the tile, whole threads of it
+            const bool active = own.need <= 4 * (nsub - 1 - s);
+            float4 out[R];
+            if (active || APPROX == kTTI) tile_step<APPROX, R>(a, own, A, Z, active, cur, old, model, out);
+            if (active) {
+                if (has_src)
+#pragma unroll
+                    for (int j = 0; j < R; j++)
+                        if (j == srow) {
+                            out[j].x += sx == own.x ? amp : 0.f;
+                            out[j].y += sx == own.x + 1 ? amp : 0.f;
+                            out[j].z += sx == own.x + 2 ? amp : 0.f;
+                            out[j].w += sx == own.x + 3 ? amp : 0.f;
+                        }
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    old[j] = cur[j];
+                    cur[j] = out[j];
+                    B[own.at + j * kTilePitch] = out[j];
+                }
+            }
+            float4* const sw = A;
+            A = B;
+            B = sw;
+            amp = next_amp;
+            if (s + 1 < nsub) __syncthreads();
+        }
+        // publish the tile into the other set
+        float* const pub0 = set ? t.ex[0][0] : t.ex[1][0];
+        float* const pub1 = set ? t.ex[0][1] : t.ex[1][1];
+        const long long o = so + (long long)own.z * a.P + own.x;
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (own.mine >> j & 1u) {
+                *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + (long long)j * a.P, pub0, fbytes, 16, 103)) = cur[j];
+                *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + (long long)j * a.P, pub1, fbytes, 16, 103)) = old[j];
+            }
+        set ^= 1;
+        if (k >= t.k1) break;
+        want += gridDim.x;
+        if (!tile_barrier(t.bar, want, t.status, &alive)) return;
+        // the halo, both fields, from the other tiles
+        const unsigned halo = own.valid & ~own.mine;
+        if (halo) {
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (halo >> j & 1u) {
+                    cur[j] = tile_fetch(pub0 + so, own.z + j, own.x, a.nz, a.P, pub0, fbytes);
+                    old[j] = tile_fetch(pub1 + so, own.z + j, own.x, a.nz, a.P, pub1, fbytes);
+                }
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (halo >> j & 1u) A[own.at + j * kTilePitch] = cur[j];
+        }
+        __syncthreads();
+    }
+}
+
+}  // namespace pam
