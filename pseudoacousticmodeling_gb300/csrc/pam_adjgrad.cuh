@@ -304,24 +304,59 @@ __global__ void __launch_bounds__(128, 3) adjgrad_kernel(const AdjGradArgs ag)
     cp_async_wait<0>();
 }
 
-// G = sum of the group partials (expanded grid, the update region); ilum on
-// the interior grid [nzi][nxi] from the illumination partials.
+// The sums over time of the shots (or groups of shots), gp and ip, into the
+// gradient and the illumination of the model, in three passes over small
+// arrays: the groups per cell, then the transpose of the edge-replicating
+// padding along z and along x (kappa = (vp vp)(dt dt) is constant along each
+// folded line), and the chain rule d kappa / d vp = 2 vp dt^2 on
+// G = kappa dJ/dkappa.  All in double: only the gradient itself is rounded.
 __global__ void adjgrad_fold_kernel(const float* __restrict__ gp, const float* __restrict__ ip, int ngroups,
                                     long long stride, int nz, int nx, int P, int N, int nzi, int nxi,
-                                    float* __restrict__ G, float* __restrict__ ilum)
+                                    double* __restrict__ G, float* __restrict__ ilum)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int z = blockIdx.y;
     if (x >= nx || z >= nz) return;
     const long long c = (long long)z * P + x;
-    float g = 0.0f, i = 0.0f;
+    double g = 0.0;
+    float i = 0.0f;
     for (int k = 0; k < ngroups; k++) {
-        g += gp[(long long)k * stride + c];
+        g += (double)gp[(long long)k * stride + c];
         i += ip[(long long)k * stride + c];
     }
     G[c] = g;
     const int zi = z - N, xi = x - N;
     if (zi >= 0 && zi < nzi && xi >= 0 && xi < nxi) ilum[(long long)zi * nxi + xi] = i;
+}
+
+// G [nz][P] in place: row N + zi becomes the sum of the rows that replicate it.
+__global__ void adjgrad_fold_rows_kernel(double* __restrict__ G, int nz, int nx, int P, int N, int nzi)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= nx) return;
+    double top = 0.0, bottom = 0.0;
+    for (int k = 0; k < N; k++) {
+        top += G[(long long)k * P + x];
+        bottom += G[(long long)(nz - 1 - k) * P + x];
+    }
+    G[(long long)N * P + x] += top;
+    G[(long long)(N + nzi - 1) * P + x] += bottom;
+}
+
+__global__ void adjgrad_fold_cols_kernel(const double* __restrict__ G, const float* __restrict__ kap,
+                                         const float* __restrict__ vp, int nx, int P, int N, int nzi, int nxi, double dt2,
+                                         float* __restrict__ grad)
+{
+    const int xi = blockIdx.x * blockDim.x + threadIdx.x, zi = blockIdx.y;
+    if (xi >= nxi) return;
+    const double* row = G + (long long)(zi + N) * P;
+    double g = row[N + xi];
+    if (xi == 0)
+        for (int k = 0; k < N; k++) g += row[k];
+    if (xi == nxi - 1)
+        for (int k = 0; k < N; k++) g += row[nx - 1 - k];
+    const double v = vp[(long long)zi * nxi + xi], k = kap[(long long)(zi + N) * P + N + xi];
+    grad[(long long)zi * nxi + xi] = (float)(g / k * 2.0 * v * dt2);
 }
 
 }  // namespace pam

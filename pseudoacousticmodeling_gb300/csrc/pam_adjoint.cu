@@ -91,7 +91,8 @@ int pam_engine::ensure_adjoint(int K, int store) {
         } else {
             // G, and the partial sums of the fused adjoint + gradient pass per group of four shots
             const size_t groups = (size_t)(B + kWarpsPerBlock - 1) / kWarpsPerBlock;
-            if (dalloc_bytes((void**)&d_gk, field * 4) || dalloc_bytes((void**)&d_gp, groups * field * 4) ||
+            if (dalloc_bytes((void**)&d_gk, field * 8) || dalloc_bytes((void**)&d_grad_b, interior * 4) ||
+                dalloc_bytes((void**)&d_gp, groups * field * 4) ||
                 dalloc_bytes((void**)&d_ip, groups * field * 4))
                 return PAM_E_CUDA;
         }
@@ -420,11 +421,24 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     if (sb && (cfg.nz < 9 || cfg.nx < 9)) return fail(PAM_E_ARG, "boundary saving needs nz, nx >= 9");
     if (!sb && !rbc && (K <= 0 || K > cfg.nt)) K = cfg.nt;
     CU(cudaSetDevice(device));
-    if (int rc = tune_segments(nshots, st)) return rc;
     if (int rc = ensure_adjoint(K, store)) return rc;
-    if (mode == kExact)
-        if (int rc = tune_adjgrad(nshots, st)) return rc;
     const int nseg = adj_nseg;
+    // small runs: the forward and backward sweeps as persistent tiles (pam_tile.cuh)
+    const TilePlan *ftiles = nullptr, *btiles = nullptr;
+    if (!sb && !rbc) {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        CU(cudaStreamIsCapturing(st, &capturing));
+        if (capturing == cudaStreamCaptureStatusNone) ftiles = tile_plan(nshots);
+        if (ftiles)
+            if (int rc = tile_begin(*ftiles, st)) return rc;
+        const TileJob bjob = mode == kExact ? kTileExactJob : kTileRtmJob;
+        if (mode != kFWIRef)
+            if (int rc = tile_adjoint_begin(nshots, bjob, st, &btiles)) return rc;
+    }
+    if (!ftiles || (!btiles && cfg.approximation == PAM_ACOUSTIC))
+        if (int rc = tune_segments(nshots, st)) return rc;
+    if (mode == kExact && !btiles)
+        if (int rc = tune_adjgrad(nshots, st)) return rc;
     if (rbc) {
         // the random border (random_boundary.cpp), velocities capped at 95% of the
         // leapfrog limit v dt sqrt(S (1/dx^2 + 1/dz^2)) <= 2, S = 6.50158 the largest
@@ -519,7 +533,6 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
 
     CU(cudaMemsetAsync(d_ilum_b, 0, interior * 4, st));     // the exact gradient's illumination of this call
     const bool mp = mode == kFWIRef && multiparameter && cfg.approximation != PAM_ACOUSTIC;
-    if (mode == kExact) CU(cudaMemsetAsync(d_gk, 0, (size_t)field * 4, st));
 
     // ---- 1. forward sweep: modelled data and checkpoints
     // the exact adjoint of a given adjoint source (pam_adjoint_gradient) needs
@@ -563,14 +576,24 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         auto lslot = [&](int t) { return d_seg + (size_t)(t - tl + 1) * B * field; };
         float* seis = need_data ? d_seis_own : nullptr;
         for (int k = 0; k < tl; k++) {
-            if (k % K == 0)
-                if (int rc = save_checkpoint(this, k / K, nshots, st, d_u[k & 1], d_u[(k + 1) & 1])) return rc;
-            enqueue_forward_step(k, nshots, seis, st);
+            if (k % K == 0) {
+                const float* const cur = ftiles ? tile_state(0) : d_u[k & 1];
+                const float* const prev = ftiles ? tile_state(1) : d_u[(k + 1) & 1];
+                if (int rc = save_checkpoint(this, k / K, nshots, st, cur, prev)) return rc;
+                if (ftiles)
+                    if (int rc = tile_forward(*ftiles, nshots, seis, k, k + K, st)) return rc;
+            }
+            if (!ftiles) enqueue_forward_step(k, nshots, seis, st);
         }
-        CU(cudaMemcpyAsync(lslot(tl - 1), d_u[(tl + 1) & 1], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice,
-                           st));
-        CU(cudaMemcpyAsync(lslot(tl), d_u[tl & 1], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
-        for (int k = tl; k < nt; k++) enqueue_forward_step(k, nshots, seis, st, lslot(k), lslot(k - 1), lslot(k + 1));
+        const float* const cur = ftiles ? tile_state(0) : d_u[tl & 1];
+        const float* const prev = ftiles ? tile_state(1) : d_u[(tl + 1) & 1];
+        CU(cudaMemcpyAsync(lslot(tl - 1), prev, (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
+        CU(cudaMemcpyAsync(lslot(tl), cur, (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
+        if (ftiles) {
+            if (int rc = tile_forward(*ftiles, nshots, seis, tl, nt, st, lslot(tl), tl)) return rc;
+        } else {
+            for (int k = tl; k < nt; k++) enqueue_forward_step(k, nshots, seis, st, lslot(k), lslot(k - 1), lslot(k + 1));
+        }
         CU(cudaGetLastError());
     }
 
@@ -810,16 +833,32 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                                    cudaMemcpyDeviceToDevice, st));
                 CU(cudaMemcpyAsync(slot(t0), d_u[t0 & 1], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
             }
-            for (int k = t0; k < t1; k++)
-                enqueue_forward_step(k, nshots, (need_data && nseg == 1) ? d_seis_own : nullptr, st, slot(k),
-                                     slot(k - 1), slot(k + 1));
+            float* const seis = need_data && nseg == 1 ? d_seis_own : nullptr;
+            if (ftiles) {
+                if (int rc = tile_forward(*ftiles, nshots, seis, t0, t1, st, slot(t0), t0)) return rc;
+            } else {
+                for (int k = t0; k < t1; k++)
+                    enqueue_forward_step(k, nshots, seis, st, slot(k), slot(k - 1), slot(k + 1));
+            }
         }
         CU(cudaGetLastError());
         if (need_data && !residual_ready)
             if (int rc = make_residual()) return rc;
 
         if (int rc = wait_obs()) return rc;
-        for (int t = t1 - 1; t >= t0; t--) receiver_step(t, slot(t - 1), slot(t), slot(t + 1));
+        if (btiles) {
+            if (mode == kRTM && t1 == nt) {
+                // the data of the last step; the tiles inject the next ones
+                const long long n = (long long)nrec * nshots;
+                inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
+                    d_ub[0], d_obs, d_rz, d_rx, nrec, nshots, nt - 1 - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
+            }
+            if (int rc = tile_adjoint(*btiles, mode == kExact ? kTileExactJob : kTileRtmJob, nshots, t0, t1, slot(t0), t0,
+                                      d_obs, inv_dxdz, st))
+                return rc;
+        } else {
+            for (int t = t1 - 1; t >= t0; t--) receiver_step(t, slot(t - 1), slot(t), slot(t + 1));
+        }
         CU(cudaGetLastError());
         if (aniso_misaligned) return fail(PAM_E_CUDA, "anisotropic adjoint: operands not 16-byte aligned");
     }
@@ -833,40 +872,34 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         // (migration images, reference-form and multiparameter gradients were
         // summed into the totals step by step)
         if (mode == kExact) {
-            // the shot groups' partial sums into G (expanded grid) and this
-            // call's illumination, then into the illumination pam_fwi_result returns
+            // the shot groups' sums into this call's gradient and illumination, the
+            // latter then into the illumination pam_fwi_result returns
             const dim3 fg((nxa + 255) / 256, nza);
-            adjgrad_fold_kernel<<<fg, 256, 0, st>>>(d_gp, d_ip, ngroups, field, nza, nxa, P, N, nzi, nxi, d_gk,
-                                                    d_ilum_b);
+            // (the tiles have a group of its own for each shot)
+            adjgrad_fold_kernel<<<fg, 256, 0, st>>>(btiles ? d_tile_sum[0] : d_gp, btiles ? d_tile_sum[1] : d_ip,
+                                                    btiles ? nshots : ngroups, field, nza, nxa, P, N, nzi, nxi, d_gk, d_ilum_b);
+            adjgrad_fold_rows_kernel<<<(nxa + 63) / 64, 64, 0, st>>>(d_gk, nza, nxa, P, N, nzi);
+            adjgrad_fold_cols_kernel<<<dim3((nxi + 127) / 128, nzi), 128, 0, st>>>(d_gk, d_kap, d_vp, nxa, P, N, nzi, nxi,
+                                                                                   (double)cfg.dt * cfg.dt, d_grad_b);
             reduce_shots_kernel<<<blocks, 256, 0, st>>>(d_ilum_b, d_grad_ilum, n, 1);   // already summed
         }
+        if (mode == kRTM && btiles) tile_fold_image(nshots, d_img, d_img_ilum, st);
         CU(cudaGetLastError());
     }
     if (mode == kExact) {
-        // G = kappa dJ/dkappa on the expanded grid, summed over the batch; the
-        // transpose of the edge-replicating padding folds it onto the model,
-        // where kappa = (vp vp)(dt dt) is constant along each folded line, then
-        // the chain rule d kappa / d vp = 2 vp dt^2
-        std::vector<float> gk((size_t)field);
-        CU(cudaMemcpyAsync(gk.data(), d_gk, gk.size() * 4, cudaMemcpyDeviceToHost, st));
+        const size_t n = (size_t)cfg.nz * cfg.nx;
+        std::vector<float> g(n);
+        CU(cudaMemcpyAsync(g.data(), d_grad_b, n * 4, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
-        const int nz = cfg.nz, nx = cfg.nx;
-        std::vector<double> acc((size_t)nz * nx, 0.0);
-        for (int z = 0; z < nza; z++) {
-            const int zi = std::min(std::max(z - N, 0), nz - 1);
-            for (int x = 0; x < nxa; x++) {
-                const int xi = std::min(std::max(x - N, 0), nx - 1);
-                acc[(size_t)zi * nx + xi] += (double)gk[(size_t)z * P + x];
-            }
-        }
-        const float dt2f = cfg.dt * cfg.dt;
-        const double dt2 = (double)cfg.dt * cfg.dt;
-        for (size_t i = 0; i < acc.size(); i++) {
-            const float kap = (h_vp[i] * h_vp[i]) * dt2f;
-            grad_vp[i] += (float)(acc[i] / (double)kap * 2.0 * (double)h_vp[i] * dt2);
-        }
+        for (size_t i = 0; i < n; i++) grad_vp[i] += g[i];
     }
     CU(cudaStreamSynchronize(st));
+    if (ftiles || btiles) {
+        // a barrier of the tiles that was given up (a non-finite sample shows in the misfit)
+        int v = 0;
+        CU(cudaMemcpy(&v, d_status, sizeof(int), cudaMemcpyDeviceToHost));
+        if (v & 2) return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
+    }
     if (misfit) *misfit += mis;
     return PAM_OK;
 }

@@ -152,6 +152,7 @@ int pam_engine::init(const pam_config& c, int dev) {
     const size_t field = (size_t)nza * P;
     shot_stride = (long long)field;
     if (dalloc(this, &d_kap, field)) return PAM_E_CUDA;
+    if (c.approximation == PAM_ACOUSTIC && dalloc(this, &d_vp, (size_t)c.nz * c.nx)) return PAM_E_CUDA;
     if (c.approximation != PAM_ACOUSTIC) {
         if (dalloc(this, &d_eps, field) || dalloc(this, &d_del, field) || dalloc(this, &d_e2, field) ||
             dalloc(this, &d_m1, field) || dalloc(this, &d_m2, field))
@@ -226,6 +227,7 @@ int pam_engine::set_models(const float* vp, const float* eps, const float* del, 
     // would not wait for a modelling call still running on one of them
     CU(cudaDeviceSynchronize());
     CU(cudaMemcpy(d_kap, kap.data(), kap.size() * sizeof(float), cudaMemcpyHostToDevice));
+    if (!aniso) CU(cudaMemcpy(d_vp, vp, n * sizeof(float), cudaMemcpyHostToDevice));
     if (aniso) {
         h_eps.assign(eps, eps + n);
         h_del.assign(del, del + n);
@@ -316,7 +318,7 @@ int pam_engine::set_receivers(int n, const int* rz, const int* rx, int per_shot)
     CU(cudaMemcpy(d_rx, rx, cnt * sizeof(int), cudaMemcpyHostToDevice));
     h_rz.assign(rz, rz + cnt);
     h_rx.assign(rx, rx + cnt);
-    tile_lists_stale = true;
+    tile_lists_stale = tile_inject_stale = true;
     nrec = n;
     rec_per_shot = per_shot ? 1 : 0;
     invalidate_graph();

@@ -10,6 +10,10 @@
 #include "../../include/pam.h"
 #include "pam_types.h"
 
+namespace pam {
+struct TileArgs;
+}
+
 struct pam_engine {
     pam_config cfg{};
     int device = 0;
@@ -101,7 +105,9 @@ struct pam_engine {
     float* d_ub[2] = {nullptr, nullptr};
     float *d_bpsix = nullptr, *d_bzetax = nullptr, *d_bpsiz = nullptr, *d_bzetaz = nullptr;
     float2 *d_bxaux = nullptr, *d_bzaux = nullptr;
-    float* d_gk = nullptr;               // [stride]: kappa dJ/dkappa summed over the batch
+    double* d_gk = nullptr;              // [stride]: kappa dJ/dkappa summed over the batch
+    float* d_grad_b = nullptr;           // [nz][nx] gradient of one exact-gradient call
+    float* d_vp = nullptr;               // [nz][nx] velocity (acoustic)
     float* d_gp = nullptr;               // [ceil(B/4)][stride] partial sums of the fused adjoint +
     float* d_ip = nullptr;               // gradient pass per group of four shots (G and illumination)
     float* d_ilum_b = nullptr;           // [nz][nx] illumination of one exact-gradient call
@@ -149,10 +155,29 @@ struct pam_engine {
         int T = 0, TZ = 0, TX = 0, nty = 0, ntx = 0, R = 0;
         int group = 0;                   // shots per launch
     };
-    std::map<int, TilePlan> tile_plans;
-    const TilePlan* tile_plan(int nshots);
+    enum TileJob { kTileForward = 0, kTileExactJob = 1, kTileRtmJob = 2 };
+    std::map<int, TilePlan> tile_plans[3];
+    const TilePlan* tile_plan(int nshots, TileJob job = kTileForward);
     int tile_begin(const TilePlan& p, cudaStream_t s);
-    int tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s);
+    pam::TileArgs tile_args(const TilePlan& p, int nshots) const;
+    // with slots every U(k) goes to slots + (k - kslot) fields and the state
+    // before step k0 is U(k0), U(k0 - 1) there
+    int tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s, float* slots = nullptr,
+                     int kslot = 0);
+    const float* tile_state(int i) const { return tile_set ? d_tile[i] : d_u[i]; }   // 0: U(k), 1: U(k-1)
+    // backward sweeps of the acoustic jobs: steps t = k1-1 .. k0 of a segment
+    // with its source fields in slots, the sums of each shot's cells in d_tile_sum
+    int tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, const TilePlan** out);
+    int tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0, int k1, const float* slots, int kslot,
+                     const float* data, float scale, cudaStream_t s);
+    void tile_fold_image(int nshots, float* img, float* ilum, cudaStream_t s) const;
+    float* d_tile_b[2] = {nullptr, nullptr};     // [B][stride] second published receiver-side state
+    float* d_tile_sum[2] = {nullptr, nullptr};   // [B][stride] sums over time: gradient or image, illumination
+    int* d_inj_beg = nullptr;
+    int2* d_inj_ent = nullptr;
+    bool tile_inject_stale = true, tile_inject_ok = false;
+    int tile_inject_shape[4] = {0, 0, 0, 0};
+    int tile_bset = 0;
     float* d_tile[2] = {nullptr, nullptr};   // [B][stride] the second published state of the tiles
     unsigned* d_tile_bar = nullptr;
     int* d_tile_beg = nullptr;           // receivers by tile (tile_begin)

@@ -32,10 +32,15 @@ constexpr int kTileSmemMax = 226 * 1024;
 // 0.5 million cells with T = 1 .. 8 and R = 2 .. 4, which they meet within 10%
 constexpr double kTileBarrierUs = 1.62, kTileRowUs = 0.265, kTileStepUs = 0.05;
 constexpr double kTileCellUs[3] = {3.2e-4, 5.5e-4, 9.0e-4};
+// ... and of the sums over time of a tile's cell (backward sweeps, by job)
+constexpr double kTileSumUs[3] = {0.0, 4.0e-4, 1.5e-4};
 // the same of a graph of one-step launches, by approximation: the latency of a
 // step, and a cell of the batch (0.15 to 2.2 million cells: 5.7 to 9.2 us
 // acoustic, 6.9 to 10.3 us VTI, 7.6 to 10.2 us TTI)
 constexpr double kGraphStepUs[3] = {5.5, 6.6, 7.2}, kGraphCellUs[3] = {1.6e-6, 2.1e-6, 3.5e-6};
+
+// ... and of a backward step as launches of its own
+constexpr double kBackStepUs = 10.0, kBackCellUs = 4.5e-6;
 
 int models_of(int approx) {
     return approx == PAM_ACOUSTIC ? tile_models<kAcoustic>() : approx == PAM_VTI ? tile_models<kVTI>() : tile_models<kTTI>();
@@ -54,22 +59,31 @@ TileShape shape_of(const pam_engine::TilePlan& p) {
     return g;
 }
 
-template <int A, int R>
-cudaError_t launch_forward(const TileArgs& t, int blocks, size_t smem, cudaStream_t s) {
-    // the shared-memory opt-in is a per-device attribute of the kernel
-    static bool configured[kMaxDevices] = {};
+size_t smem_of(const TileShape& g, int approx, int job) {
+    return job == pam_engine::kTileForward ? tile_smem_bytes(g, models_of(approx)) : tile_adj_smem_bytes(g);
+}
+
+// A cooperative launch; the shared-memory opt-in is a per-device attribute of
+// the kernel.
+template <class Args>
+cudaError_t launch(void (*kernel)(const Args), bool* configured, const Args& args, int blocks, int threads, size_t smem,
+                   cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices || !configured[dev]) {
-        cudaError_t err = cudaFuncSetAttribute(tile_forward_kernel<A, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kTileSmemMax);
+        cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
         if (err != cudaSuccess) return err;
         if (dev >= 0 && dev < kMaxDevices) configured[dev] = true;
     }
-    TileArgs q = t;
-    void* args[] = {&q};
-    return cudaLaunchCooperativeKernel((const void*)tile_forward_kernel<A, R>, dim3(blocks), dim3(tile_threads(t.g)), args,
-                                       smem, s);
+    Args q = args;
+    void* list[] = {&q};
+    return cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(threads), list, smem, s);
+}
+
+template <int A, int R>
+cudaError_t launch_forward(const TileArgs& t, int blocks, size_t smem, cudaStream_t s) {
+    static bool configured[kMaxDevices] = {};
+    return launch<TileArgs>(tile_forward_kernel<A, R>, configured, t, blocks, tile_threads(t.g), smem, s);
 }
 
 template <int A>
@@ -77,6 +91,35 @@ cudaError_t launch_forward(const TileArgs& t, int blocks, size_t smem, cudaStrea
     return t.g.R == 2   ? launch_forward<A, 2>(t, blocks, smem, s)
            : t.g.R == 3 ? launch_forward<A, 3>(t, blocks, smem, s)
                         : launch_forward<A, 4>(t, blocks, smem, s);
+}
+
+template <int MODE, int R>
+cudaError_t launch_adjoint(const TileAdjArgs& t, int blocks, size_t smem, cudaStream_t s) {
+    static bool configured[kMaxDevices] = {};
+    return launch<TileAdjArgs>(tile_adjoint_kernel<MODE, R>, configured, t, blocks, tile_threads(t.f.g), smem, s);
+}
+
+template <int MODE>
+cudaError_t launch_adjoint(const TileAdjArgs& t, int blocks, size_t smem, cudaStream_t s) {
+    return t.f.g.R == 2   ? launch_adjoint<MODE, 2>(t, blocks, smem, s)
+           : t.f.g.R == 3 ? launch_adjoint<MODE, 3>(t, blocks, smem, s)
+                          : launch_adjoint<MODE, 4>(t, blocks, smem, s);
+}
+
+__global__ void tile_fold_image_kernel(const float* __restrict__ gsum, const float* __restrict__ isum, long long stride,
+                                       int B, int P, int N, int nzi, int nxi, float* __restrict__ img,
+                                       float* __restrict__ ilum)
+{
+    const int xi = blockIdx.x * blockDim.x + threadIdx.x, zi = blockIdx.y;
+    if (xi >= nxi || zi >= nzi) return;
+    const long long c = (long long)(zi + N) * P + xi + N;
+    float g = 0.0f, i = 0.0f;
+    for (int b = 0; b < B; b++) {
+        g += gsum[(long long)b * stride + c];
+        i += isum[(long long)b * stride + c];
+    }
+    img[(long long)zi * nxi + xi] += g;
+    ilum[(long long)zi * nxi + xi] += i;
 }
 
 }  // namespace
@@ -88,10 +131,11 @@ cudaError_t launch_forward(const TileArgs& t, int blocks, size_t smem, cudaStrea
 // and the cells of each step's region at the rate one SM updates them; a batch
 // may go in several launches of some shots each.  The tiles are taken where
 // the best of these is below the cost of the one-step launches.
-const pam_engine::TilePlan* pam_engine::tile_plan(int nshots) {
+const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
     if (cfg.boundary != PAM_CERJAN || prof_stride > 0 || std::getenv("PAM_NO_PERSISTENT")) return nullptr;
-    auto it = tile_plans.find(nshots);
-    if (it == tile_plans.end()) {
+    std::map<int, TilePlan>& plans = tile_plans[job];
+    auto it = plans.find(nshots);
+    if (it == plans.end()) {
         TilePlan best;
         int sms = 0, coop = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 0;
@@ -101,7 +145,9 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots) {
         // (a receiver's place is held in 16 bits each way)
         const bool fits = nza < 32768 && nxa < 65536;
         const int approx = cfg.approximation;
-        double best_cost = kGraphStepUs[approx] + kGraphCellUs[approx] * nshots * (double)nza * nxa;
+        const double cells_all = nshots * (double)nza * nxa;
+        double best_cost = job == kTileForward ? kGraphStepUs[approx] + kGraphCellUs[approx] * cells_all
+                                               : kBackStepUs + kBackCellUs * cells_all;
         for (int group = nshots; fits && coop && group >= 1; group = group > 1 ? (group + 1) / 2 : 0) {
             const int launches = (nshots + group - 1) / group;
             for (int ntx0 = 1; ntx0 * group <= sms && ntx0 <= (cols + 3) / 4; ntx0++) {
@@ -122,13 +168,14 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots) {
                         p.group = group;
                         const TileShape g = shape_of(p);
                         if (tile_threads(g) > kTileThreads || g.EXq >= kTilePitch ||
-                            tile_smem_bytes(g, models_of(approx)) > (size_t)kTileSmemMax)
+                            smem_of(g, approx, job) > (size_t)kTileSmemMax)
                             break;
                         double cost = kTileBarrierUs + kTileRowUs * R;
                         for (int s = 0; s < T; s++) {
                             const double cells =
                                 (double)std::min(TZ + 8 * s, rows) * std::min(TX + 8 * s, (cols + 3) / 4 * 4);
                             cost += kTileStepUs + cells * kTileCellUs[approx];
+                            if (job != kTileForward) cost += (double)TZ * TX * kTileSumUs[job];
                         }
                         cost *= (double)launches / T;
                         if (cost < best_cost) {
@@ -138,7 +185,7 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots) {
                     }
             }
         }
-        it = tile_plans.emplace(nshots, best).first;
+        it = plans.emplace(nshots, best).first;
     }
     return it->second.usable ? &it->second : nullptr;
 }
@@ -188,31 +235,39 @@ int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
     return PAM_OK;
 }
 
-int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s) {
-    if (k1 <= k0) return PAM_OK;
-    TileArgs t;
+TileArgs pam_engine::tile_args(const TilePlan& p, int nshots) const {
+    TileArgs t{};
     t.s = step_args(0, nshots, nullptr, nullptr, 0);
     t.g = shape_of(p);
+    t.wavelet = d_wavelet;
+    t.rec.nrec = nrec;
+    t.rec.nt_data = nt_data;
+    t.rec.per_shot = rec_per_shot;
+    t.nt = cfg.nt;
+    t.itlag = cfg.itlag;
+    t.bar = d_tile_bar;
+    t.status = d_status;
+    return t;
+}
+
+int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s, float* slots,
+                             int kslot) {
+    if (k1 <= k0) return PAM_OK;
+    TileArgs t = tile_args(p, nshots);
     t.ex[0][0] = d_u[0];
     t.ex[0][1] = d_u[1];
     t.ex[1][0] = d_tile[0];
     t.ex[1][1] = d_tile[1];
     t.set0 = tile_set;
-    t.wavelet = d_wavelet;
-    t.rec = RecordArgs{};
     t.rec.seis = d_seis;
-    t.rec.nrec = nrec;
-    t.rec.nt_data = nt_data;
-    t.rec.per_shot = rec_per_shot;
     t.rec_beg = d_tile_beg;
     t.rec_ent = d_tile_ent;
-    t.nt = cfg.nt;
-    t.itlag = cfg.itlag;
     t.k0 = k0;
     t.k1 = k1;
-    t.bar = d_tile_bar;
-    t.status = d_status;
-    const size_t smem = tile_smem_bytes(t.g, models_of(cfg.approximation));
+    t.slots = slots;
+    t.slot_stride = shot_stride * B;
+    t.kslot = kslot;
+    const size_t smem = smem_of(t.g, cfg.approximation, kTileForward);
     for (int b = 0; b < nshots; b += p.group) {
         t.shot0 = b;
         const int blocks = std::min(p.group, nshots - b) * p.nty * p.ntx;
@@ -224,6 +279,125 @@ int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k
         if (err != cudaSuccess) return fail(PAM_E_CUDA, "cooperative launch failed: %s", cudaGetErrorString(err));
     }
     // every group of T steps publishes into the other set
-    tile_set ^= ((k1 - k0 + p.T - 1) / p.T) & 1;
+    if (!slots) tile_set ^= ((k1 - k0 + p.T - 1) / p.T) & 1;
     return PAM_OK;
+}
+
+// ---------------------------------------------------------------- backward sweeps
+
+// The plan of a backward sweep, its buffers and each thread's receivers; nullptr
+// in *out for the one-step launches.  Receivers off the update region, which
+// the one-step kernels inject into cells that no step writes, and lists too
+// long for shared memory stay with those.
+int pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, const TilePlan** out) {
+    pam_engine* e = this;
+    *out = nullptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(s, &cs));
+    if (cfg.approximation != PAM_ACOUSTIC || cs != cudaStreamCaptureStatusNone) return PAM_OK;
+    const TilePlan* p = tile_plan(nshots, job);
+    if (!p) return PAM_OK;
+    const TileShape g = shape_of(*p);
+    const bool same = !tile_inject_stale && tile_inject_shape[0] == p->T && tile_inject_shape[1] == p->TZ &&
+                      tile_inject_shape[2] == p->TX && tile_inject_shape[3] == p->R;
+    if (!same) {
+        const int nt = p->nty * p->ntx, lists = rec_per_shot ? B : 1, nthr = tile_threads(g);
+        std::vector<int> beg((size_t)nt * lists * (nthr + 1));
+        std::vector<int2> ent;
+        std::vector<std::vector<int2>> of(nthr);
+        tile_inject_ok = true;
+        for (size_t i = 0; i < h_rz.size() && tile_inject_ok; i++)
+            tile_inject_ok = h_rz[i] >= 4 && h_rz[i] < nza - 4 && h_rx[i] >= 4 && h_rx[i] < nxa - 4;
+        for (int l = 0; l < lists * nt && tile_inject_ok; l++) {
+            const int tile = l % nt;
+            const int ez0 = 4 + (tile / p->ntx) * p->TZ - 4 * p->T, ex0 = 4 + (tile % p->ntx) * p->TX - 4 * p->T;
+            for (auto& v : of) v.clear();
+            for (int r = 0; r < nrec; r++) {
+                const size_t i = (size_t)(l / nt) * nrec + r;
+                const int er = h_rz[i] - ez0, ec = h_rx[i] - ex0;
+                if (er < 0 || er >= g.nrg * g.R || ec < 0 || ec >= 4 * g.EXq) continue;
+                of[(er / g.R) * g.EXq + ec / 4].push_back(make_int2(h_rz[i] << 16 | h_rx[i], r));
+            }
+            const size_t first = ent.size();
+            int* const b = &beg[(size_t)l * (nthr + 1)];
+            for (int j = 0; j < nthr; j++) {
+                b[j] = (int)ent.size();
+                ent.insert(ent.end(), of[j].begin(), of[j].end());
+            }
+            b[nthr] = (int)ent.size();
+            if (ent.size() - first > (size_t)kTileInject) tile_inject_ok = false;
+        }
+        if (tile_inject_ok) {
+            dfree(d_inj_beg);
+            dfree(d_inj_ent);
+            d_inj_beg = nullptr;
+            d_inj_ent = nullptr;
+            ent.resize(std::max<size_t>(ent.size(), 1));
+            if (dalloc_bytes((void**)&d_inj_beg, beg.size() * sizeof(int)) ||
+                dalloc_bytes((void**)&d_inj_ent, ent.size() * sizeof(int2)))
+                return PAM_E_CUDA;
+            CU(cudaMemcpyAsync(d_inj_beg, beg.data(), beg.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+            CU(cudaMemcpyAsync(d_inj_ent, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+            CU(cudaStreamSynchronize(s));   // the vectors go out of scope
+        }
+        tile_inject_stale = false;
+        tile_inject_shape[0] = p->T;
+        tile_inject_shape[1] = p->TZ;
+        tile_inject_shape[2] = p->TX;
+        tile_inject_shape[3] = p->R;
+    }
+    if (!tile_inject_ok) return PAM_OK;
+    const size_t field = (size_t)shot_stride * B;
+    for (float*& d : d_tile_b)
+        if (!d) {
+            if (dalloc_bytes((void**)&d, field * 4)) return PAM_E_CUDA;
+            CU(cudaMemsetAsync(d, 0, field * 4, s));
+        }
+    for (float*& d : d_tile_sum)
+        if (!d && dalloc_bytes((void**)&d, field * 4)) return PAM_E_CUDA;
+    if (!d_tile_bar && dalloc_bytes((void**)&d_tile_bar, 128)) return PAM_E_CUDA;
+    for (float* d : d_tile_sum) CU(cudaMemsetAsync(d, 0, (size_t)shot_stride * nshots * 4, s));
+    tile_bset = 0;
+    *out = p;
+    return PAM_OK;
+}
+
+int pam_engine::tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0, int k1, const float* slots, int kslot,
+                             const float* data, float scale, cudaStream_t s) {
+    if (k1 <= k0) return PAM_OK;
+    TileAdjArgs t{};
+    t.f = tile_args(p, nshots);
+    t.f.ex[0][0] = d_ub[0];
+    t.f.ex[0][1] = d_ub[1];
+    t.f.ex[1][0] = d_tile_b[0];
+    t.f.ex[1][1] = d_tile_b[1];
+    t.f.set0 = tile_bset;
+    t.f.k0 = k0;
+    t.f.k1 = k1;
+    t.f.slots = const_cast<float*>(slots);
+    t.f.slot_stride = shot_stride * B;
+    t.f.kslot = kslot;
+    t.inj_beg = d_inj_beg;
+    t.inj_ent = d_inj_ent;
+    t.data = data;
+    t.scale = scale;
+    t.gsum = d_tile_sum[0];
+    t.isum = d_tile_sum[1];
+    const size_t smem = smem_of(t.f.g, cfg.approximation, job);
+    for (int b = 0; b < nshots; b += p.group) {
+        t.f.shot0 = b;
+        const int blocks = std::min(p.group, nshots - b) * p.nty * p.ntx;
+        cudaError_t err = cudaMemsetAsync(d_tile_bar, 0, sizeof(unsigned), s);
+        if (err == cudaSuccess)
+            err = job == kTileExactJob ? launch_adjoint<kTileExact>(t, blocks, smem, s)
+                                       : launch_adjoint<kTileRtm>(t, blocks, smem, s);
+        if (err != cudaSuccess) return fail(PAM_E_CUDA, "cooperative launch failed: %s", cudaGetErrorString(err));
+    }
+    tile_bset ^= ((k1 - k0 + p.T - 1) / p.T) & 1;
+    return PAM_OK;
+}
+
+void pam_engine::tile_fold_image(int nshots, float* img, float* ilum, cudaStream_t s) const {
+    tile_fold_image_kernel<<<dim3((cfg.nx + 255) / 256, cfg.nz), 256, 0, s>>>(d_tile_sum[0], d_tile_sum[1], shot_stride, nshots,
+                                                                             P, N, cfg.nz, cfg.nx, img, ilum);
 }

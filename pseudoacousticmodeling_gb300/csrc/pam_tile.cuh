@@ -74,6 +74,12 @@ struct TileArgs {
     int nt, itlag, k0, k1;
     unsigned* bar;                       // barrier counter, zero at the launch
     int* status;                         // bit 1 set when a barrier was given up
+    // every U(k) kept: U(k) at slots + (k - kslot) * slot_stride; the state before
+    // step k0 is U(k0), U(k0 - 1) there, and so is what the tiles exchange
+    // (nullptr: the two published sets)
+    float* slots;
+    long long slot_stride;
+    int kslot;
 };
 
 // Grid-wide barrier of resident blocks: each block's writes before it are
@@ -116,14 +122,14 @@ struct TileCells {
 };
 
 template <int R>
-__device__ __forceinline__ TileCells<R> tile_cells(const StepArgs& a, const TileShape& g, int tile) {
+__device__ __forceinline__ TileCells<R> tile_cells(const StepArgs& a, const TileShape& g, int tile, int pitch) {
     const int z0 = 4 + (tile / g.ntx) * g.TZ, x0 = 4 + (tile % g.ntx) * g.TX;
     const int z1 = min(z0 + g.TZ, a.nz - 4), x1 = min(x0 + g.TX, a.nx - 4);
     const int rg = threadIdx.x / g.EXq, q = threadIdx.x - rg * g.EXq;
     TileCells<R> c;
     c.z = z0 - 4 * g.T + rg * R;
     c.x = x0 - 4 * g.T + 4 * q;
-    c.at = (4 + min(rg, g.nrg - 1) * R) * kTilePitch + q;
+    c.at = (4 + min(rg, g.nrg - 1) * R) * pitch + q;
     c.need = 1 << 20;
     c.valid = c.mine = 0;
     auto factor = [&](int i, int len) {
@@ -158,15 +164,16 @@ __device__ __forceinline__ TileCells<R> tile_cells(const StepArgs& a, const Tile
 // calls it (Z passes the z derivatives on, with a barrier), and out is left
 // alone where the thread is not active.
 template <int APPROX, int R, class Model>
-__device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>& t, const float4* __restrict__ A,
+__device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>& t, int pitch,
+                                          const float4* __restrict__ A,
                                           float4* __restrict__ Z, bool active, const float4 (&cur)[R],
                                           const float4 (&old)[R], Model model, float4 (&out)[R]) {
     const float4* const col = A + t.at;
     float4 w[R + 8];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        w[j] = col[(j - 4) * kTilePitch];
-        w[R + 4 + j] = col[(R + j) * kTilePitch];
+        w[j] = col[(j - 4) * pitch];
+        w[R + 4 + j] = col[(R + j) * pitch];
     }
 #pragma unroll
     for (int j = 0; j < R; j++) w[j + 4] = cur[j];
@@ -181,14 +188,14 @@ __device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>&
             pzv[j][1] = d1_pair_ref(hi2(w[j + 5]), hi2(w[j + 3]), hi2(w[j + 6]), hi2(w[j + 2]), hi2(w[j + 7]), hi2(w[j + 1]),
                                     hi2(w[j + 8]), hi2(w[j]), a.inv_dz);
             if (APPROX == kTTI && t.valid)
-                Z[t.at + j * kTilePitch] = make_float4(pzv[j][0].x, pzv[j][0].y, pzv[j][1].x, pzv[j][1].y);
+                Z[t.at + j * pitch] = make_float4(pzv[j][0].x, pzv[j][0].y, pzv[j][1].x, pzv[j][1].y);
         }
     }
     if (APPROX == kTTI) __syncthreads();
     if (!active) return;
 #pragma unroll
     for (int j = 0; j < R; j++) {
-        const float4 c = cur[j], l = col[j * kTilePitch - 1], r = col[j * kTilePitch + 1];
+        const float4 c = cur[j], l = col[j * pitch - 1], r = col[j * pitch + 1];
         const float4 kap = model(0, j);
         const float2 P0 = lo2(l), P1 = hi2(l), P2 = lo2(c), P3 = hi2(c), P4 = lo2(r), P5 = hi2(r);
         const float2 O0 = make_float2(l.y, l.z), O1 = make_float2(l.w, c.x), O2 = make_float2(c.y, c.z);
@@ -208,7 +215,7 @@ __device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>&
             pz[1] = pzv[j][1];
         }
         if (APPROX == kTTI) {
-            const float4 zl = Z[t.at + j * kTilePitch - 1], zr = Z[t.at + j * kTilePitch + 1];
+            const float4 zl = Z[t.at + j * pitch - 1], zr = Z[t.at + j * pitch + 1];
             const float2 V0 = lo2(zl), V1 = hi2(zl), V4 = lo2(zr), V5 = hi2(zr);
             const float2 W0 = make_float2(zl.y, zl.z), W1 = make_float2(zl.w, pz[0].x);
             const float2 W2 = make_float2(pz[0].y, pz[1].x), W3 = make_float2(pz[1].y, zr.x);
@@ -260,7 +267,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
     const int ntiles = g.nty * g.ntx;
     const int shot = t.shot0 + blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
     const int tid = threadIdx.x, nthr = blockDim.x;
-    const TileCells<R> own = tile_cells<R>(a, g, tile);
+    const TileCells<R> own = tile_cells<R>(a, g, tile, kTilePitch);
     const int copy = (g.nrg * R + 8) * kTilePitch;
     float4* A = tsm;                       // U(k)
     float4* B = tsm + copy;                // U(k+1)
@@ -275,8 +282,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
     float4 cur[R], old[R], kap[R];
     {
         for (int i = tid; i < ncopy * copy; i += nthr) tsm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* const in0 = t.set0 ? t.ex[1][0] : t.ex[0][0];
-        const float* const in1 = t.set0 ? t.ex[1][1] : t.ex[0][1];
+        const float* const in0 = t.slots ? t.slots + (t.k0 - t.kslot) * t.slot_stride : t.set0 ? t.ex[1][0] : t.ex[0][0];
+        const float* const in1 = t.slots ? in0 - t.slot_stride : t.set0 ? t.ex[1][1] : t.ex[0][1];
         const float* const mod[6] = {a.kap, a.e2, a.m1, a.m2, a.cth, a.sth};
 #pragma unroll
         for (int j = 0; j < R; j++) {
@@ -332,6 +339,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
 
     int k = t.k0, set = t.set0;
     unsigned want = 0;
+    const long long o = so + (long long)own.z * a.P + own.x;   // the thread's first cell in a field
     float amp = k + 1 < t.nt ? t.wavelet[k + 1] : 0.0f;
     while (k < t.k1) {
         const int nsub = min(g.T, t.k1 - k);
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
             // a region of halo 4 (nsub - 1 - s) around the tile, whole threads of it
             const bool active = own.need <= 4 * (nsub - 1 - s);
             float4 out[R];
-            if (active || APPROX == kTTI) tile_step<APPROX, R>(a, own, A, Z, active, cur, old, model, out);
+            if (active || APPROX == kTTI) tile_step<APPROX, R>(a, own, kTilePitch, A, Z, active, cur, old, model, out);
             if (active) {
                 if (has_src)
 #pragma unroll
@@ -372,18 +380,25 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
             A = B;
             B = sw;
             amp = next_amp;
+            if (t.slots && own.mine) {
+                float* const u = t.slots + (k + 1 - t.kslot) * t.slot_stride;
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                    if (own.mine >> j & 1u)
+                        *reinterpret_cast<float4*>(PAM_CHK(u + o + (long long)j * a.P, u, fbytes, 16, 105)) = cur[j];
+            }
             if (s + 1 < nsub) __syncthreads();
         }
         // publish the tile into the other set
-        float* const pub0 = set ? t.ex[0][0] : t.ex[1][0];
-        float* const pub1 = set ? t.ex[0][1] : t.ex[1][1];
-        const long long o = so + (long long)own.z * a.P + own.x;
+        float* const pub0 = t.slots ? t.slots + (k - t.kslot) * t.slot_stride : set ? t.ex[0][0] : t.ex[1][0];
+        float* const pub1 = t.slots ? pub0 - t.slot_stride : set ? t.ex[0][1] : t.ex[1][1];
+        if (!t.slots)
 #pragma unroll
-        for (int j = 0; j < R; j++)
-            if (own.mine >> j & 1u) {
-                *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + (long long)j * a.P, pub0, fbytes, 16, 103)) = cur[j];
-                *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + (long long)j * a.P, pub1, fbytes, 16, 103)) = old[j];
-            }
+            for (int j = 0; j < R; j++)
+                if (own.mine >> j & 1u) {
+                    *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + (long long)j * a.P, pub0, fbytes, 16, 103)) = cur[j];
+                    *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + (long long)j * a.P, pub1, fbytes, 16, 103)) = old[j];
+                }
         set ^= 1;
         if (k >= t.k1) break;
         want += gridDim.x;
@@ -403,6 +418,266 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
         }
         __syncthreads();
     }
+}
+
+// ---------------------------------------------------------------- backward sweeps
+
+// The backward sweep of a small acoustic batch over the steps t = k1-1 .. k0
+// of a segment whose source fields U(t) are stored, with the fields as
+// tiles, like the forward loop; the receiver-side field advances by the forward
+// recursion (see inject_adjoint_kernel), and the sums of each cell over time
+// stay in the block until the launch ends.
+//   kTileExact: w(t) from w(t+1), w(t+2), then the residual of time t at the
+//               receivers; G += w(t+1) L U(t) (t <= nt-2), I += U(t)^2
+//   kTileRtm:   G += Ub(t) U(t), I += U(t)^2, Ub(t-1) from Ub(t), Ub(t+1), then
+//               the data of time t-1
+// U(t) of the tile and four cells around it comes through a ring of shared
+// copies filled by cp.async three steps ahead; the data of a group's steps are
+// staged in shared memory one group ahead.
+enum TileMode { kTileExact = 0, kTileRtm = 1 };
+
+constexpr int kTileRing = 4;
+constexpr int kTileInject = 1024;      // most receiver entries of a tile with its halo
+
+struct TileAdjArgs {
+    TileArgs f;                          // k0, k1: the segment; slots: U(t); ex: the receiver-side field
+    const int* __restrict__ inj_beg;     // [tiles (per shot)][threads + 1] entries of each thread's cells
+    const int2* __restrict__ inj_ent;    // (row << 16 | column of the expanded grid, receiver)
+    const float* __restrict__ data;      // [B][nt_data][nrec] residual or observed data
+    float scale;                         // of the data (kTileRtm)
+    float* gsum;                         // [B][nz][P] sums, continued
+    float* isum;
+};
+
+__host__ __device__ inline int tile_pitch(const TileShape& g) { return g.EXq; }
+__host__ __device__ inline size_t tile_adj_smem_bytes(const TileShape& g) {
+    const size_t copy = (size_t)(g.nrg * g.R + 8) * tile_pitch(g) * 16;
+    return (2 + kTileRing) * copy + (size_t)2 * g.R * tile_threads(g) * 16 + (size_t)kTileInject * (16 + 2 * 4 * g.T);
+}
+
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// s + a b, the product rounded before it is added, as where the one-step
+// kernels pass it through shared memory
+__device__ __forceinline__ float4 add_product(float4 s, float4 a, float4 b) {
+    return make_float4(__fadd_rn(s.x, __fmul_rn(a.x, b.x)), __fadd_rn(s.y, __fmul_rn(a.y, b.y)),
+                       __fadd_rn(s.z, __fmul_rn(a.z, b.z)), __fadd_rn(s.w, __fmul_rn(a.w, b.w)));
+}
+
+template <int MODE, int R>
+__global__ void __launch_bounds__(kTileThreads, 1) tile_adjoint_kernel(const TileAdjArgs ta)
+{
+    extern __shared__ float4 tsm[];
+    __shared__ int alive;
+    const TileArgs& t = ta.f;
+    const StepArgs& a = t.s;
+    const TileShape& g = t.g;
+    const int ntiles = g.nty * g.ntx;
+    const int shot = t.shot0 + blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
+    const int tid = threadIdx.x, nthr = blockDim.x, pitch = tile_pitch(g);
+    const TileCells<R> own = tile_cells<R>(a, g, tile, pitch);
+    const int copy = (g.nrg * R + 8) * pitch;
+    float4* A = tsm;                               // the field read by the step
+    float4* B = tsm + copy;                        // the field it writes
+    float4* const ring = tsm + 2 * copy;           // copies of U(t), at t & 3
+    float4* const G = ring + kTileRing * copy + tid;   // [R] sums of the thread's cells
+    float4* const I = G + R * nthr;
+    float4* const ient = ring + kTileRing * copy + 2 * R * nthr;       // entries: offset, factors, kappa
+    float* const idat = reinterpret_cast<float*>(ient + kTileInject);  // [2][T][entries] staged data
+    const long long so = (long long)shot * a.shot_stride;
+    const long long o = so + (long long)own.z * a.P + own.x;
+    [[maybe_unused]] const long long fbytes = (long long)a.B * a.shot_stride * 4;
+    [[maybe_unused]] const long long mbytes = (long long)a.nz * a.P * 4;
+
+    // U(t) is needed on the tile (kTileRtm) and four cells around it (kTileExact)
+    const bool want_u = own.need <= (MODE == kTileExact ? 4 : 0);
+    auto fetch_u = [&](int tt) {
+        if (tt >= t.k0 && want_u) {
+            const float* const u = t.slots + (tt - t.kslot) * t.slot_stride;
+            float4* const dst = ring + (tt & (kTileRing - 1)) * copy + own.at;
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (own.valid >> j & 1u) cp_async16(dst + j * pitch, PAM_CHK(u + o + (long long)j * a.P, u, fbytes, 16, 110));
+        }
+        cp_async_commit();
+    };
+
+    float4 cur[R], old[R], kap[R];
+    for (int i = tid; i < (2 + kTileRing) * copy; i += nthr) tsm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    {
+        const float* const in0 = t.set0 ? t.ex[1][0] : t.ex[0][0];
+        const float* const in1 = t.set0 ? t.ex[1][1] : t.ex[0][1];
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int z = own.valid >> j & 1u ? own.z + j : -1;
+            cur[j] = tile_fetch(in0 + so, z, own.x, a.nz, a.P, in0, fbytes);
+            old[j] = tile_fetch(in1 + so, z, own.x, a.nz, a.P, in1, fbytes);
+            kap[j] = tile_fetch(a.kap, z, own.x, a.nz, a.P, a.kap, mbytes);
+            // the sums go on from the last segment's
+            G[j * nthr] = tile_fetch(ta.gsum + so, z, own.x, a.nz, a.P, ta.gsum, fbytes);
+            I[j * nthr] = tile_fetch(ta.isum + so, z, own.x, a.nz, a.P, ta.isum, fbytes);
+        }
+    }
+    auto model = [&](int, int j) { return kap[j]; };
+
+    // the receivers of the thread's cells: entries [ib, ie) of the tile's list,
+    // which starts at il; the field time of the injection after step t is t - lag
+    const long long list = (long long)(t.rec.per_shot ? shot * ntiles + tile : tile) * (nthr + 1);
+    const int il = ta.inj_beg[list], nent = ta.inj_beg[list + nthr] - il;
+    const int ib = ta.inj_beg[list + tid] - il, ie = ta.inj_beg[list + tid + 1] - il;
+    constexpr int lag = MODE == kTileExact ? 0 : 1;
+    const float* const data = ta.data + (long long)shot * t.rec.nt_data * t.rec.nrec;
+    for (int i = ib; i < ie; i++) {
+        const int2 e = ta.inj_ent[il + i];
+        const int z = e.x >> 16, x = e.x & 0xffff;
+        const float fx = x < a.N ? a.cerjan[x] : x >= a.nx - a.N ? a.cerjan[a.nx - 1 - x] : 1.0f;
+        const float fz = z < a.N ? a.cerjan[z] : z >= a.nz - a.N ? a.cerjan[a.nz - 1 - z] : 1.0f;
+        const int off = (own.at + (z - own.z) * pitch) * 4 + x - own.x;
+        ient[i] = make_float4(__int_as_float(off), fx, fz, a.kap[(long long)z * a.P + x]);
+    }
+    // the data of the group of n steps whose first is tt, staged at parity p
+    auto stage = [&](int tt, int n, int p) {
+        for (int i = tid; i < nent; i += nthr) {
+            const int r = ta.inj_ent[il + i].y;
+            for (int s = 0; s < n; s++) {
+                const int it = tt - s - lag - t.itlag;
+                float* const dst = idat + (p * g.T + s) * nent + i;
+                if (it >= 0) cp_async4(dst, data + (long long)it * t.rec.nrec + r);
+                else *dst = 0.0f;
+            }
+        }
+    };
+
+    int k = t.k1 - 1, set = t.set0, parity = 0;
+    unsigned want = 0;
+    stage(k, min(g.T, k - t.k0 + 1), 0);
+    __syncthreads();                               // the copies are zero before they are written
+    fetch_u(k);
+    fetch_u(k - 1);
+    fetch_u(k - 2);
+    if (own.valid)
+#pragma unroll
+        for (int j = 0; j < R; j++) A[own.at + j * pitch] = cur[j];
+    cp_async_wait<2>();                            // U(k) and the first group's data
+    __syncthreads();
+
+    while (k >= t.k0) {
+        const int nsub = min(g.T, k - t.k0 + 1);
+        if (k - nsub >= t.k0) stage(k - nsub, min(g.T, k - nsub - t.k0 + 1), parity ^ 1);
+        for (int s = 0; s < nsub; s++, k--) {
+            fetch_u(k - 3);
+            if (own.mine) {
+                // the sums of the tile's cells
+                const float4* const U = ring + (k & (kTileRing - 1)) * copy + own.at;
+                float4 w[R + 8];
+                if (MODE == kTileExact)
+#pragma unroll
+                    for (int j = 0; j < R + 8; j++) w[j] = U[(j - 4) * pitch];
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    if (!(own.mine >> j & 1u)) continue;
+                    const float4 c = MODE == kTileExact ? w[j + 4] : U[j * pitch];
+                    float4 q = I[j * nthr];
+                    if (MODE == kTileExact) {
+                        const float4 l = U[j * pitch - 1], r = U[j * pitch + 1];
+                        const float2 P0 = lo2(l), P1 = hi2(l), P2 = lo2(c), P3 = hi2(c), P4 = lo2(r), P5 = hi2(r);
+                        const float2 O0 = make_float2(l.y, l.z), O1 = make_float2(l.w, c.x), O2 = make_float2(c.y, c.z);
+                        const float2 O3 = make_float2(c.w, r.x), O4 = make_float2(r.y, r.z);
+                        q = add_product(q, c, c);
+                        if (k <= t.nt - 2) {
+                            const float2 L0 = padd2(d2_pair(P2, O2, O1, P3, P1, O3, O0, P4, P0, a.inv_dx2),
+                                                    d2_pair(lo2(c), lo2(w[j + 5]), lo2(w[j + 3]), lo2(w[j + 6]),
+                                                            lo2(w[j + 2]), lo2(w[j + 7]), lo2(w[j + 1]), lo2(w[j + 8]),
+                                                            lo2(w[j]), a.inv_dz2));
+                            const float2 L1 = padd2(d2_pair(P3, O3, O2, P4, P2, O4, O1, P5, P1, a.inv_dx2),
+                                                    d2_pair(hi2(c), hi2(w[j + 5]), hi2(w[j + 3]), hi2(w[j + 6]),
+                                                            hi2(w[j + 2]), hi2(w[j + 7]), hi2(w[j + 1]), hi2(w[j + 8]),
+                                                            hi2(w[j]), a.inv_dz2));
+                            G[j * nthr] = add_product(G[j * nthr], cur[j], make_float4(L0.x, L0.y, L1.x, L1.y));
+                        }
+                    } else {
+                        const float2 i0 = pfma2(lo2(c), lo2(c), lo2(q)), i1 = pfma2(hi2(c), hi2(c), hi2(q));
+                        q = make_float4(i0.x, i0.y, i1.x, i1.y);
+                        const float4 p = G[j * nthr];
+                        const float2 g0 = pfma2(lo2(cur[j]), lo2(c), lo2(p)), g1 = pfma2(hi2(cur[j]), hi2(c), hi2(p));
+                        G[j * nthr] = make_float4(g0.x, g0.y, g1.x, g1.y);
+                    }
+                    I[j * nthr] = q;
+                }
+            }
+            if (own.need <= 4 * (nsub - 1 - s)) {
+                float4 out[R];
+                tile_step<kAcoustic, R>(a, own, pitch, A, nullptr, true, cur, old, model, out);
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    old[j] = cur[j];
+                    cur[j] = out[j];
+                    B[own.at + j * pitch] = out[j];
+                }
+                if (ie > ib) {
+                    const float* const d = idat + (parity * g.T + s) * nent;
+                    for (int i = ib; i < ie; i++) {
+                        const float4 e = ient[i];
+                        float* const p = reinterpret_cast<float*>(B) + __float_as_int(e.x);
+                        float v = d[i];
+                        if (MODE == kTileExact) {
+                            v = __fmul_rn(__fmul_rn(v, e.y), e.z);
+                            v = __fmul_rn(e.w, __fmul_rn(__fmul_rn(v, e.y), e.z));
+                        } else {
+                            v = __fmul_rn(v, ta.scale);
+                        }
+                        *p = __fadd_rn(*p, v);
+                    }
+#pragma unroll
+                    for (int j = 0; j < R; j++) cur[j] = B[own.at + j * pitch];
+                }
+            }
+            float4* const sw = A;
+            A = B;
+            B = sw;
+            if (s + 1 < nsub) {
+                cp_async_wait<2>();                // U of the next step
+                __syncthreads();
+            }
+        }
+        parity ^= 1;
+        float* const pub0 = set ? t.ex[0][0] : t.ex[1][0];
+        float* const pub1 = set ? t.ex[0][1] : t.ex[1][1];
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (own.mine >> j & 1u) {
+                *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + (long long)j * a.P, pub0, fbytes, 16, 111)) = cur[j];
+                *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + (long long)j * a.P, pub1, fbytes, 16, 111)) = old[j];
+            }
+        set ^= 1;
+        if (k < t.k0) break;
+        cp_async_wait<0>();                        // the next group's data (and U)
+        want += gridDim.x;
+        if (!tile_barrier(t.bar, want, t.status, &alive)) return;
+        const unsigned halo = own.valid & ~own.mine;
+        if (halo) {
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (halo >> j & 1u) {
+                    cur[j] = tile_fetch(pub0 + so, own.z + j, own.x, a.nz, a.P, pub0, fbytes);
+                    old[j] = tile_fetch(pub1 + so, own.z + j, own.x, a.nz, a.P, pub1, fbytes);
+                }
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (halo >> j & 1u) A[own.at + j * pitch] = cur[j];
+        }
+        __syncthreads();
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int j = 0; j < R; j++)
+        if (own.mine >> j & 1u) {
+            *reinterpret_cast<float4*>(PAM_CHK(ta.gsum + o + (long long)j * a.P, ta.gsum, fbytes, 16, 112)) = G[j * nthr];
+            *reinterpret_cast<float4*>(PAM_CHK(ta.isum + o + (long long)j * a.P, ta.isum, fbytes, 16, 112)) = I[j * nthr];
+        }
 }
 
 }  // namespace pam

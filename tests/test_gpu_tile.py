@@ -67,3 +67,60 @@ def test_tiles_in_chunks_with_pinned_output(approx):
     ref = e.forward(sz, sx)
     out = torch.zeros((2, 74, 30)).pin_memory()
     assert np.array_equal(e.forward(sz, sx, out=out.numpy()), ref)
+
+
+# (nz, nx, border, steps, lag, shots): odd sizes, several shots per launch and
+# more than fit at once, a step count that no group divides, two segments or more
+BACK = [(8, 8, 8, 40, 0, 1), (61, 133, 12, 61, 11, 2), (20, 24, 9, 47, 3, 170), (90, 61, 20, 97, 30, 5),
+        (201, 401, 50, 83, 10, 1)]
+
+
+@pytest.mark.parametrize("job", ["gradient", "rtm"])
+@pytest.mark.parametrize("shape", BACK, ids=lambda s: "x".join(map(str, s)))
+def test_backward_tiles_match_the_one_step_launches(job, shape, monkeypatch):
+    """The fields of the backward tiles are the one-step launches' bit for bit;
+    the sums over time and shots are added in another order: each sum has at
+    most steps x shots terms in float32, so the two differ by a random walk of
+    that many roundings, 2^-24 sqrt(steps x shots) of the sum of magnitudes,
+    here held to 16 times that in relative L2 (cancellation within a cell)."""
+    nz, nx, N, nt, itlag, shots = shape
+    e, rng = _engine("acoustic", nz, nx, N, nt, itlag, shots)
+    nza, nxa = nz + 2 * N, nx + 2 * N
+    sz, sx = rng.integers(4, nza - 4, shots).astype(np.int32), rng.integers(4, nxa - 4, shots).astype(np.int32)
+    rz, rx = rng.integers(4, nza - 4, 60).astype(np.int32), rng.integers(4, nxa - 4, 60).astype(np.int32)
+    # one source, and receivers beside it, inside the model, so that its sums are not zero
+    sz[0], sx[0] = nza // 2, nxa // 2
+    rz[:6], rx[:6] = sz[0] + 1, sx[0] + np.arange(6) - 3
+    rz[1], rx[1] = rz[0], rx[0]
+    prz, prx = rng.integers(4, nza - 4, (shots, 9)).astype(np.int32), rng.integers(4, nxa - 4, (shots, 9)).astype(np.int32)
+    prz[0, :4], prx[0, :4] = rz[:4], rx[:4]
+    tol = 16 * 2.0 ** -24 * np.sqrt(nt * shots)
+
+    def run(z, d, K):
+        e.rtm_reset()
+        if job == "rtm":
+            e.rtm(sz, sx, d, ckpt_interval=K)
+            return e.rtm_result(norm="none")
+        J, g = e.misfit_gradient(sz, sx, d, ckpt_interval=K)
+        return g, e.fwi_result()[1], np.array([J])
+
+    def close(a, b):
+        for x, y in zip(a, b):
+            n = np.linalg.norm(y.astype(np.float64))
+            assert np.isfinite(y).all() and n > 0
+            assert np.linalg.norm(x.astype(np.float64) - y) <= tol * n
+
+    for z, x, per_shot in ((rz, rx, False), (prz, prx, True)):
+        e.set_receivers(z, x, per_shot=per_shot)
+        d = (1e-2 * rng.standard_normal((shots, nt - itlag, z.shape[-1]))).astype(np.float32)
+        tiles = run(z, d, 0)
+        for K in (17, nt - 1):      # the order of the sums does not depend on the segments
+            assert all(np.array_equal(a, b) for a, b in zip(run(z, d, K), tiles))
+        monkeypatch.setenv("PAM_NO_PERSISTENT", "1")
+        one_step = run(z, d, 0)
+        monkeypatch.delenv("PAM_NO_PERSISTENT")
+        close(tiles, one_step)
+    # receivers on the frame stay with the one-step launches
+    e.set_receivers(np.array([0, N + 1, sz[0] + 1], np.int32), np.array([N, N + 2, sx[0]], np.int32))
+    d = (1e-2 * rng.standard_normal((shots, nt - itlag, 3))).astype(np.float32)
+    close(run(rz, d, 0), run(rz, d, 17))
