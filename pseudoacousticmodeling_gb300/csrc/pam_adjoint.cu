@@ -240,23 +240,27 @@ int restore_checkpoint(pam_engine* e, int s, int nshots, cudaStream_t st, float*
     return PAM_OK;
 }
 
-// Boundary saving: save / write back the band of a source-field buffer.
-int save_band(pam_engine* e, const float* field, int slot, int nshots, cudaStream_t st) {
+// Boundary saving: save / write back the band of a source-field buffer; the save
+// takes `times` consecutive fields from the first slot on.
+int save_band(pam_engine* e, const float* field, int slot, int nshots, cudaStream_t st, int times = 1) {
     const GridDims g = dims(e);
     const long long nb = band_cells(e->cfg.nz, e->cfg.nx);
     const int nchunk = (int)((nb + kBandChunk - 1) / kBandChunk);
     const size_t sb = store_bytes(e->adj_store);
     char* dst = (char*)e->d_band + (size_t)slot * e->B * (size_t)nb * sb;
     float* sc = e->d_band_scale + (size_t)slot * e->B * nchunk;
-    const dim3 grid(nchunk, nshots);
+    if (times < 1) return PAM_OK;
+    const dim3 grid(nchunk, nshots, times);
+    const long long fs = e->shot_stride * e->B;
     if (e->adj_store == PAM_STORE_F32)
-        band_save_kernel<float><<<grid, kBandChunk, 0, st>>>(field, (float*)dst, sc, g, e->cfg.nz, e->cfg.nx, 0.0f);
+        band_save_kernel<float><<<grid, kBandChunk, 0, st>>>(field, (float*)dst, sc, g, e->cfg.nz, e->cfg.nx, 0.0f, fs,
+                                                             e->B);
     else if (e->adj_store == PAM_STORE_BF16)
         band_save_kernel<__nv_bfloat16><<<grid, kBandChunk, 0, st>>>(field, (__nv_bfloat16*)dst, sc, g, e->cfg.nz,
-                                                                     e->cfg.nx, 1.0f);
+                                                                     e->cfg.nx, 1.0f, fs, e->B);
     else
         band_save_kernel<__half><<<grid, kBandChunk, 0, st>>>(field, (__half*)dst, sc, g, e->cfg.nz, e->cfg.nx,
-                                                              16384.0f);
+                                                              16384.0f, fs, e->B);
     CU(cudaGetLastError());
     return PAM_OK;
 }
@@ -423,19 +427,32 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     CU(cudaSetDevice(device));
     if (int rc = ensure_adjoint(K, store)) return rc;
     const int nseg = adj_nseg;
-    // small runs: the forward and backward sweeps as persistent tiles (pam_tile.cuh)
-    const TilePlan *ftiles = nullptr, *btiles = nullptr;
-    if (!sb && !rbc) {
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        CU(cudaStreamIsCapturing(st, &capturing));
-        if (capturing == cudaStreamCaptureStatusNone) ftiles = tile_plan(nshots);
+    // small runs: the forward and backward sweeps as persistent tiles (pam_tile.cuh);
+    // rtiles: the source field backwards in time (boundary saving, random border).
+    // Forward sweeps that checkpoint CPML memory variables stay with the one-step
+    // launches; their backward sweeps do not, so that a sum over time has one order.
+    const TilePlan *ftiles = nullptr, *btiles = nullptr, *rtiles = nullptr;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(st, &capturing));
+    if (capturing == cudaStreamCaptureStatusNone) {
+        if (cfg.boundary != PAM_CPML || nseg <= 1) ftiles = tile_plan(nshots, kTileForwardLaunched);
+        if (sb || rbc) rtiles = tile_plan(nshots, kTileReverse);
+        if (sb && !rtiles) ftiles = nullptr;
         if (ftiles)
             if (int rc = tile_begin(*ftiles, st)) return rc;
-        const TileJob bjob = mode == kExact ? kTileExactJob : kTileRtmJob;
-        if (mode != kFWIRef)
-            if (int rc = tile_adjoint_begin(nshots, bjob, st, &btiles)) return rc;
+        if (mode != kFWIRef && (rtiles || !(sb || rbc)))
+            if (int rc = tile_adjoint_begin(nshots, mode == kExact ? kTileExactJob : kTileRtmJob, st, &btiles)) return rc;
+        if (rtiles) {
+            if (int rc = tile_buffers(st)) return rc;
+            if (!d_tile_slots) {
+                const size_t n = (size_t)shot_stride * B * (kTileSegment + 2);
+                if (dalloc_bytes((void**)&d_tile_slots, n * 4)) return PAM_E_CUDA;
+                CU(cudaMemsetAsync(d_tile_slots, 0, n * 4, st));   // the outer rows and columns stay zero
+            }
+        }
     }
-    if (!ftiles || (!btiles && cfg.approximation == PAM_ACOUSTIC))
+    if (!(rbc ? rtiles && (ftiles || mode == kRTM) : ftiles != nullptr) ||
+        (!btiles && cfg.approximation == PAM_ACOUSTIC))
         if (int rc = tune_segments(nshots, st)) return rc;
     if (mode == kExact && !btiles)
         if (int rc = tune_adjgrad(nshots, st)) return rc;
@@ -550,10 +567,37 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         if (need_data) {
             // the modelled data come from the absorbing scheme
             if (int rc = reset_fields(nshots, st)) return rc;
-            for (int k = 0; k < nt; k++) enqueue_forward_step(k, nshots, d_seis_own, st);
+            if (ftiles) {
+                if (int rc = tile_forward(*ftiles, nshots, d_seis_own, 0, nt, st)) return rc;
+            } else {
+                for (int k = 0; k < nt; k++) enqueue_forward_step(k, nshots, d_seis_own, st);
+            }
         }
         if (int rc = reset_fields(nshots, st)) return rc;
-        for (int k = 0; k < nt; k++) rbc_step(k, d_u[k & 1], nullptr, d_u[(k + 1) & 1]);
+        if (rtiles) {
+            if (int rc = tile_undamped(*rtiles, nshots, d_kap_rbc, st)) return rc;
+        } else {
+            for (int k = 0; k < nt; k++) rbc_step(k, d_u[k & 1], nullptr, d_u[(k + 1) & 1]);
+        }
+        CU(cudaGetLastError());
+    } else if (rtiles && ftiles) {
+        // boundary saving as tiles: segments of fields in the slots (slot j holds
+        // U(k0 - 1 + j)), then their bands in one launch
+        if (int rc = reset_fields(nshots, st)) return rc;
+        const size_t fb = (size_t)field * B;
+        CU(cudaMemcpyAsync(d_tile_slots, d_u[1], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
+        CU(cudaMemcpyAsync(d_tile_slots + fb, d_u[0], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
+        for (int k0 = 0; k0 < nt; k0 += kTileSegment) {
+            const int k1 = std::min(k0 + kTileSegment, nt), n = k1 - k0;
+            if (int rc = tile_forward(*ftiles, nshots, need_data ? d_seis_own : nullptr, k0, k1, st, d_tile_slots + fb, k0))
+                return rc;
+            if (int rc = save_band(this, d_tile_slots + fb, k0, nshots, st, std::min(n, nt - 1 - k0))) return rc;
+            // the state before step k1 to the front, or, at the end, to the field buffers
+            for (int i = 0; i < 2; i++) {
+                float* const to = k1 < nt ? d_tile_slots + i * fb : i == 0 ? d_u[(nt - 1) & 1] : d_u[nt & 1];
+                CU(cudaMemcpyAsync(to, d_tile_slots + (n + i) * fb, (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
+            }
+        }
         CU(cudaGetLastError());
     } else if (sb) {
         // every step's band of U(t), t = 0 .. nt-2; U(nt-1) and U(nt) stay in the buffers
@@ -783,7 +827,39 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     };
 
     // ---- 2. backward sweep
-    if (sb || rbc) {
+    if (rtiles) {
+        // segments t0 <= t < t1, last first: the source fields S(t0 - 1) .. S(t1)
+        // backwards in time into the slots (slot j holds S(t0 - 1 + j)), then the
+        // receiver side of the segment
+        if (int rc = wait_obs()) return rc;
+        const size_t fb = (size_t)field * B, bytes = (size_t)field * nshots * 4;
+        if (btiles) {
+            const long long n = (long long)nrec * nshots;
+            inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
+                d_ub[0], d_obs, d_rz, d_rx, nrec, nshots, nt - 1 - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
+        }
+        const float *s0 = d_u[(nt - 1) & 1], *s1 = d_u[nt & 1];   // S(t1 - 1), S(t1)
+        for (int t1 = nt; t1 > 0; t1 -= kTileSegment) {
+            const int t0 = std::max(t1 - kTileSegment, 0), n = t1 - t0;
+            CU(cudaMemcpyAsync(d_tile_slots + (n + 1) * fb, s1, bytes, cudaMemcpyDeviceToDevice, st));
+            CU(cudaMemcpyAsync(d_tile_slots + n * fb, s0, bytes, cudaMemcpyDeviceToDevice, st));
+            if (int rc = tile_reverse(*rtiles, nshots, std::max(t0, 1), t1, st, d_tile_slots + fb, t0, rbc ? d_kap_rbc : d_kap,
+                                      sb))
+                return rc;
+            auto slot = [&](int t) { return d_tile_slots + (size_t)(t - t0 + 1) * fb; };
+            if (btiles) {
+                if (int rc = tile_adjoint(*btiles, kTileRtmJob, nshots, t0, t1, slot(t0), t0, d_obs, inv_dxdz, st)) return rc;
+            } else {
+                for (int t = t1 - 1; t >= t0; t--) receiver_step(t, t ? slot(t - 1) : slot(0), slot(t), slot(t + 1));
+            }
+            // S(t0) and S(t0 - 1) are the next segment's S(t1), S(t1 - 1); its last
+            // slots lie behind these two (n >= 2 unless it is the last segment)
+            s1 = slot(t0);
+            s0 = slot(t0 - 1);
+        }
+        CU(cudaGetLastError());
+        if (aniso_misaligned) return fail(PAM_E_CUDA, "anisotropic adjoint: operands not 16-byte aligned");
+    } else if (sb || rbc) {
         // S(t-1) = 2 S(t) - S(t+1) + kappa L S(t) + w(t+1): the stepping kernel with
         // the time direction reversed and no damping, then (boundary saving) the
         // saved band of S(t-1); with the random border the whole grid reverses
@@ -894,7 +970,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         for (size_t i = 0; i < n; i++) grad_vp[i] += g[i];
     }
     CU(cudaStreamSynchronize(st));
-    if (ftiles || btiles) {
+    if (ftiles || btiles || rtiles) {
         // a barrier of the tiles that was given up (a non-finite sample shows in the misfit)
         int v = 0;
         CU(cudaMemcpy(&v, d_status, sizeof(int), cudaMemcpyDeviceToHost));

@@ -146,24 +146,38 @@ struct pam_engine {
     int tune_segments(int nshots, cudaStream_t s);
     // set by pam_adjoint_gradient: the exact job's data are the adjoint source
     bool adjoint_source_given = false;
+    // The one-barrier-per-step path of small Cerjan runs (step_persistent_kernel):
+    // the segment height to use for this batch, 0 for the graph path
+    static constexpr long long kPersistCells = 1LL << 20;
+    int persist_capacity = -1;
+    int persistent_height(int nshots);
+    int launch_persistent(int nshots, int H, float* d_seis, int k0, int k1, cudaStream_t s);
     // Small runs as persistent tiles (pam_tile.cu): the plan of a batch size, or
     // nullptr for the one-step launches; tile_begin makes the buffers and lists
     // of a plan ready, tile_forward runs steps k0 .. k1-1 from the state that
     // the run's earlier launches left (before the first: d_u[0], d_u[1])
     struct TilePlan {
         bool usable = false;
-        int T = 0, TZ = 0, TX = 0, nty = 0, ntx = 0, R = 0;
+        int T = 0, TZ = 0, TX = 0, nty = 0, ntx = 0, R = 0, halo = 4;
         int group = 0;                   // shots per launch
     };
-    enum TileJob { kTileForward = 0, kTileExactJob = 1, kTileRtmJob = 2 };
-    std::map<int, TilePlan> tile_plans[3];
+    enum TileJob { kTileForward = 0, kTileExactJob = 1, kTileRtmJob = 2, kTileReverse = 3, kTileForwardLaunched = 4 };
+    std::map<int, TilePlan> tile_plans[5];
     const TilePlan* tile_plan(int nshots, TileJob job = kTileForward);
+    int tile_buffers(cudaStream_t s);
     int tile_begin(const TilePlan& p, cudaStream_t s);
+    int tile_undamped(const TilePlan& p, int nshots, const float* kap, cudaStream_t s);
     pam::TileArgs tile_args(const TilePlan& p, int nshots) const;
     // with slots every U(k) goes to slots + (k - kslot) fields and the state
     // before step k0 is U(k0), U(k0 - 1) there
     int tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s, float* slots = nullptr,
                      int kslot = 0);
+    int tile_reverse(const TilePlan& p, int nshots, int k0, int k1, cudaStream_t s, float* slots, int kslot,
+                     const float* kap, bool bands);
+    float* d_tile_mem[2] = {nullptr, nullptr};    // [4][B][stride] CPML memory variables as published
+    float* d_tile_bmem[2] = {nullptr, nullptr};   // ... of the receiver-side field
+    float* d_tile_slots = nullptr;                // [kTileSegment + 2][B][stride] source fields of a segment
+    static constexpr int kTileSegment = 48;       // (boundary saving and the random border)
     const float* tile_state(int i) const { return tile_set ? d_tile[i] : d_u[i]; }   // 0: U(k), 1: U(k-1)
     // backward sweeps of the acoustic jobs: steps t = k1-1 .. k0 of a segment
     // with its source fields in slots, the sums of each shot's cells in d_tile_sum

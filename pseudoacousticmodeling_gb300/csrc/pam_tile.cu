@@ -32,6 +32,8 @@ constexpr int kTileSmemMax = 226 * 1024;
 // 0.5 million cells with T = 1 .. 8 and R = 2 .. 4, which they meet within 10%
 constexpr double kTileBarrierUs = 1.62, kTileRowUs = 0.265, kTileStepUs = 0.05;
 constexpr double kTileCellUs[3] = {3.2e-4, 5.5e-4, 9.0e-4};
+// ... more for a step with CPML strips
+constexpr double kTileStripUs = 1.2, kTileStripCellUs[2] = {1.1e-3, 1.9e-3};
 // ... and of the sums over time of a tile's cell (backward sweeps, by job)
 constexpr double kTileSumUs[3] = {0.0, 4.0e-4, 1.5e-4};
 // the same of a graph of one-step launches, by approximation: the latency of a
@@ -39,6 +41,13 @@ constexpr double kTileSumUs[3] = {0.0, 4.0e-4, 1.5e-4};
 // acoustic, 6.9 to 10.3 us VTI, 7.6 to 10.2 us TTI)
 constexpr double kGraphStepUs[3] = {5.5, 6.6, 7.2}, kGraphCellUs[3] = {1.6e-6, 2.1e-6, 3.5e-6};
 
+constexpr double kCpmlGraphStepUs = 9.6, kCpmlGraphCellUs[2] = {1.9e-6, 3.5e-6};
+// ... and of the one-barrier-per-step persistent loop (0.3 to 0.9 million cells:
+// 3.6 to 4.9 us acoustic, 4.6 to 5.9 us VTI, 5.4 to 8.5 us TTI)
+constexpr double kPersistStepUs[3] = {3.1, 4.1, 4.2}, kPersistCellUs[3] = {1.9e-6, 2.1e-6, 4.0e-6};
+// ... and what a step costs more as separate launches than as a graph (the
+// forward sweeps of migration and gradient jobs)
+constexpr double kLaunchUs = 1.0, kCpmlLaunchUs = 4.0;
 // ... and of a backward step as launches of its own
 constexpr double kBackStepUs = 10.0, kBackCellUs = 4.5e-6;
 
@@ -48,20 +57,25 @@ int models_of(int approx) {
 
 TileShape shape_of(const pam_engine::TilePlan& p) {
     TileShape g;
+    g.halo = p.halo;
     g.T = p.T;
     g.TZ = p.TZ;
     g.TX = p.TX;
     g.nty = p.nty;
     g.ntx = p.ntx;
     g.R = p.R;
-    g.nrg = (p.TZ + 8 * p.T + p.R - 1) / p.R;
-    g.EXq = p.TX / 4 + 2 * p.T;
+    g.nrg = (p.TZ + 2 * p.halo * p.T + p.R - 1) / p.R;
+    g.EXq = p.TX / 4 + p.halo / 2 * p.T;
     return g;
 }
 
 size_t smem_of(const TileShape& g, int approx, int job) {
-    return job == pam_engine::kTileForward ? tile_smem_bytes(g, models_of(approx)) : tile_adj_smem_bytes(g);
+    const bool forward = job != pam_engine::kTileExactJob && job != pam_engine::kTileRtmJob;
+    if (g.halo == 8) return tile_cpml_smem_bytes(g, models_of(approx), forward ? kTileForwardRole : kTileRtmRole);
+    return forward ? tile_smem_bytes(g, models_of(approx)) : tile_adj_smem_bytes(g);
 }
+
+int threads_of(const TileShape& g) { return g.halo == 8 ? tile_cpml_threads(g.R) : kTileThreads; }
 
 // A cooperative launch; the shared-memory opt-in is a per-device attribute of
 // the kernel.
@@ -80,17 +94,35 @@ cudaError_t launch(void (*kernel)(const Args), bool* configured, const Args& arg
     return cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(threads), list, smem, s);
 }
 
-template <int A, int R>
+template <int A, int R, bool REVERSE>
 cudaError_t launch_forward(const TileArgs& t, int blocks, size_t smem, cudaStream_t s) {
     static bool configured[kMaxDevices] = {};
-    return launch<TileArgs>(tile_forward_kernel<A, R>, configured, t, blocks, tile_threads(t.g), smem, s);
+    return launch<TileArgs>(tile_forward_kernel<A, R, REVERSE>, configured, t, blocks, tile_threads(t.g), smem, s);
 }
 
-template <int A>
+template <int A, bool REVERSE>
 cudaError_t launch_forward(const TileArgs& t, int blocks, size_t smem, cudaStream_t s) {
-    return t.g.R == 2   ? launch_forward<A, 2>(t, blocks, smem, s)
-           : t.g.R == 3 ? launch_forward<A, 3>(t, blocks, smem, s)
-                        : launch_forward<A, 4>(t, blocks, smem, s);
+    return t.g.R == 2   ? launch_forward<A, 2, REVERSE>(t, blocks, smem, s)
+           : t.g.R == 3 ? launch_forward<A, 3, REVERSE>(t, blocks, smem, s)
+                        : launch_forward<A, 4, REVERSE>(t, blocks, smem, s);
+}
+
+template <bool REVERSE>
+cudaError_t launch_forward(int approx, const TileArgs& t, int blocks, size_t smem, cudaStream_t s) {
+    return approx == PAM_ACOUSTIC ? launch_forward<kAcoustic, REVERSE>(t, blocks, smem, s)
+           : approx == PAM_VTI    ? launch_forward<kVTI, REVERSE>(t, blocks, smem, s)
+                                  : launch_forward<kTTI, REVERSE>(t, blocks, smem, s);
+}
+
+template <int A, int R, int ROLE>
+cudaError_t launch_cpml(const TileCpmlArgs& t, int blocks, size_t smem, cudaStream_t s) {
+    static bool configured[kMaxDevices] = {};
+    return launch<TileCpmlArgs>(tile_cpml_kernel<A, R, ROLE>, configured, t, blocks, tile_threads(t.r.f.g), smem, s);
+}
+
+template <int A, int ROLE>
+cudaError_t launch_cpml(const TileCpmlArgs& t, int blocks, size_t smem, cudaStream_t s) {
+    return t.r.f.g.R == 1 ? launch_cpml<A, 1, ROLE>(t, blocks, smem, s) : launch_cpml<A, 2, ROLE>(t, blocks, smem, s);
 }
 
 template <int MODE, int R>
@@ -132,7 +164,11 @@ __global__ void tile_fold_image_kernel(const float* __restrict__ gsum, const flo
 // may go in several launches of some shots each.  The tiles are taken where
 // the best of these is below the cost of the one-step launches.
 const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
-    if (cfg.boundary != PAM_CERJAN || prof_stride > 0 || std::getenv("PAM_NO_PERSISTENT")) return nullptr;
+    const int approx = cfg.approximation;
+    const bool cpml = cfg.boundary == PAM_CPML && job != kTileReverse;
+    if (prof_stride > 0 || std::getenv("PAM_NO_PERSISTENT")) return nullptr;
+    // with the matched layer: the forward loop of the acoustic and VTI operators, acoustic migration
+    if (cpml && (approx == PAM_TTI || job == kTileExactJob)) return nullptr;
     std::map<int, TilePlan>& plans = tile_plans[job];
     auto it = plans.find(nshots);
     if (it == plans.end()) {
@@ -144,10 +180,15 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
         const int rows = nza - 8, cols = nxa - 8;
         // (a receiver's place is held in 16 bits each way)
         const bool fits = nza < 32768 && nxa < 65536;
-        const int approx = cfg.approximation;
+        const bool forward = job != kTileExactJob && job != kTileRtmJob;
         const double cells_all = nshots * (double)nza * nxa;
-        double best_cost = job == kTileForward ? kGraphStepUs[approx] + kGraphCellUs[approx] * cells_all
-                                               : kBackStepUs + kBackCellUs * cells_all;
+        double best_cost = forward ? kGraphStepUs[approx] + kGraphCellUs[approx] * cells_all
+                                   : kBackStepUs + kBackCellUs * cells_all;
+        if (job == kTileForward && !cpml && cells_all <= kPersistCells)
+            best_cost = std::min(best_cost, kPersistStepUs[approx] + kPersistCellUs[approx] * cells_all);
+        if (cpml) best_cost = kCpmlGraphStepUs + kCpmlGraphCellUs[approx] * cells_all + (forward ? 0.0 : kBackStepUs);
+        if (job == kTileForwardLaunched) best_cost += cpml ? kCpmlLaunchUs : kLaunchUs;
+        const int halo = cpml ? 8 : 4;
         for (int group = nshots; fits && coop && group >= 1; group = group > 1 ? (group + 1) / 2 : 0) {
             const int launches = (nshots + group - 1) / group;
             for (int ntx0 = 1; ntx0 * group <= sms && ntx0 <= (cols + 3) / 4; ntx0++) {
@@ -155,7 +196,7 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
                 const int nty0 = std::min(sms / (ntx * group), rows);
                 if (nty0 < 1) break;
                 const int TZ = (rows + nty0 - 1) / nty0, nty = (rows + TZ - 1) / TZ;
-                for (int R = 2; R <= 4; R++)
+                for (int R = cpml ? 1 : 2; R <= (cpml ? 2 : 4); R++)
                     for (int T = 1; T <= kTileMaxT; T++) {
                         TilePlan p;
                         p.usable = true;
@@ -165,17 +206,19 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
                         p.nty = nty;
                         p.ntx = ntx;
                         p.R = R;
+                        p.halo = halo;
                         p.group = group;
                         const TileShape g = shape_of(p);
-                        if (tile_threads(g) > kTileThreads || g.EXq >= kTilePitch ||
+                        if (tile_threads(g) > threads_of(g) || g.EXq >= kTilePitch ||
                             smem_of(g, approx, job) > (size_t)kTileSmemMax)
                             break;
                         double cost = kTileBarrierUs + kTileRowUs * R;
                         for (int s = 0; s < T; s++) {
-                            const double cells =
-                                (double)std::min(TZ + 8 * s, rows) * std::min(TX + 8 * s, (cols + 3) / 4 * 4);
+                            const double cells = (double)std::min(TZ + 2 * halo * s, rows) *
+                                                 std::min(TX + 2 * halo * s, (cols + 3) / 4 * 4);
                             cost += kTileStepUs + cells * kTileCellUs[approx];
-                            if (job != kTileForward) cost += (double)TZ * TX * kTileSumUs[job];
+                            if (cpml) cost += kTileStripUs + cells * kTileStripCellUs[approx];
+                            if (!forward) cost += (double)TZ * TX * kTileSumUs[job];
                         }
                         cost *= (double)launches / T;
                         if (cost < best_cost) {
@@ -190,10 +233,7 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
     return it->second.usable ? &it->second : nullptr;
 }
 
-// The buffers of the persistent tiles, and each tile's list of the receivers
-// in it (receivers off the update region, whose samples are zero, go to the
-// nearest tile, which holds those cells in its halo).
-int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
+int pam_engine::tile_buffers(cudaStream_t s) {
     pam_engine* e = this;
     const size_t field = (size_t)shot_stride * B;
     for (float*& d : d_tile)
@@ -202,7 +242,22 @@ int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
             CU(cudaMemsetAsync(d, 0, field * 4, s));
         }
     if (!d_tile_bar && dalloc_bytes((void**)&d_tile_bar, 128)) return PAM_E_CUDA;
+    return PAM_OK;
+}
+
+// The buffers of the persistent tiles, and each tile's list of the receivers
+// in it (receivers off the update region, whose samples are zero, go to the
+// nearest tile, which holds those cells in its halo).
+int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
+    pam_engine* e = this;
+    const size_t field = (size_t)shot_stride * B;
+    if (int rc = tile_buffers(s)) return rc;
     tile_set = 0;
+    if (p.halo == 8) {
+        for (float*& d : d_tile_mem)
+            if (!d && dalloc_bytes((void**)&d, 4 * field * 4)) return PAM_E_CUDA;
+        CU(cudaMemsetAsync(d_tile_mem[0], 0, 4 * field * 4, s));
+    }
     if (!tile_lists_stale && tile_lists_TZ == p.TZ && tile_lists_TX == p.TX) return PAM_OK;
     const int nt = p.nty * p.ntx, lists = rec_per_shot ? B : 1;
     std::vector<int> beg((size_t)nt * lists + 1, 0);
@@ -247,6 +302,8 @@ TileArgs pam_engine::tile_args(const TilePlan& p, int nshots) const {
     t.itlag = cfg.itlag;
     t.bar = d_tile_bar;
     t.status = d_status;
+    t.mem_shots = B;
+    t.slot_stride = shot_stride * B;
     return t;
 }
 
@@ -265,21 +322,94 @@ int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k
     t.k0 = k0;
     t.k1 = k1;
     t.slots = slots;
-    t.slot_stride = shot_stride * B;
     t.kslot = kslot;
     const size_t smem = smem_of(t.g, cfg.approximation, kTileForward);
     for (int b = 0; b < nshots; b += p.group) {
         t.shot0 = b;
         const int blocks = std::min(p.group, nshots - b) * p.nty * p.ntx;
         cudaError_t err = cudaMemsetAsync(d_tile_bar, 0, sizeof(unsigned), s);
-        if (err == cudaSuccess)
-            err = cfg.approximation == PAM_ACOUSTIC ? launch_forward<kAcoustic>(t, blocks, smem, s)
-                : cfg.approximation == PAM_VTI      ? launch_forward<kVTI>(t, blocks, smem, s)
-                                                    : launch_forward<kTTI>(t, blocks, smem, s);
+        if (err == cudaSuccess && p.halo == 8) {
+            TileCpmlArgs c{};
+            c.r.f = t;
+            c.mem[0] = d_tile_mem[0];
+            c.mem[1] = d_tile_mem[1];
+            c.cxab = d_cxab;
+            c.czab = d_czab;
+            err = cfg.approximation == PAM_ACOUSTIC ? ::launch_cpml<kAcoustic, kTileForwardRole>(c, blocks, smem, s)
+                                                    : ::launch_cpml<kVTI, kTileForwardRole>(c, blocks, smem, s);
+        } else if (err == cudaSuccess) {
+            err = launch_forward<false>(cfg.approximation, t, blocks, smem, s);
+        }
         if (err != cudaSuccess) return fail(PAM_E_CUDA, "cooperative launch failed: %s", cudaGetErrorString(err));
     }
     // every group of T steps publishes into the other set
-    if (!slots) tile_set ^= ((k1 - k0 + p.T - 1) / p.T) & 1;
+    if (!slots || p.halo == 8) tile_set ^= ((k1 - k0 + p.T - 1) / p.T) & 1;
+    return PAM_OK;
+}
+
+// Steps t = k1-1 .. k0 of the source field backwards in time, undamped, from
+// S(k1-1), S(k1) in the slots to S(k0-1): with the random border (its kappa) or
+// the saved bands written over each new field.
+int pam_engine::tile_reverse(const TilePlan& p, int nshots, int k0, int k1, cudaStream_t s, float* slots, int kslot,
+                             const float* kap, bool bands) {
+    if (k1 <= k0) return PAM_OK;
+    TileArgs t = tile_args(p, nshots);
+    t.s.kap = kap;
+    t.s.cerjan = nullptr;
+    t.k0 = k0;
+    t.k1 = k1;
+    t.slots = slots;
+    t.kslot = kslot;
+    if (bands) {
+        t.band = d_band;
+        t.band_scale = d_band_scale;
+        t.band_store = adj_store;
+        t.nzi = cfg.nz;
+        t.nxi = cfg.nx;
+    }
+    const size_t smem = smem_of(t.g, cfg.approximation, kTileReverse);
+    for (int b = 0; b < nshots; b += p.group) {
+        t.shot0 = b;
+        const int blocks = std::min(p.group, nshots - b) * p.nty * p.ntx;
+        cudaError_t err = cudaMemsetAsync(d_tile_bar, 0, sizeof(unsigned), s);
+        if (err == cudaSuccess) err = launch_forward<true>(cfg.approximation, t, blocks, smem, s);
+        if (err != cudaSuccess) return fail(PAM_E_CUDA, "cooperative launch failed: %s", cudaGetErrorString(err));
+    }
+    return PAM_OK;
+}
+
+// Steps 0 .. nt-1 of the source field with the random border, undamped, from
+// d_u[0], d_u[1]; leaves U(nt - 1), U(nt) in the two field buffers.
+int pam_engine::tile_undamped(const TilePlan& p, int nshots, const float* kap, cudaStream_t s) {
+    pam_engine* e = this;
+    TileArgs t = tile_args(p, nshots);
+    t.ex[0][0] = d_u[0];
+    t.ex[0][1] = d_u[1];
+    t.ex[1][0] = d_tile[0];
+    t.ex[1][1] = d_tile[1];
+    t.s.kap = kap;
+    t.s.cerjan = nullptr;
+    t.k1 = cfg.nt;
+    const size_t smem = smem_of(t.g, cfg.approximation, kTileReverse);
+    for (int b = 0; b < nshots; b += p.group) {
+        t.shot0 = b;
+        const int blocks = std::min(p.group, nshots - b) * p.nty * p.ntx;
+        cudaError_t err = cudaMemsetAsync(d_tile_bar, 0, sizeof(unsigned), s);
+        if (err == cudaSuccess) err = launch_forward<false>(cfg.approximation, t, blocks, smem, s);
+        if (err != cudaSuccess) return fail(PAM_E_CUDA, "cooperative launch failed: %s", cudaGetErrorString(err));
+    }
+    // from the set that holds the state: U(nt) into d_u[nt & 1], U(nt - 1) into the other
+    const bool second = ((cfg.nt + p.T - 1) / p.T) & 1;
+    const size_t bytes = (size_t)shot_stride * nshots * 4;
+    const float* cur = second ? d_tile[0] : d_u[0];
+    const float* prev = second ? d_tile[1] : d_u[1];
+    if (!second && (cfg.nt & 1)) {   // in the field buffers, the wrong way round
+        CU(cudaMemcpyAsync(d_tile[0], d_u[0], bytes, cudaMemcpyDeviceToDevice, s));
+        cur = d_tile[0];
+    }
+    if (prev != d_u[(cfg.nt + 1) & 1])
+        CU(cudaMemcpyAsync(d_u[(cfg.nt + 1) & 1], prev, bytes, cudaMemcpyDeviceToDevice, s));
+    if (cur != d_u[cfg.nt & 1]) CU(cudaMemcpyAsync(d_u[cfg.nt & 1], cur, bytes, cudaMemcpyDeviceToDevice, s));
     return PAM_OK;
 }
 
@@ -310,7 +440,7 @@ int pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, cons
             tile_inject_ok = h_rz[i] >= 4 && h_rz[i] < nza - 4 && h_rx[i] >= 4 && h_rx[i] < nxa - 4;
         for (int l = 0; l < lists * nt && tile_inject_ok; l++) {
             const int tile = l % nt;
-            const int ez0 = 4 + (tile / p->ntx) * p->TZ - 4 * p->T, ex0 = 4 + (tile % p->ntx) * p->TX - 4 * p->T;
+            const int ez0 = 4 + (tile / p->ntx) * p->TZ - p->halo * p->T, ex0 = 4 + (tile % p->ntx) * p->TX - p->halo * p->T;
             for (auto& v : of) v.clear();
             for (int r = 0; r < nrec; r++) {
                 const size_t i = (size_t)(l / nt) * nrec + r;
@@ -357,6 +487,11 @@ int pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, cons
         if (!d && dalloc_bytes((void**)&d, field * 4)) return PAM_E_CUDA;
     if (!d_tile_bar && dalloc_bytes((void**)&d_tile_bar, 128)) return PAM_E_CUDA;
     for (float* d : d_tile_sum) CU(cudaMemsetAsync(d, 0, (size_t)shot_stride * nshots * 4, s));
+    if (p->halo == 8) {
+        for (float*& d : d_tile_bmem)
+            if (!d && dalloc_bytes((void**)&d, 4 * field * 4)) return PAM_E_CUDA;
+        CU(cudaMemsetAsync(d_tile_bmem[0], 0, 4 * field * 4, s));
+    }
     tile_bset = 0;
     *out = p;
     return PAM_OK;
@@ -375,7 +510,6 @@ int pam_engine::tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0,
     t.f.k0 = k0;
     t.f.k1 = k1;
     t.f.slots = const_cast<float*>(slots);
-    t.f.slot_stride = shot_stride * B;
     t.f.kslot = kslot;
     t.inj_beg = d_inj_beg;
     t.inj_ent = d_inj_ent;
@@ -388,9 +522,18 @@ int pam_engine::tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0,
         t.f.shot0 = b;
         const int blocks = std::min(p.group, nshots - b) * p.nty * p.ntx;
         cudaError_t err = cudaMemsetAsync(d_tile_bar, 0, sizeof(unsigned), s);
-        if (err == cudaSuccess)
+        if (err == cudaSuccess && p.halo == 8) {
+            TileCpmlArgs c{};
+            c.r = t;
+            c.mem[0] = d_tile_bmem[0];
+            c.mem[1] = d_tile_bmem[1];
+            c.cxab = d_cxab;
+            c.czab = d_czab;
+            err = ::launch_cpml<kAcoustic, kTileRtmRole>(c, blocks, smem, s);
+        } else if (err == cudaSuccess) {
             err = job == kTileExactJob ? launch_adjoint<kTileExact>(t, blocks, smem, s)
                                        : launch_adjoint<kTileRtm>(t, blocks, smem, s);
+        }
         if (err != cudaSuccess) return fail(PAM_E_CUDA, "cooperative launch failed: %s", cudaGetErrorString(err));
     }
     tile_bset ^= ((k1 - k0 + p.T - 1) / p.T) & 1;

@@ -28,6 +28,7 @@
 // TTI 381 x 681 3.1 against 7.3.  At 1.4 us a step the 301 x 501 tile spends
 // about 0.65 us a step in the exchange and issues 28% of the cycles.
 #pragma once
+#include "pam_band.cuh"
 #include "pam_kernels.cuh"
 
 namespace pam {
@@ -48,6 +49,7 @@ struct TileShape {
     int T;              // steps between barriers
     int TZ, TX;         // cells of a tile (TX a multiple of 4)
     int nty, ntx;       // tiles of one shot
+    int halo;           // cells that a step's region loses on each side: 4, with CPML strips 8
     int R;              // rows per thread
     int nrg, EXq;       // row groups and quads of a tile with its halo
 };
@@ -80,6 +82,14 @@ struct TileArgs {
     float* slots;
     long long slot_stride;
     int kslot;
+    int mem_shots;                       // shots of the memory variables' arrays (CPML)
+    // the source field backwards in time (with slots, undamped, kTileReverse): the
+    // state before step k1-1 is S(k1-1), S(k1); step t gives
+    // S(t-1) = 2 S(t) - S(t+1) + kappa L S(t) + w(t+1), down to S(k0-1), with the
+    // saved band of time t-1 written over it (band == nullptr: none)
+    const void* band;                    // [nt-1][B][nb] in the storage type
+    const float* __restrict__ band_scale;   // [nt-1][B][chunks]
+    int band_store, nzi, nxi;
 };
 
 // Grid-wide barrier of resident blocks: each block's writes before it are
@@ -109,6 +119,12 @@ __device__ __forceinline__ float4 tile_fetch(const float* src, int z, int x, int
     return __ldcg(reinterpret_cast<const float4*>(PAM_CHK(src + (long long)z * P + x, base, bytes, 16, 100)));
 }
 
+// A quad that another block published, at a cell of the update region.
+__device__ __forceinline__ float4 tile_halo(const float* p, [[maybe_unused]] const void* base,
+                                            [[maybe_unused]] long long bytes) {
+    return __ldcg(reinterpret_cast<const float4*>(PAM_CHK(p, base, bytes, 16, 104)));
+}
+
 // What a thread owns, worked out once per launch.
 template <int R>
 struct TileCells {
@@ -127,8 +143,8 @@ __device__ __forceinline__ TileCells<R> tile_cells(const StepArgs& a, const Tile
     const int z1 = min(z0 + g.TZ, a.nz - 4), x1 = min(x0 + g.TX, a.nx - 4);
     const int rg = threadIdx.x / g.EXq, q = threadIdx.x - rg * g.EXq;
     TileCells<R> c;
-    c.z = z0 - 4 * g.T + rg * R;
-    c.x = x0 - 4 * g.T + 4 * q;
+    c.z = z0 - g.halo * g.T + rg * R;
+    c.x = x0 - g.halo * g.T + 4 * q;
     c.at = (4 + min(rg, g.nrg - 1) * R) * pitch + q;
     c.need = 1 << 20;
     c.valid = c.mine = 0;
@@ -160,14 +176,21 @@ __device__ __forceinline__ TileCells<R> tile_cells(const StepArgs& a, const Tile
 
 // One step of a thread's cells: out[j] = U(k+1) from cur[j] = U(k), old[j] =
 // U(k-1) and the neighbours' U(k) in the shared copy A.  model(i, j) gives row
-// j of model array i.  For TTI every thread that holds cells of the block
+// j of model array i; strips(j, ...) may add CPML strip terms to the derivatives
+// of row j.  For TTI every thread that holds cells of the block
 // calls it (Z passes the z derivatives on, with a barrier), and out is left
 // alone where the thread is not active.
-template <int APPROX, int R, class Model>
+struct TileNoStrips {
+    template <class W, class D>
+    __device__ __forceinline__ void operator()(int, const W&, D&, D&, D&, D&) const {}
+};
+
+template <int APPROX, int R, class Model, class Strips = TileNoStrips>
 __device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>& t, int pitch,
                                           const float4* __restrict__ A,
                                           float4* __restrict__ Z, bool active, const float4 (&cur)[R],
-                                          const float4 (&old)[R], Model model, float4 (&out)[R]) {
+                                          const float4 (&old)[R], Model model, float4 (&out)[R],
+                                          Strips strips = Strips()) {
     const float4* const col = A + t.at;
     float4 w[R + 8];
 #pragma unroll
@@ -223,6 +246,7 @@ __device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>&
             pxz[0] = d1_pair(W2, W1, pz[1], V1, W3, W0, V4, V0, a.cx1);
             pxz[1] = d1_pair(W3, W2, V4, pz[0], W4, W1, V5, V1, a.cx1);
         }
+        strips(j, w, pxx, pzz, px, pz);
         float4 e4 = kap, n4 = kap, b4 = kap, c4 = kap, s4 = kap;
         if (APPROX != kAcoustic) { e4 = model(1, j); n4 = model(2, j); b4 = model(3, j); }
         if (APPROX == kTTI) { c4 = model(4, j); s4 = model(5, j); }
@@ -255,9 +279,31 @@ __device__ __forceinline__ void tile_step(const StepArgs& a, const TileCells<R>&
         }
 }
 
+// Index of a cell in the list of saved band cells (band_cell's inverse), -1 off
+// the band.
+__device__ __forceinline__ int tile_band_index(int zi, int xi, int nzi, int nxi) {
+    if (zi < 0 || zi >= nzi || xi < 0 || xi >= nxi) return -1;
+    if (zi < 4) return zi * nxi + xi;
+    if (zi >= nzi - 4) return (zi - (nzi - 8)) * nxi + xi;
+    if (xi < 4) return 8 * nxi + (zi - 4) * 4 + xi;
+    if (xi >= nxi - 4) return 8 * nxi + 4 * (nzi - 8) + (zi - 4) * 4 + xi - (nxi - 4);
+    return -1;
+}
+
+// The saved value of band cell i of a shot at time `tt`.
+__device__ __forceinline__ float tile_band_value(const TileArgs& t, int shot, int tt, int i) {
+    const long long nb = band_cells(t.nzi, t.nxi);
+    const long long nchunk = (nb + kBandChunk - 1) / kBandChunk;
+    const long long row = (long long)tt * t.mem_shots + shot;
+    if (t.band_store == 0) return reinterpret_cast<const float*>(t.band)[row * nb + i];
+    const float v = t.band_store == 1 ? band_unpack(reinterpret_cast<const __nv_bfloat16*>(t.band)[row * nb + i])
+                                      : band_unpack(reinterpret_cast<const __half*>(t.band)[row * nb + i]);
+    return v * t.band_scale[row * nchunk + i / kBandChunk];
+}
+
 // Forward time loop, steps k0 .. k1-1, of the shots shot0 .. (one block per
 // tile of each): see the head of the file.
-template <int APPROX, int R>
+template <int APPROX, int R, bool REVERSE = false>
 __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const TileArgs t)
 {
     extern __shared__ float4 tsm[];
@@ -278,12 +324,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
     [[maybe_unused]] const long long fbytes = (long long)a.B * a.shot_stride * 4;
     [[maybe_unused]] const long long mbytes = (long long)a.nz * a.P * 4;
 
+    constexpr int dir = REVERSE ? -1 : 1;
+
     // the state and the models of the thread's cells
     float4 cur[R], old[R], kap[R];
     {
         for (int i = tid; i < ncopy * copy; i += nthr) tsm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* const in0 = t.slots ? t.slots + (t.k0 - t.kslot) * t.slot_stride : t.set0 ? t.ex[1][0] : t.ex[0][0];
-        const float* const in1 = t.slots ? in0 - t.slot_stride : t.set0 ? t.ex[1][1] : t.ex[0][1];
+        const float* const in0 = t.slots ? t.slots + ((REVERSE ? t.k1 - 1 : t.k0) - t.kslot) * t.slot_stride
+                                 : t.set0 ? t.ex[1][0] : t.ex[0][0];
+        const float* const in1 = t.slots ? in0 - dir * t.slot_stride : t.set0 ? t.ex[1][1] : t.ex[0][1];
         const float* const mod[6] = {a.kap, a.e2, a.m1, a.m2, a.cth, a.sth};
 #pragma unroll
         for (int j = 0; j < R; j++) {
@@ -314,7 +363,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
     // factors, x then z, as in the one-step kernels' recording
     const int rl = t.rec.per_shot ? shot * ntiles + tile : tile;
     const int rb = t.rec.seis ? t.rec_beg[rl] : 0, re = t.rec.seis ? t.rec_beg[rl + 1] : 0;
-    const int ez0 = 4 + (tile / g.ntx) * g.TZ - 4 * g.T - 4, ex0 = 4 + (tile % g.ntx) * g.TX - 4 * g.T;
+    const int ez0 = 4 + (tile / g.ntx) * g.TZ - g.halo * g.T - 4, ex0 = 4 + (tile % g.ntx) * g.TX - g.halo * g.T;
     [[maybe_unused]] const long long sbytes = (long long)a.B * t.rec.nt_data * t.rec.nrec * 4;
     float* const seis = t.rec.seis + (long long)shot * t.rec.nt_data * t.rec.nrec;
     auto place = [&](int2 e, int& off, float& fx, float& fz) {
@@ -337,15 +386,41 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
     }
     __syncthreads();
 
-    int k = t.k0, set = t.set0;
+    int k = REVERSE ? t.k1 - 1 : t.k0, left = t.k1 - t.k0, set = t.set0;
     unsigned want = 0;
     const long long o = so + (long long)own.z * a.P + own.x;   // the thread's first cell in a field
     float amp = k + 1 < t.nt ? t.wavelet[k + 1] : 0.0f;
-    while (k < t.k1) {
-        const int nsub = min(g.T, t.k1 - k);
-        for (int s = 0; s < nsub; s++, k++) {
-            const float next_amp = k + 2 < t.nt ? t.wavelet[k + 2] : 0.0f;
-            if (k >= t.itlag) {
+    // rows with cells of the saved band, and their values at the next time
+    unsigned brow = 0;
+    float4 bval[REVERSE ? R : 1];
+    auto band_fetch = [&](int tt) {
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (REVERSE && (brow >> j & 1u) && tt >= 0) {
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int c = tile_band_index(own.z + j - a.N, own.x + i - a.N, t.nzi, t.nxi);
+                    if (c >= 0) v[i] = tile_band_value(t, shot, tt, c);
+                }
+                bval[j] = make_float4(v[0], v[1], v[2], v[3]);
+            }
+    };
+    if (REVERSE && t.band) {
+#pragma unroll
+        for (int j = 0; j < R; j++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if ((own.valid >> j & 1u) && tile_band_index(own.z + j - a.N, own.x + i - a.N, t.nzi, t.nxi) >= 0)
+                    brow |= 1u << j;
+        band_fetch(k - 1);
+    }
+    while (left > 0) {
+        const int nsub = min(g.T, left);
+        for (int s = 0; s < nsub; s++, k += dir, left--) {
+            const int kn = k + dir + 1;
+            const float next_amp = kn < t.nt && kn >= 0 ? t.wavelet[kn] : 0.0f;
+            if (!REVERSE && k >= t.itlag) {
                 if (rr >= 0) sample(k - t.itlag, rr, roff, rfx, rfz);
                 for (int i = rb + tid + nthr; i < re; i += nthr) {
                     const int2 e = t.rec_ent[i];
@@ -369,6 +444,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
                             out[j].z += sx == own.x + 2 ? amp : 0.f;
                             out[j].w += sx == own.x + 3 ? amp : 0.f;
                         }
+                if (REVERSE && brow)
+#pragma unroll
+                    for (int j = 0; j < R; j++)
+                        if (brow >> j & 1u) {
+                            const int zi = own.z + j - a.N, xi = own.x - a.N;
+                            if (tile_band_index(zi, xi, t.nzi, t.nxi) >= 0) out[j].x = bval[j].x;
+                            if (tile_band_index(zi, xi + 1, t.nzi, t.nxi) >= 0) out[j].y = bval[j].y;
+                            if (tile_band_index(zi, xi + 2, t.nzi, t.nxi) >= 0) out[j].z = bval[j].z;
+                            if (tile_band_index(zi, xi + 3, t.nzi, t.nxi) >= 0) out[j].w = bval[j].w;
+                        }
 #pragma unroll
                 for (int j = 0; j < R; j++) {
                     old[j] = cur[j];
@@ -376,31 +461,32 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
                     B[own.at + j * kTilePitch] = out[j];
                 }
             }
+            if (REVERSE && brow) band_fetch(k - 2);
             float4* const sw = A;
             A = B;
             B = sw;
             amp = next_amp;
             if (t.slots && own.mine) {
-                float* const u = t.slots + (k + 1 - t.kslot) * t.slot_stride;
+                float* const u = t.slots + (k + dir - t.kslot) * t.slot_stride;
 #pragma unroll
                 for (int j = 0; j < R; j++)
                     if (own.mine >> j & 1u)
-                        *reinterpret_cast<float4*>(PAM_CHK(u + o + (long long)j * a.P, u, fbytes, 16, 105)) = cur[j];
+                        *reinterpret_cast<float4*>(PAM_CHK(u + o + j * a.P, u, fbytes, 16, 105)) = cur[j];
             }
             if (s + 1 < nsub) __syncthreads();
         }
         // publish the tile into the other set
         float* const pub0 = t.slots ? t.slots + (k - t.kslot) * t.slot_stride : set ? t.ex[0][0] : t.ex[1][0];
-        float* const pub1 = t.slots ? pub0 - t.slot_stride : set ? t.ex[0][1] : t.ex[1][1];
+        float* const pub1 = t.slots ? pub0 - dir * t.slot_stride : set ? t.ex[0][1] : t.ex[1][1];
         if (!t.slots)
 #pragma unroll
             for (int j = 0; j < R; j++)
                 if (own.mine >> j & 1u) {
-                    *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + (long long)j * a.P, pub0, fbytes, 16, 103)) = cur[j];
-                    *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + (long long)j * a.P, pub1, fbytes, 16, 103)) = old[j];
+                    *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + j * a.P, pub0, fbytes, 16, 103)) = cur[j];
+                    *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + j * a.P, pub1, fbytes, 16, 103)) = old[j];
                 }
         set ^= 1;
-        if (k >= t.k1) break;
+        if (left <= 0) break;
         want += gridDim.x;
         if (!tile_barrier(t.bar, want, t.status, &alive)) return;
         // the halo, both fields, from the other tiles
@@ -409,8 +495,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
 #pragma unroll
             for (int j = 0; j < R; j++)
                 if (halo >> j & 1u) {
-                    cur[j] = tile_fetch(pub0 + so, own.z + j, own.x, a.nz, a.P, pub0, fbytes);
-                    old[j] = tile_fetch(pub1 + so, own.z + j, own.x, a.nz, a.P, pub1, fbytes);
+                    cur[j] = tile_halo(pub0 + o + j * a.P, pub0, fbytes);
+                    old[j] = tile_halo(pub1 + o + j * a.P, pub1, fbytes);
                 }
 #pragma unroll
             for (int j = 0; j < R; j++)
@@ -500,7 +586,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_adjoint_kernel(const Til
             float4* const dst = ring + (tt & (kTileRing - 1)) * copy + own.at;
 #pragma unroll
             for (int j = 0; j < R; j++)
-                if (own.valid >> j & 1u) cp_async16(dst + j * pitch, PAM_CHK(u + o + (long long)j * a.P, u, fbytes, 16, 110));
+                if (own.valid >> j & 1u) cp_async16(dst + j * pitch, PAM_CHK(u + o + j * a.P, u, fbytes, 16, 110));
         }
         cp_async_commit();
     };
@@ -649,8 +735,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_adjoint_kernel(const Til
 #pragma unroll
         for (int j = 0; j < R; j++)
             if (own.mine >> j & 1u) {
-                *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + (long long)j * a.P, pub0, fbytes, 16, 111)) = cur[j];
-                *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + (long long)j * a.P, pub1, fbytes, 16, 111)) = old[j];
+                *reinterpret_cast<float4*>(PAM_CHK(pub0 + o + j * a.P, pub0, fbytes, 16, 111)) = cur[j];
+                *reinterpret_cast<float4*>(PAM_CHK(pub1 + o + j * a.P, pub1, fbytes, 16, 111)) = old[j];
             }
         set ^= 1;
         if (k < t.k0) break;
@@ -662,8 +748,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_adjoint_kernel(const Til
 #pragma unroll
             for (int j = 0; j < R; j++)
                 if (halo >> j & 1u) {
-                    cur[j] = tile_fetch(pub0 + so, own.z + j, own.x, a.nz, a.P, pub0, fbytes);
-                    old[j] = tile_fetch(pub1 + so, own.z + j, own.x, a.nz, a.P, pub1, fbytes);
+                    cur[j] = tile_halo(pub0 + o + j * a.P, pub0, fbytes);
+                    old[j] = tile_halo(pub1 + o + j * a.P, pub1, fbytes);
                 }
 #pragma unroll
             for (int j = 0; j < R; j++)
@@ -678,6 +764,512 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_adjoint_kernel(const Til
             *reinterpret_cast<float4*>(PAM_CHK(ta.gsum + o + (long long)j * a.P, ta.gsum, fbytes, 16, 112)) = G[j * nthr];
             *reinterpret_cast<float4*>(PAM_CHK(ta.isum + o + (long long)j * a.P, ta.isum, fbytes, 16, 112)) = I[j * nthr];
         }
+}
+
+// ---------------------------------------------------------------- CPML
+
+// Steps of a field with the perfectly matched layer as tiles: the forward loop
+// (kTileForwardRole) and the receiver side of acoustic migration (kTileRtmRole,
+// as tile_adjoint_kernel<kTileRtm>).  A step needs the new psi of the strip
+// cells four cells away, hence U eight cells away, so the regions lose eight
+// cells a step; psi goes to the neighbours through two more shared copies
+// (a second barrier per step), zeta stays with its thread in shared memory.
+// Per cell the expressions of the strip kernels and of step_kernel.
+//
+// One shot of 377 x 743 cells takes 10.7 us a step as a graph of four launches
+// (two strip kernels, the step, the recording).
+enum TileRole { kTileForwardRole = 0, kTileRtmRole = 1 };
+
+struct TileCpmlArgs {
+    TileAdjArgs r;                   // r.f: the loop; the rest of r: kTileRtmRole
+    float* mem[2];                   // [set][4][B][nz][P] psi x, zeta x, psi z, zeta z as published; [0] zero before step 0
+    const float2* __restrict__ cxab; // [nz][2N]
+    const float2* __restrict__ czab; // [2N][P]
+};
+
+__host__ __device__ inline size_t tile_cpml_smem_bytes(const TileShape& g, int models, int role) {
+    const size_t copy = (size_t)(g.nrg * g.R + 8) * tile_pitch(g) * 16, rows = (size_t)g.R * tile_threads(g) * 16;
+    return 4 * copy + 6 * rows + (models > 1 ? models * rows : 0) +
+           (role == kTileRtmRole ? 2 * rows + (size_t)kTileInject * (16 + 2 * 4 * g.T) : 0);
+}
+
+// Sums and differences of pairs, each half on its own: the packed forms of a
+// product and a sum that follow each other in straight-line code are contracted
+// into one operation whatever their rounding mode says.  step_kernel's branch
+// around its strip terms and the strip kernels keep them apart here.
+__device__ __forceinline__ float2 add_apart(float2 a, float2 b) {
+    return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+// The recursions of psi and zeta, a old + b v, contracted as in the strip
+// kernels; d1_pair_ref and d2_pair are their derivatives, bit for bit.
+__device__ __forceinline__ float2 cpml_recursion(float2 a, float2 b, float2 old, float2 v) {
+    return pfma2(a, old, pmul2(b, v));
+}
+// Second derivative without its 1/d^2 (d2_pair is this times inv).
+__device__ __forceinline__ float2 d2_pair_sum(float2 c, float2 p1, float2 m1, float2 p2, float2 m2, float2 p3, float2 m3,
+                                              float2 p4, float2 m4) {
+    float2 t = pmul2(bc2(kC0), c);
+    t = pfma2(bc2(kC1), padd2(p1, m1), t);
+    t = pfma2(bc2(kC2), padd2(p2, m2), t);
+    t = pfma2(bc2(kC3), padd2(p3, m3), t);
+    return pfma2(bc2(kC4), padd2(p4, m4), t);
+}
+__device__ __forceinline__ void d2_quad_sum(const float4& l, const float4& c, const float4& r, float2 (&d)[2]) {
+    const float2 P0 = lo2(l), P1 = hi2(l), P2 = lo2(c), P3 = hi2(c), P4 = lo2(r), P5 = hi2(r);
+    const float2 O0 = make_float2(l.y, l.z), O1 = make_float2(l.w, c.x), O2 = make_float2(c.y, c.z);
+    const float2 O3 = make_float2(c.w, r.x), O4 = make_float2(r.y, r.z);
+    d[0] = d2_pair_sum(P2, O2, O1, P3, P1, O3, O0, P4, P0);
+    d[1] = d2_pair_sum(P3, O3, O2, P4, P2, O4, O1, P5, P1);
+}
+// First derivative along x of the two pairs of a quad c with its neighbours l, r.
+__device__ __forceinline__ void d1_quad(const float4& l, const float4& c, const float4& r, float inv, float2 (&d)[2]) {
+    const float2 P0 = lo2(l), P1 = hi2(l), P2 = lo2(c), P3 = hi2(c), P4 = lo2(r), P5 = hi2(r);
+    const float2 O0 = make_float2(l.y, l.z), O1 = make_float2(l.w, c.x), O2 = make_float2(c.y, c.z);
+    const float2 O3 = make_float2(c.w, r.x), O4 = make_float2(r.y, r.z);
+    d[0] = d1_pair_ref(O2, O1, P3, P1, O3, O0, P4, P0, inv);
+    d[1] = d1_pair_ref(O3, O2, P4, P2, O4, O1, P5, P1, inv);
+}
+
+// threads of a block at most, by rows per thread: one row in 64 registers, two in 168
+__host__ __device__ constexpr int tile_cpml_threads(int R) { return R == 1 ? 1024 : 384; }
+
+template <int APPROX, int R, int ROLE>
+__global__ void __launch_bounds__(tile_cpml_threads(R), 1) tile_cpml_kernel(const TileCpmlArgs tc)
+{
+    extern __shared__ float4 tsm[];
+    __shared__ int alive;
+    const TileAdjArgs& ta = tc.r;
+    const TileArgs& t = ta.f;
+    const StepArgs& a = t.s;
+    const TileShape& g = t.g;
+    const int ntiles = g.nty * g.ntx;
+    const int shot = t.shot0 + blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
+    const int tid = threadIdx.x, nthr = blockDim.x, pitch = tile_pitch(g);
+    const TileCells<R> own = tile_cells<R>(a, g, tile, pitch);
+    const int copy = (g.nrg * R + 8) * pitch;
+    float4* A = tsm;                               // U(k)
+    float4* B = tsm + copy;                        // U(k+1)
+    float4* __restrict__ const PX = tsm + 2 * copy;             // psi of the x strips, of the z strips
+    float4* __restrict__ const PZ = tsm + 3 * copy;
+    float4* __restrict__ const ZX = tsm + 4 * copy + tid;       // [R] zeta of the thread's cells
+    float4* __restrict__ const ZZ = ZX + R * nthr;
+    float4* __restrict__ const AX = ZZ + R * nthr;              // [R] (a, b) of the thread's cells, zero off the strips
+    float4* __restrict__ const BX = AX + R * nthr;
+    float4* __restrict__ const AZ = BX + R * nthr;
+    float4* __restrict__ const BZ = AZ + R * nthr;
+    float4* const M = BZ + R * nthr;               // models (not acoustic)
+    constexpr int nmod = APPROX == kAcoustic ? 0 : tile_models<APPROX>();
+    float4* const G = M + nmod * R * nthr;         // kTileRtmRole: the sums, the entries and the staged data
+    float4* const I = G + R * nthr;
+    float4* const ient = I + R * nthr - tid;
+    float* const idat = reinterpret_cast<float*>(ient + kTileInject);
+    const long long so = (long long)shot * a.shot_stride;
+    const long long o = so + (long long)own.z * a.P + own.x;
+    [[maybe_unused]] const long long fbytes = (long long)a.B * a.shot_stride * 4;
+    [[maybe_unused]] const long long mbytes = (long long)a.nz * a.P * 4;
+    const long long mstride = (long long)t.mem_shots * a.shot_stride;
+
+    // which of the thread's cells lie in a strip
+    unsigned xin = 0;                              // columns
+    unsigned zin = 0;                              // rows
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int x = own.x + i;
+        if ((x >= 4 && x < a.N) || (x >= a.nx - a.N && x < a.nx - 4)) xin |= 1u << i;
+    }
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const int z = own.z + j;
+        if ((own.valid >> j & 1u) && (z < a.N || z >= a.nz - a.N)) zin |= 1u << j;
+    }
+    if (!own.valid) xin = 0;
+    // acoustic: rows that step_kernel takes in its march without border code (a
+    // 128-column tile and an 8-row segment, the height that small batches run
+    // with, clear of the border), where its sum of the two second derivatives
+    // takes the x one's scaling with it in one operation; elsewhere the branch
+    // around the strip terms keeps the two apart
+    unsigned inner = 0;
+    if (APPROX == kAcoustic) {
+        const int tx = own.x / kTileWide * kTileWide - 4;
+        if (own.valid && tx >= a.N && tx + kTileWide + 8 <= a.nx - a.N)
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                const int z = 4 + (own.z + j - 4) / 8 * 8;
+                if ((own.valid >> j & 1u) && z >= a.N && min(z + 8, a.nz - 4) <= a.nz - a.N) inner |= 1u << j;
+            }
+    }
+
+    float4 cur[R], old[R], kap[R];
+    for (int i = tid; i < 4 * copy; i += nthr) tsm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    {
+        const float* const in0 = t.slots && ROLE == kTileForwardRole ? t.slots + (t.k0 - t.kslot) * t.slot_stride
+                                 : t.set0                            ? t.ex[1][0] : t.ex[0][0];
+        const float* const in1 = t.slots && ROLE == kTileForwardRole ? in0 - t.slot_stride
+                                 : t.set0                            ? t.ex[1][1] : t.ex[0][1];
+        const float* const mod[6] = {a.kap, a.e2, a.m1, a.m2, a.cth, a.sth};
+        const float* const mem = t.set0 ? tc.mem[1] : tc.mem[0];
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int z = own.valid >> j & 1u ? own.z + j : -1;
+            cur[j] = tile_fetch(in0 + so, z, own.x, a.nz, a.P, in0, fbytes);
+            old[j] = tile_fetch(in1 + so, z, own.x, a.nz, a.P, in1, fbytes);
+            kap[j] = tile_fetch(a.kap, z, own.x, a.nz, a.P, a.kap, mbytes);
+            if (APPROX != kAcoustic)
+#pragma unroll
+                for (int i = 0; i < tile_models<APPROX>(); i++)
+                    M[(i * R + j) * nthr] = tile_fetch(mod[i], z, own.x, a.nz, a.P, mod[i], mbytes);
+            const int zx = xin ? z : -1, zz = zin >> j & 1u ? z : -1;
+            const float4 px = tile_fetch(mem + so, zx, own.x, a.nz, a.P, mem, fbytes);
+            ZX[j * nthr] = tile_fetch(mem + mstride + so, zx, own.x, a.nz, a.P, mem + mstride, fbytes);
+            const float4 pz = tile_fetch(mem + 2 * mstride + so, zz, own.x, a.nz, a.P, mem + 2 * mstride, fbytes);
+            ZZ[j * nthr] = tile_fetch(mem + 3 * mstride + so, zz, own.x, a.nz, a.P, mem + 3 * mstride, fbytes);
+            if (own.valid) {
+                A[own.at + j * pitch] = cur[j];
+                PX[own.at + j * pitch] = px;
+                PZ[own.at + j * pitch] = pz;
+            }
+            if (ROLE == kTileRtmRole) {
+                G[j * nthr] = tile_fetch(ta.gsum + so, z, own.x, a.nz, a.P, ta.gsum, fbytes);
+                I[j * nthr] = tile_fetch(ta.isum + so, z, own.x, a.nz, a.P, ta.isum, fbytes);
+            }
+        }
+    }
+    auto model = [&](int i, int j) { return APPROX == kAcoustic ? kap[j] : M[(i * R + j) * nthr]; };
+    // (a, b) of the thread's cells; zero off the strips, where psi and zeta stay zero
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        float2 x[4], z[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int xx = own.x + i, zz = own.z + j;
+            const int c = xx < a.N ? xx : xx - (a.nx - 2 * a.N), r = zz < a.N ? zz : zz - (a.nz - 2 * a.N);
+            x[i] = z[i] = make_float2(0.f, 0.f);
+            if ((own.valid >> j & 1u) && (xin >> i & 1u))
+                x[i] = __ldg(PAM_CHK(&tc.cxab[(long long)zz * (2 * a.N) + c], tc.cxab, (long long)a.nz * 2 * a.N * 8, 8, 120));
+            if ((zin >> j & 1u) && xx < a.nx - 4)
+                z[i] = __ldg(PAM_CHK(&tc.czab[(long long)r * a.P + xx], tc.czab, (long long)2 * a.N * a.P * 8, 8, 121));
+        }
+        AX[j * nthr] = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+        BX[j * nthr] = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+        AZ[j * nthr] = make_float4(z[0].x, z[1].x, z[2].x, z[3].x);
+        BZ[j * nthr] = make_float4(z[0].y, z[1].y, z[2].y, z[3].y);
+    }
+
+    // source and recording (kTileForwardRole), as in tile_forward_kernel
+    int sz = 0, sx = 0, srow = 0, rb = 0, re = 0, roff = 0, rr = -1;
+    bool has_src = false;
+    const int ez0 = 4 + (tile / g.ntx) * g.TZ - g.halo * g.T - 4, ex0 = 4 + (tile % g.ntx) * g.TX - g.halo * g.T;
+    [[maybe_unused]] const long long sbytes = (long long)a.B * t.rec.nt_data * t.rec.nrec * 4;
+    float* const seis = t.rec.seis + (long long)shot * t.rec.nt_data * t.rec.nrec;
+    auto place = [&](int2 e) { return ((e.x >> 16) - ez0) * (4 * pitch) + (e.x & 0xffff) - ex0; };
+    auto sample = [&](int it, int r, int off) {
+        const float v = reinterpret_cast<const float*>(A)[off];
+        *PAM_CHK(&seis[(long long)it * t.rec.nrec + r], t.rec.seis, sbytes, 4, 122) = v;
+        if (!isfinite(v)) atomicOr(t.status, 1);
+    };
+    if (ROLE == kTileForwardRole) {
+        sz = *PAM_CHK(&a.src_z[shot], a.src_z, a.B * 4, 4, 101);
+        sx = *PAM_CHK(&a.src_x[shot], a.src_x, a.B * 4, 4, 101);
+        srow = sz - own.z;
+        has_src = own.valid && srow >= 0 && srow < R && (own.valid >> srow & 1u) && sx >= own.x && sx < own.x + 4 &&
+                  sx < a.nx - 4;
+        const int rl = t.rec.per_shot ? shot * ntiles + tile : tile;
+        rb = t.rec.seis ? t.rec_beg[rl] : 0;
+        re = t.rec.seis ? t.rec_beg[rl + 1] : 0;
+        if (rb + tid < re) {
+            const int2 e = t.rec_ent[rb + tid];
+            rr = e.y;
+            roff = place(e);
+        }
+    }
+    // the data injected (kTileRtmRole), as in tile_adjoint_kernel
+    int il = 0, nent = 0, ib = 0, ie = 0;
+    const float* const data = ta.data + (long long)shot * t.rec.nt_data * t.rec.nrec;
+    auto stage = [&](int tt, int n, int p) {
+        for (int i = tid; i < nent; i += nthr) {
+            const int r = ta.inj_ent[il + i].y;
+            for (int s = 0; s < n; s++) {
+                const int it = tt - s - 1 - t.itlag;
+                float* const dst = idat + (p * g.T + s) * nent + i;
+                if (it >= 0) cp_async4(dst, data + (long long)it * t.rec.nrec + r);
+                else *dst = 0.0f;
+            }
+        }
+    };
+    float4 pc[R], pn[R];                           // source field U(t) of the tile's cells, and the next one
+    auto fetch_p = [&](int tt, float4 (&p)[R]) {
+        const float* const u = t.slots + (tt - t.kslot) * t.slot_stride;
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            p[j] = tile_fetch(u + so, tt >= t.k0 && (own.mine >> j & 1u) ? own.z + j : -1, own.x, a.nz, a.P, u, fbytes);
+    };
+    int k = ROLE == kTileForwardRole ? t.k0 : t.k1 - 1;
+    constexpr int dir = ROLE == kTileForwardRole ? 1 : -1;
+    int left = t.k1 - t.k0;                        // steps to go
+    if (ROLE == kTileRtmRole) {
+        const long long list = (long long)(t.rec.per_shot ? shot * ntiles + tile : tile) * (nthr + 1);
+        il = ta.inj_beg[list];
+        nent = ta.inj_beg[list + nthr] - il;
+        ib = ta.inj_beg[list + tid] - il;
+        ie = ta.inj_beg[list + tid + 1] - il;
+        for (int i = ib; i < ie; i++) {
+            const int2 e = ta.inj_ent[il + i];
+            ient[i].x = __int_as_float((own.at + ((e.x >> 16) - own.z) * pitch) * 4 + (e.x & 0xffff) - own.x);
+        }
+        stage(k, min(g.T, left), 0);
+        cp_async_commit();
+        fetch_p(k, pc);
+        cp_async_wait<0>();
+    }
+    __syncthreads();
+
+    int set = t.set0, parity = 0;
+    unsigned want = 0;
+    while (left > 0) {
+        const int nsub = min(g.T, left);
+        if (ROLE == kTileRtmRole && left > nsub) {
+            stage(k - nsub, min(g.T, left - nsub), parity ^ 1);
+            cp_async_commit();
+        }
+        for (int s = 0; s < nsub; s++, k += dir, left--) {
+            const int h = g.halo * (nsub - 1 - s);
+            const float amp = ROLE == kTileForwardRole && k + 1 < t.nt ? t.wavelet[k + 1] : 0.0f;
+            if (ROLE == kTileForwardRole && k >= t.itlag) {
+                if (rr >= 0) sample(k - t.itlag, rr, roff);
+                for (int i = rb + tid + nthr; i < re; i += nthr) sample(k - t.itlag, t.rec_ent[i].y, place(t.rec_ent[i]));
+            }
+            if (ROLE == kTileRtmRole) {
+                fetch_p(k - 1, pn);
+                if (own.mine)
+#pragma unroll
+                    for (int j = 0; j < R; j++) {
+                        const float4 p = pc[j], q = I[j * nthr], v = G[j * nthr];
+                        const float2 i0 = pfma2(lo2(p), lo2(p), lo2(q)), i1 = pfma2(hi2(p), hi2(p), hi2(q));
+                        const float2 g0 = pfma2(lo2(cur[j]), lo2(p), lo2(v)), g1 = pfma2(hi2(cur[j]), hi2(p), hi2(v));
+                        I[j * nthr] = make_float4(i0.x, i0.y, i1.x, i1.y);
+                        G[j * nthr] = make_float4(g0.x, g0.y, g1.x, g1.y);
+                    }
+            }
+            const float4* const col = A + own.at;
+            // psi of the strip cells, four cells past the region
+            if (own.need <= h + 4 && (xin | zin)) {
+                if (xin)
+#pragma unroll
+                    for (int j = 0; j < R; j++) {
+                        if (!(own.valid >> j & 1u)) continue;
+                        float2 px[2];
+                        d1_quad(col[j * pitch - 1], cur[j], col[j * pitch + 1], a.inv_dx, px);
+                        const float4 ps = PX[own.at + j * pitch], aa = AX[j * nthr], bb = BX[j * nthr];
+                        const float2 n0 = cpml_recursion(lo2(aa), lo2(bb), lo2(ps), px[0]);
+                        const float2 n1 = cpml_recursion(hi2(aa), hi2(bb), hi2(ps), px[1]);
+                        PX[own.at + j * pitch] = make_float4(n0.x, n0.y, n1.x, n1.y);
+                    }
+                if (zin) {
+                    float4 w[R + 8];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        w[j] = col[(j - 4) * pitch];
+                        w[R + 4 + j] = col[(R + j) * pitch];
+                    }
+#pragma unroll
+                    for (int j = 0; j < R; j++) w[j + 4] = cur[j];
+#pragma unroll
+                    for (int j = 0; j < R; j++) {
+                        if (!(zin >> j & 1u)) continue;
+                        const float4 ps = PZ[own.at + j * pitch], aa = AZ[j * nthr], bb = BZ[j * nthr];
+                        const float2 p0 = d1_pair_ref(lo2(w[j + 5]), lo2(w[j + 3]), lo2(w[j + 6]), lo2(w[j + 2]),
+                                                      lo2(w[j + 7]), lo2(w[j + 1]), lo2(w[j + 8]), lo2(w[j]), a.inv_dz);
+                        const float2 p1 = d1_pair_ref(hi2(w[j + 5]), hi2(w[j + 3]), hi2(w[j + 6]), hi2(w[j + 2]),
+                                                      hi2(w[j + 7]), hi2(w[j + 1]), hi2(w[j + 8]), hi2(w[j]), a.inv_dz);
+                        const float2 n0 = cpml_recursion(lo2(aa), lo2(bb), lo2(ps), p0);
+                        const float2 n1 = cpml_recursion(hi2(aa), hi2(bb), hi2(ps), p1);
+                        PZ[own.at + j * pitch] = make_float4(n0.x, n0.y, n1.x, n1.y);
+                    }
+                }
+            }
+            __syncthreads();
+            if (own.need <= h) {
+                float4 out[R];
+                // the strip terms of a row: zeta, and (d psi, d psi + zeta) added to the derivatives
+                tile_step<APPROX, R>(
+                    a, own, pitch, A, nullptr, true, cur, old, model, out,
+                    [&](int j, const float4 (&w)[R + 8], float2 (&pxx)[2], float2 (&pzz)[2], float2 (&px)[2], float2 (&pz)[2]) {
+                        if (APPROX == kAcoustic && (inner >> j & 1u)) {
+                            float2 s[2];
+                            d2_quad_sum(col[j * pitch - 1], cur[j], col[j * pitch + 1], s);
+#pragma unroll
+                            for (int m = 0; m < 2; m++) {
+                                pxx[m] = pfma2(s[m], bc2(a.inv_dx2), pzz[m]);
+                                pzz[m] = make_float2(0.f, 0.f);
+                            }
+                            return;
+                        }
+                        if (!(xin | zin)) return;
+                        float2 hx[2], hz[2];
+                        hx[0] = hx[1] = hz[0] = hz[1] = make_float2(0.f, 0.f);
+                        if (xin && (own.valid >> j & 1u)) {
+                            float2 d[2];
+                            d1_quad(PX[own.at + j * pitch - 1], PX[own.at + j * pitch], PX[own.at + j * pitch + 1], a.inv_dx, d);
+                            const float4 zo = ZX[j * nthr], aa = AX[j * nthr], bb = BX[j * nthr];
+                            const float2 z0 = cpml_recursion(lo2(aa), lo2(bb), lo2(zo), add_apart(pxx[0], d[0]));
+                            const float2 z1 = cpml_recursion(hi2(aa), hi2(bb), hi2(zo), add_apart(pxx[1], d[1]));
+                            ZX[j * nthr] = make_float4(z0.x, z0.y, z1.x, z1.y);
+                            // (psi's derivative reaches past the strip, its term does not)
+                            if (!(xin & 1u)) d[0].x = 0.f;
+                            if (!(xin & 2u)) d[0].y = 0.f;
+                            if (!(xin & 4u)) d[1].x = 0.f;
+                            if (!(xin & 8u)) d[1].y = 0.f;
+                            hx[0] = add_apart(d[0], z0);
+                            hx[1] = add_apart(d[1], z1);
+                            if (APPROX != kAcoustic) {
+                                px[0] = add_apart(px[0], d[0]);
+                                px[1] = add_apart(px[1], d[1]);
+                            }
+                        }
+                        if (zin >> j & 1u) {
+                            float4 q[8];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                q[i] = PZ[own.at + (j - 4 + i) * pitch];
+                                q[4 + i] = PZ[own.at + (j + 1 + i) * pitch];
+                            }
+                            const float2 d0 = d1_pair_ref(lo2(q[4]), lo2(q[3]), lo2(q[5]), lo2(q[2]), lo2(q[6]), lo2(q[1]),
+                                                          lo2(q[7]), lo2(q[0]), a.inv_dz);
+                            const float2 d1 = d1_pair_ref(hi2(q[4]), hi2(q[3]), hi2(q[5]), hi2(q[2]), hi2(q[6]), hi2(q[1]),
+                                                          hi2(q[7]), hi2(q[0]), a.inv_dz);
+                            const float2 s0 = d2_pair_sum(lo2(w[j + 4]), lo2(w[j + 5]), lo2(w[j + 3]), lo2(w[j + 6]),
+                                                          lo2(w[j + 2]), lo2(w[j + 7]), lo2(w[j + 1]), lo2(w[j + 8]), lo2(w[j]));
+                            const float2 s1 = d2_pair_sum(hi2(w[j + 4]), hi2(w[j + 5]), hi2(w[j + 3]), hi2(w[j + 6]),
+                                                          hi2(w[j + 2]), hi2(w[j + 7]), hi2(w[j + 1]), hi2(w[j + 8]), hi2(w[j]));
+                            const float4 zo = ZZ[j * nthr], aa = AZ[j * nthr], bb = BZ[j * nthr];
+                            const float2 z0 = cpml_recursion(lo2(aa), lo2(bb), lo2(zo), pfma2(s0, bc2(a.inv_dz2), d0));
+                            const float2 z1 = cpml_recursion(hi2(aa), hi2(bb), hi2(zo), pfma2(s1, bc2(a.inv_dz2), d1));
+                            ZZ[j * nthr] = make_float4(z0.x, z0.y, z1.x, z1.y);
+                            hz[0] = add_apart(d0, z0);
+                            hz[1] = add_apart(d1, z1);
+                            if (APPROX != kAcoustic) {
+                                pz[0] = add_apart(pz[0], d0);
+                                pz[1] = add_apart(pz[1], d1);
+                            }
+                        }
+#pragma unroll
+                        for (int m = 0; m < 2; m++) {
+                            if (APPROX == kAcoustic) {
+                                pxx[m] = add_apart(pxx[m], pzz[m]);
+                                pzz[m] = add_apart(hx[m], hz[m]);
+                            } else {
+                                pxx[m] = add_apart(pxx[m], hx[m]);
+                                pzz[m] = add_apart(pzz[m], hz[m]);
+                            }
+                        }
+                    });
+                if (has_src)
+#pragma unroll
+                    for (int j = 0; j < R; j++)
+                        if (j == srow) {
+                            out[j].x += sx == own.x ? amp : 0.f;
+                            out[j].y += sx == own.x + 1 ? amp : 0.f;
+                            out[j].z += sx == own.x + 2 ? amp : 0.f;
+                            out[j].w += sx == own.x + 3 ? amp : 0.f;
+                        }
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    old[j] = cur[j];
+                    cur[j] = out[j];
+                    B[own.at + j * pitch] = out[j];
+                }
+                if (ROLE == kTileRtmRole && ie > ib) {
+                    const float* const d = idat + (parity * g.T + s) * nent;
+                    for (int i = ib; i < ie; i++) {
+                        float* const p = reinterpret_cast<float*>(B) + __float_as_int(ient[i].x);
+                        *p = __fadd_rn(*p, __fmul_rn(d[i], ta.scale));
+                    }
+#pragma unroll
+                    for (int j = 0; j < R; j++) cur[j] = B[own.at + j * pitch];
+                }
+            }
+            float4* const sw = A;
+            A = B;
+            B = sw;
+            if (ROLE == kTileRtmRole)
+#pragma unroll
+                for (int j = 0; j < R; j++) pc[j] = pn[j];
+            if (ROLE == kTileForwardRole && t.slots && own.mine) {
+                float* const u = t.slots + (k + 1 - t.kslot) * t.slot_stride;
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                    if (own.mine >> j & 1u)
+                        *reinterpret_cast<float4*>(PAM_CHK(u + o + j * a.P, u, fbytes, 16, 123)) = cur[j];
+            }
+            if (s + 1 < nsub) __syncthreads();
+        }
+        parity ^= 1;
+        // publish the tile: fields (unless the slots hold them) and memory variables
+        const bool slots = ROLE == kTileForwardRole && t.slots;
+        float* const pub0 = slots ? t.slots + (k - t.kslot) * t.slot_stride : set ? t.ex[0][0] : t.ex[1][0];
+        float* const pub1 = slots ? pub0 - t.slot_stride : set ? t.ex[0][1] : t.ex[1][1];
+        float* const pubm = set ? tc.mem[0] : tc.mem[1];
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (own.mine >> j & 1u) {
+                const long long c = o + j * a.P;
+                auto put = [&](float* base, float4 v) {
+                    *reinterpret_cast<float4*>(PAM_CHK(base + c, base, fbytes, 16, 124)) = v;
+                };
+                if (!slots) {
+                    put(pub0, cur[j]);
+                    put(pub1, old[j]);
+                }
+                if (xin) {
+                    put(pubm, PX[own.at + j * pitch]);
+                    put(pubm + mstride, ZX[j * nthr]);
+                }
+                if (zin >> j & 1u) {
+                    put(pubm + 2 * mstride, PZ[own.at + j * pitch]);
+                    put(pubm + 3 * mstride, ZZ[j * nthr]);
+                }
+            }
+        set ^= 1;
+        if (left <= 0) break;
+        if (ROLE == kTileRtmRole) cp_async_wait<0>();
+        want += gridDim.x;
+        if (!tile_barrier(t.bar, want, t.status, &alive)) return;
+        const unsigned halo = own.valid & ~own.mine;
+        if (halo) {
+            float4 px[R], pz[R];
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (halo >> j & 1u) {
+                    const float* const m = pubm + o + j * a.P;
+                    cur[j] = tile_halo(pub0 + o + j * a.P, pub0, fbytes);
+                    old[j] = tile_halo(pub1 + o + j * a.P, pub1, fbytes);
+                    if (xin) {
+                        px[j] = tile_halo(m, pubm, fbytes);
+                        ZX[j * nthr] = tile_halo(m + mstride, pubm + mstride, fbytes);
+                    }
+                    if (zin >> j & 1u) {
+                        pz[j] = tile_halo(m + 2 * mstride, pubm + 2 * mstride, fbytes);
+                        ZZ[j * nthr] = tile_halo(m + 3 * mstride, pubm + 3 * mstride, fbytes);
+                    }
+                }
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (halo >> j & 1u) {
+                    A[own.at + j * pitch] = cur[j];
+                    if (xin) PX[own.at + j * pitch] = px[j];
+                    if (zin >> j & 1u) PZ[own.at + j * pitch] = pz[j];
+                }
+        }
+        __syncthreads();
+    }
+    if (ROLE == kTileRtmRole)
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (own.mine >> j & 1u) {
+                *reinterpret_cast<float4*>(PAM_CHK(ta.gsum + o + (long long)j * a.P, ta.gsum, fbytes, 16, 125)) = G[j * nthr];
+                *reinterpret_cast<float4*>(PAM_CHK(ta.isum + o + (long long)j * a.P, ta.isum, fbytes, 16, 125)) = I[j * nthr];
+            }
 }
 
 }  // namespace pam

@@ -27,11 +27,12 @@ SHAPES = [(8, 8, 8, 40, 0, 1), (9, 11, 8, 37, 5, 3), (61, 133, 12, 61, 11, 2), (
           (40, 50, 10, 1, 0, 1), (90, 61, 20, 97, 30, 9), (201, 401, 50, 53, 10, 1), (401, 1001, 50, 31, 7, 1)]
 
 
-@pytest.mark.parametrize("approx", ["acoustic", "VTI", "TTI"])
+@pytest.mark.parametrize("approx,boundary", [("acoustic", "cerjan"), ("VTI", "cerjan"), ("TTI", "cerjan"),
+                                             ("acoustic", "CPML"), ("VTI", "CPML")])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
-def test_tiles_are_bitwise_the_one_step_launches(approx, shape, monkeypatch):
+def test_tiles_are_bitwise_the_one_step_launches(approx, boundary, shape, monkeypatch):
     nz, nx, N, nt, itlag, shots = shape
-    e, rng = _engine(approx, nz, nx, N, nt, itlag, shots)
+    e, rng = _engine(approx, nz, nx, N, nt, itlag, shots, boundary=boundary)
     nza, nxa = nz + 2 * N, nx + 2 * N
     sz = rng.integers(4, nza - 4, shots).astype(np.int32)
     sx = rng.integers(4, nxa - 4, shots).astype(np.int32)
@@ -56,12 +57,12 @@ def test_tiles_are_bitwise_the_one_step_launches(approx, shape, monkeypatch):
         assert np.array_equal(again[0], one_step[0])
 
 
-@pytest.mark.parametrize("approx", ["acoustic", "TTI"])
-def test_tiles_in_chunks_with_pinned_output(approx):
+@pytest.mark.parametrize("approx,boundary", [("acoustic", "cerjan"), ("TTI", "cerjan"), ("acoustic", "CPML")])
+def test_tiles_in_chunks_with_pinned_output(approx, boundary):
     """A pinned output cuts the loop into launches of a few steps each, which
     hand the state over through either published set."""
     torch = pytest.importorskip("torch")
-    e, rng = _engine(approx, 61, 133, 12, 83, 9, 2)
+    e, rng = _engine(approx, 61, 133, 12, 83, 9, 2, boundary=boundary)
     e.set_receivers(np.full(30, 14, np.int32), np.arange(20, 50, dtype=np.int32))
     sz, sx = np.array([14, 40], np.int32), np.array([30, 90], np.int32)
     ref = e.forward(sz, sx)
@@ -124,3 +125,38 @@ def test_backward_tiles_match_the_one_step_launches(job, shape, monkeypatch):
     e.set_receivers(np.array([0, N + 1, sz[0] + 1], np.int32), np.array([N, N + 2, sx[0]], np.int32))
     d = (1e-2 * rng.standard_normal((shots, nt - itlag, 3))).astype(np.float32)
     close(run(rz, d, 0), run(rz, d, 17))
+
+
+@pytest.mark.parametrize("approx,boundary", [("acoustic", "cerjan"), ("acoustic", "CPML"), ("VTI", "cerjan"), ("TTI", "cerjan")])
+@pytest.mark.parametrize("shape", [(9, 9, 8, 61, 7, 2), (61, 133, 12, 150, 11, 2), (90, 61, 21, 97, 30, 5)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_migration_strategies_as_tiles(approx, boundary, shape, monkeypatch):
+    """Migration with every way of keeping the source field - all steps, bands in
+    each storage format, the random border - as tiles against the one-step
+    launches: the fields are the same bit for bit, the sums in the order of the
+    test above, to the same tolerance (anisotropic images are summed by the same
+    kernel, so they are equal)."""
+    nz, nx, N, nt, itlag, shots = shape
+    e, rng = _engine(approx, nz, nx, N, nt, itlag, shots, boundary=boundary)
+    nza, nxa = nz + 2 * N, nx + 2 * N
+    sz, sx = np.full(shots, nza // 2, np.int32), (N + np.linspace(2, nx - 3, shots)).astype(np.int32)
+    e.set_receivers(np.full(nx - 4, N + 2, np.int32), (N + 2 + np.arange(nx - 4)).astype(np.int32))
+    e.set_random_boundary(400.0, 30.0, 3)
+    d = (1e-2 * rng.standard_normal((shots, nt - itlag, nx - 4))).astype(np.float32)
+    tol = 16 * 2.0 ** -24 * np.sqrt(nt * shots)
+    for K, store in ((0, "f32"), (-1, "f32"), (-1, "bf16"), (-1, "f16"), (-2, "f32"), (19, "f16")):
+        out = []
+        for env in (None, "1"):
+            if env:
+                monkeypatch.setenv("PAM_NO_PERSISTENT", env)
+            e.rtm_reset()
+            e.rtm(sz, sx, d, ckpt_interval=K, store=store)
+            out.append(e.rtm_result(norm="none"))
+            if approx != "acoustic":
+                e.fwi_gradient(sz, sx, d, ckpt_interval=K, store=store)
+                out[-1] += e.fwi_result()
+        monkeypatch.delenv("PAM_NO_PERSISTENT")
+        for x, y in zip(*out):
+            n = np.linalg.norm(y.astype(np.float64))
+            assert np.isfinite(y).all() and n > 0
+            assert np.linalg.norm(x.astype(np.float64) - y) <= (tol * n if approx == "acoustic" else 0.0), (K, store)
