@@ -300,27 +300,57 @@ static bool aniso_operands_aligned(const AnisoArgs& aa, const float* nxt, const 
            aa.g.P % 4 == 0 && aa.g.stride % 4 == 0 && aa.pstride % 4 == 0;
 }
 
-static cudaError_t launch_aniso_adjoint(const AnisoArgs& aa, float* nxt, const float* kap, cudaStream_t s) {
-    if (!aniso_operands_aligned(aa, nxt, kap)) return cudaErrorMisalignedAddress;
-    static bool configured[2][64] = {};
+// Segment height: the warps run in waves of `resident`; a wave marches H rows,
+// eight more for the products around them and some to fill its pipeline.  The
+// number of segments is what is chosen, so that a wave can be filled exactly
+// (8 shots of 901 x 2101: 8 segments of 112 rows are one wave of four blocks
+// per SM).
+static int aniso_height(int B, int ntiles, int rows, int resident) {
+    int best = rows;
+    double least = 1e30;
+    for (int nseg = 1; nseg <= rows; nseg++) {
+        const int h = (rows + nseg - 1) / nseg;
+        if (h < 4 && nseg > 1) break;
+        const long long warps = (long long)B * ntiles * ((rows + h - 1) / h);
+        // a last wave that is not full runs faster, with less contention
+        const double waves = (double)warps / resident, whole = std::floor(waves), part = waves - whole;
+        const double cost = (whole + (part > 0.0 ? 0.7 + 0.3 * part : 0.0)) * (h + 12);
+        if (cost < least) {
+            least = cost;
+            best = h;
+        }
+    }
+    return best;
+}
+
+template <bool TTI>
+static void launch_aniso_t(AnisoArgs aa, float* nxt, const float* kap, cudaStream_t s) {
+    static bool configured[64] = {};
+    static int resident[64] = {};
+    constexpr int smem = aniso_smem_bytes<TTI>();
     int dev = 0;
     cudaGetDevice(&dev);
-    const int smem = aniso_tile_smem_bytes(aa.tti);
-    const dim3 grid((aa.g.nx + kAnTX - 1) / kAnTX, (aa.g.nz + kAnTZ - 1) / kAnTZ, aa.B);
-    const dim3 block(32, 8);
-    if (aa.tti) {
-        if (dev < 0 || dev >= 64 || !configured[1][dev]) {
-            cudaFuncSetAttribute(aniso_adjoint_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (dev >= 0 && dev < 64) configured[1][dev] = true;
-        }
-        aniso_adjoint_tile_kernel<true><<<grid, block, smem, s>>>(aa, nxt, kap);
-    } else {
-        if (dev < 0 || dev >= 64 || !configured[0][dev]) {
-            cudaFuncSetAttribute(aniso_adjoint_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (dev >= 0 && dev < 64) configured[0][dev] = true;
-        }
-        aniso_adjoint_tile_kernel<false><<<grid, block, smem, s>>>(aa, nxt, kap);
+    const int d = dev >= 0 && dev < 64 ? dev : 0;
+    if (d != dev || !configured[d]) {
+        cudaFuncSetAttribute(aniso_adjoint_kernel<TTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        int sms = 152, blocks = 3;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, aniso_adjoint_kernel<TTI>, 32 * kWarpsPerBlock, smem);
+        resident[d] = std::max(sms * blocks, 1) * kWarpsPerBlock;
+        configured[d] = true;
     }
+    aa.ntiles = (aa.g.nx - 8 + kAnCols - 1) / kAnCols;
+    aa.H = aniso_height(aa.B, aa.ntiles, aa.g.nz - 8, resident[d]);
+    aa.nseg = (aa.g.nz - 8 + aa.H - 1) / aa.H;
+    const long long warps = (long long)aa.B * aa.ntiles * aa.nseg;
+    aniso_adjoint_kernel<TTI><<<(unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock), 32 * kWarpsPerBlock, smem, s>>>(
+        aa, nxt, kap);
+}
+
+static cudaError_t launch_aniso_adjoint(const AnisoArgs& aa, float* nxt, const float* kap, cudaStream_t s) {
+    if (!aniso_operands_aligned(aa, nxt, kap)) return cudaErrorMisalignedAddress;
+    if (aa.tti) launch_aniso_t<true>(aa, nxt, kap, s);
+    else launch_aniso_t<false>(aa, nxt, kap, s);
     return cudaSuccess;
 }
 

@@ -8,18 +8,13 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "pam_aniso.cuh"
 #include "pam_band.cuh"
 #include "pam_check.cuh"
 #include "pam_kernels.cuh"
 #include "pam_types.h"
 
 namespace pam {
-
-struct GridDims {
-    int nz, nx, P, N;          // expanded grid, pitch, absorbing width
-    long long stride;          // nz * P
-    const float* cerjan;       // [N] or nullptr (CPML)
-};
 
 // Cerjan factor of a cell in the order x then z (cpp/Modeling.cu:535-550);
 // 1 outside the border, for CPML runs and outside the update region.
@@ -212,341 +207,6 @@ __global__ void reduce_shots_kernel(const float* __restrict__ part, float* __res
     float s = out[i];
     for (int b = 0; b < B; b++) s += part[(long long)b * n + i];
     out[i] = s;
-}
-
-// ---------------------------------------------------------------- anisotropic adjoint (RTM)
-
-struct AnisoArgs {
-    const float* ub;      // receiver field U(t) [B][nz][P] (after injection)
-    const float* pf;      // source field at t (stored U(t)), [B][...] with pstride
-    long long pstride;
-    const float *eps, *del, *cth, *sth;   // [nz][P]
-    GridDims g;
-    int B, tti;
-    float inv_dx, inv_dz, inv_dx2, inv_dz2;
-};
-
-#define PAM_C0 (-1435.0f / 504.0f)
-#define PAM_C1 (8.0f / 5.0f)
-#define PAM_C2 (-1.0f / 5.0f)
-#define PAM_C3 (8.0f / 315.0f)
-#define PAM_C4 (-1.0f / 560.0f)
-#define PAM_A1 (4.0f / 5.0f)
-#define PAM_A2 (-1.0f / 5.0f)
-#define PAM_A3 (4.0f / 105.0f)
-#define PAM_A4 (-1.0f / 280.0f)
-
-// One backward step of the reference's anisotropic adjoint in a single pass.
-//
-// The reference (cpp/Migration.cu:573-973) runs it in two kernels: the first
-// writes five products of the receiver field U with coefficients taken from
-// the source field P (cpp/Migration.cu:573-666 VTI, :757-861 TTI)
-//   AU = A U, BU = B U, HU = 2 eps sin(2 theta) U (TTI), QCxU, QCzU,
-// the second applies their derivatives (cpp/Migration.cu:668-755, :863-973)
-//   new = D (2 U - D U_prev + kappa (dxx AU + dzz BU - dxz HU - dx QCxU - dz QCzU)).
-// Here a block owns a 32 x 32 output tile of one shot.  It loads the damped
-// source field of the tile with an 8-cell halo into shared memory, forms the
-// products of the tile with a 4-cell halo (the update's stencil reach) in
-// shared memory, and applies the update from there: no product ever goes to
-// HBM.  Per cell and shot the step reads P, U, U_prev and writes the new
-// field (16 B) instead of also writing and re-reading five product fields;
-// the products of the halo cells are computed again by the neighbouring
-// tiles (1.56x the product arithmetic).  The per-cell expressions are the
-// reference's, in its order, with its correctly rounded divisions (the
-// hardware reciprocal in their place measured no faster).  (Keeping four rows of the z-differentiated products per thread in
-// registers raised the registers from 41 to 57, cut the resident blocks from
-// six to four per SM and made the kernel 15% slower.)
-// Packed second and first derivatives of a cell pair for the anisotropic
-// adjoint: (C0 c + C1 (p1 + m1) + ... + C4 (p4 + m4)) * inv and
-// (A1 (p1 - m1) + ... + A4 (p4 - m4)) * inv, the coefficients of the
-// reference's adjoint kernels (cpp/Migration.cu:600-640).
-__device__ __forceinline__ float2 an_d2(float2 c, float2 p1, float2 m1, float2 p2, float2 m2, float2 p3, float2 m3,
-                                       float2 p4, float2 m4, float inv) {
-    float2 t = pmul2(bc2(PAM_C0), c);
-    t = pfma2(bc2(PAM_C1), padd2(p1, m1), t);
-    t = pfma2(bc2(PAM_C2), padd2(p2, m2), t);
-    t = pfma2(bc2(PAM_C3), padd2(p3, m3), t);
-    t = pfma2(bc2(PAM_C4), padd2(p4, m4), t);
-    return pmul2(t, bc2(inv));
-}
-__device__ __forceinline__ float2 an_d1(float2 p1, float2 m1, float2 p2, float2 m2, float2 p3, float2 m3, float2 p4,
-                                       float2 m4, float inv) {
-    float2 t = pmul2(bc2(PAM_A1), fsub2(p1, m1));
-    t = pfma2(bc2(PAM_A2), fsub2(p2, m2), t);
-    t = pfma2(bc2(PAM_A3), fsub2(p3, m3), t);
-    t = pfma2(bc2(PAM_A4), fsub2(p4, m4), t);
-    return pmul2(t, bc2(inv));
-}
-
-constexpr int kAnTX = 32, kAnTZ = 32;                 // output tile
-constexpr int kAnQX = kAnTX + 8, kAnQZ = kAnTZ + 8;   // products: tile + 4-cell halo
-constexpr int kAnSX = kAnTX + 16, kAnSZ = kAnTZ + 16; // source field: tile + 8-cell halo
-constexpr int kAnThreads = 256;                       // launched as (32, 8) threads
-
-__host__ __device__ constexpr int aniso_tile_smem_bytes(int tti) {
-    return (kAnSZ * kAnSX + kAnQZ * kAnQX * (tti ? 5 : 4)) * 4;
-}
-
-template <bool TTI>
-__global__ void __launch_bounds__(kAnThreads, TTI ? 4 : 5) aniso_adjoint_tile_kernel(const AnisoArgs a, float* __restrict__ nxt,
-                                                                 const float* __restrict__ kap)
-{
-    extern __shared__ float an_sm[];
-    float* Ps = an_sm;                                  // [kAnSZ][kAnSX] damped P
-    float* AUs = Ps + kAnSZ * kAnSX;                    // [kAnQZ][kAnQX] each
-    float* BUs = AUs + kAnQZ * kAnQX;
-    float* QXs = BUs + kAnQZ * kAnQX;
-    float* QZs = QXs + kAnQZ * kAnQX;
-    float* HUs = QZs + kAnQZ * kAnQX;                   // TTI only
-    const GridDims& g = a.g;
-    const int x0 = blockIdx.x * kAnTX, z0 = blockIdx.y * kAnTZ, b = blockIdx.z;
-    // launched as (32, 8) threads: in the update threadIdx.x runs along x, a warp per row
-    [[maybe_unused]] const long long pbytes = (long long)a.B * a.pstride * 4;
-    [[maybe_unused]] const long long fbytes = (long long)a.B * g.stride * 4;
-    [[maybe_unused]] const long long mbytes = (long long)g.nz * g.P * 4;
-    const float* Pb = a.pf + (long long)b * a.pstride;
-    const float* Ub = a.ub + (long long)b * g.stride;
-
-    // 1. the damped source field of the tile and its 8-cell halo (zero off
-    //    the grid, where only products outside the update region would read)
-    // block-uniform: does the source-field region / the output tile reach
-    // into the damped border (damp_apply leaves every other cell as it is)?
-    const bool src_damped = g.cerjan && !(x0 - 8 >= g.N && x0 + kAnTX + 8 <= g.nx - g.N && z0 - 8 >= g.N &&
-                                          z0 + kAnTZ + 8 <= g.nz - g.N);
-    const bool out_damped = g.cerjan && !(x0 >= g.N && x0 + kAnTX <= g.nx - g.N && z0 >= g.N &&
-                                          z0 + kAnTZ <= g.nz - g.N);
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    // every global operand of the products arrives in one batch of 16-byte
-    // cp.async (x0 is a multiple of 32, so every quad below starts on a
-    // 16-byte boundary of its row: the launcher checks the bases and pitches):
-    // the source field of the tile and its 8-cell halo into Ps (zero off the
-    // grid, where only products outside the update region would read), and
-    // the products' per-cell operands - eps, delta, U (and cos, sin for TTI) -
-    // into the product arrays AU, BU, QX (QZ, HU), each at the cell whose
-    // product later overwrites it, for quads that reach into the update region
-    constexpr int SQX = kAnSX / 4;                       // quads per source row
-    for (int i = tid; i < kAnSZ * SQX; i += kAnThreads) {
-        const int r = i / SQX, cq = (i % SQX) * 4;
-        const int z = z0 - 8 + r, x = x0 - 8 + cq;
-        float* dst = Ps + r * kAnSX + cq;
-        const bool zon = z >= 0 && z < g.nz;
-        if (zon && x >= 0 && x + 3 < g.nx) {
-            cp_async16(dst, PAM_CHK(Pb + (long long)z * g.P + x, a.pf, pbytes, 16, 92));
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                dst[k] = (zon && x + k >= 0 && x + k < g.nx)
-                             ? *PAM_CHK(Pb + (long long)z * g.P + x + k, a.pf, pbytes, 4, 92) : 0.0f;
-        }
-    }
-    constexpr int QQX = kAnQX / 4;                       // quads per product row
-    constexpr int NSTAGE = TTI ? 5 : 3;
-    for (int i = tid; i < NSTAGE * kAnQZ * QQX; i += kAnThreads) {
-        const int arr = i / (kAnQZ * QQX), j = i % (kAnQZ * QQX);
-        const int r = j / QQX, cq = (j % QQX) * 4;
-        const int z = z0 - 4 + r, x = x0 - 4 + cq;
-        if (z >= 4 && z < g.nz - 4 && x >= 4 && x < g.nx - 4) {
-            const long long m = (long long)z * g.P + x;
-            const float* src;
-            switch (arr) {
-                case 0: src = PAM_CHK(a.eps + m, a.eps, mbytes, 16, 93); break;
-                case 1: src = PAM_CHK(a.del + m, a.del, mbytes, 16, 93); break;
-                case 2: src = PAM_CHK(Ub + m, a.ub, fbytes, 16, 94); break;
-                case 3: src = PAM_CHK(a.cth + m, a.cth, mbytes, 16, 93); break;
-                default: src = PAM_CHK(a.sth + m, a.sth, mbytes, 16, 93); break;
-            }
-            cp_async16(AUs + arr * (kAnQZ * kAnQX) + r * kAnQX + cq, src);
-        }
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    if (src_damped) {
-        for (int i = tid; i < kAnSZ * kAnSX; i += kAnThreads) {
-            const int z = z0 - 8 + i / kAnSX, x = x0 - 8 + i % kAnSX;
-            if (z >= 0 && z < g.nz && x >= 0 && x < g.nx) Ps[i] = damp_apply(g, z, x, Ps[i]);
-        }
-        __syncthreads();
-    }
-
-    // 2. the products of the tile and its 4-cell halo (zero outside the
-    //    update region, as the reference's products kernel leaves them), for
-    //    pairs of x-adjacent cells: 8-byte shared loads and the packed FP32x2
-    //    instructions for the derivatives, the Sd ratio per cell
-    constexpr int QXP = kAnQX / 2;
-    for (int i = tid; i < kAnQZ * QXP; i += kAnThreads) {   // whole warps on consecutive pairs
-        const int qz = i / QXP, qx = (i % QXP) * 2;
-        const int z = z0 - 4 + qz, x = x0 - 4 + qx;
-        const bool zin = z >= 4 && z < g.nz - 4;
-        const bool in0 = zin && x >= 4 && x < g.nx - 4, in1 = zin && x + 1 >= 4 && x + 1 < g.nx - 4;
-        float2 av = make_float2(0.f, 0.f), bv = av, hv = av, qxv = av, qzv = av;
-        if (in0 || in1) {
-            const float* c = Ps + (qz + 4) * kAnSX + (qx + 4);
-            auto L = [&](int off) { return *reinterpret_cast<const float2*>(c + off); };   // even offsets
-            const float2 A0 = L(-4), A1 = L(-2), A2 = L(0), A3 = L(2), A4 = L(4);
-            const float2 Om3 = make_float2(A0.y, A1.x), Om1 = make_float2(A1.y, A2.x);
-            const float2 Op1 = make_float2(A2.y, A3.x), Op3 = make_float2(A3.y, A4.x);
-            const float2 Z1 = L(kAnSX), Zm1 = L(-kAnSX), Z2 = L(2 * kAnSX), Zm2 = L(-2 * kAnSX);
-            const float2 Z3 = L(3 * kAnSX), Zm3 = L(-3 * kAnSX), Z4 = L(4 * kAnSX), Zm4 = L(-4 * kAnSX);
-            const float2 pxx = an_d2(A2, Op1, Om1, A3, A1, Op3, Om3, A4, A0, a.inv_dx2);
-            const float2 pzz = an_d2(A2, Z1, Zm1, Z2, Zm2, Z3, Zm3, Z4, Zm4, a.inv_dz2);
-            const float2 px = an_d1(Op1, Om1, A3, A1, Op3, Om3, A4, A0, a.inv_dx);
-            const float2 pz = an_d1(Z1, Zm1, Z2, Zm2, Z3, Zm3, Z4, Zm4, a.inv_dz);
-            // the staged operands of this pair (overwritten by its products below)
-            const int qs = qz * kAnQX + qx;
-            const float2 e2v = *reinterpret_cast<const float2*>(AUs + qs);
-            const float2 d2v = *reinterpret_cast<const float2*>(BUs + qs);
-            const float2 u2 = *reinterpret_cast<const float2*>(QXs + qs);
-            float2 cs2 = make_float2(0.f, 0.f), sn2 = cs2;
-            if (TTI) {
-                cs2 = *reinterpret_cast<const float2*>(QZs + qs);
-                sn2 = *reinterpret_cast<const float2*>(HUs + qs);
-            }
-            // the reference's per-cell products (cpp/Migration.cu:573-666, 757-861)
-            auto cell = [&](float pxs, float pzs, float pxxs, float pzzs, float e, float d, float u, float cs, float sn,
-                            float& A_u, float& B_u, float& H_u, float& QX_u, float& QZ_u) {
-                float sd = 0.f, Cx = 0.f, Cz = 0.f, A_, B_, hs = 0.f;
-                if (!TTI) {
-                    const float px2 = pxs * pxs, pz2 = pzs * pzs, px4 = px2 * px2, pz4 = pz2 * pz2;
-                    const float num = -2.0f * (e - d) * px2 * pz2;
-                    const float den = (1.0f + 2.0f * e) * px4 + pz4 + 2.0f * (1.0f + d) * px2 * pz2;
-                    if (fabsf(den) > 1.0e-12f) {
-                        sd = num / den;
-                        const float inv_den2 = 1.0f / (den * den);
-                        const float factor = 4.0f * (e - d) * ((1.0f + 2.0f * e) * px4 - pz4) * inv_den2;
-                        Cx = factor * pxs * pz2;
-                        Cz = -factor * px2 * pzs;
-                    }
-                    A_ = 1.0f + 2.0f * e + sd;
-                    B_ = 1.0f + sd;
-                } else {
-                    const float xi = pxs * cs - pzs * sn, eta = pxs * sn + pzs * cs;
-                    const float xi2 = xi * xi, eta2 = eta * eta, xi4 = xi2 * xi2, eta4 = eta2 * eta2;
-                    const float num = -2.0f * (e - d) * xi2 * eta2;
-                    const float den = (1.0f + 2.0f * e) * xi4 + eta4 + 2.0f * (1.0f + d) * xi2 * eta2;
-                    if (fabsf(den) > 1.0e-12f) {
-                        sd = num / den;
-                        const float K = (1.0f + 2.0f * e) * xi4 - eta4;
-                        const float factor = 4.0f * (e - d) * xi * eta * K / (den * den);
-                        Cx = factor * pzs;
-                        Cz = -factor * pxs;
-                    }
-                    const float cos2 = cs * cs, sin2 = sn * sn;
-                    A_ = (1.0f + 2.0f * e) * cos2 + sin2 + sd;
-                    B_ = (1.0f + 2.0f * e) * sin2 + cos2 + sd;
-                    hs = 2.0f * e * (2.0f * sn * cs);   // 2 eps sin(2 theta)
-                }
-                const float Q = pxxs + pzzs;
-                A_u = A_ * u;
-                B_u = B_ * u;
-                H_u = hs * u;
-                QX_u = Q * Cx * u;
-                QZ_u = Q * Cz * u;
-            };
-            if (in0) cell(px.x, pz.x, pxx.x, pzz.x, e2v.x, d2v.x, u2.x, cs2.x, sn2.x, av.x, bv.x, hv.x, qxv.x, qzv.x);
-            if (in1) cell(px.y, pz.y, pxx.y, pzz.y, e2v.y, d2v.y, u2.y, cs2.y, sn2.y, av.y, bv.y, hv.y, qxv.y, qzv.y);
-        }
-        const int q = qz * kAnQX + qx;
-        *reinterpret_cast<float2*>(AUs + q) = av;
-        *reinterpret_cast<float2*>(BUs + q) = bv;
-        *reinterpret_cast<float2*>(QXs + q) = qxv;
-        *reinterpret_cast<float2*>(QZs + q) = qzv;
-        if (TTI) *reinterpret_cast<float2*>(HUs + q) = hv;
-    }
-    __syncthreads();
-
-    // 3. the update of the tile's cells, by pairs of x-adjacent cells:
-    //    new = D (2 U - D U_prev + kappa (dxx AU + dzz BU - dxz HU - dx QCxU - dz QCzU))
-    //    (each thread's U, kappa and U_prev loaded before any of its arithmetic)
-    constexpr int TXP = kAnTX / 2;
-    constexpr int NUPD = kAnTZ * TXP / kAnThreads;      // pairs per thread
-    static_assert(kAnTZ * TXP % kAnThreads == 0, "whole pairs per thread");
-    float2 ucv[NUPD], kvv[NUPD], pvv[NUPD];
-#pragma unroll
-    for (int it = 0; it < NUPD; it++) {
-        const int i = tid + it * kAnThreads;
-        const int z = z0 + i / TXP, x = x0 + (i % TXP) * 2;
-        const bool zin = z >= 4 && z < g.nz - 4;
-        ucv[it] = kvv[it] = pvv[it] = make_float2(0.f, 0.f);
-        if (zin && x + 1 >= 4 && x < g.nx - 4) {
-            const long long m = (long long)z * g.P + x;
-            const long long o = (long long)b * g.stride + m;
-            ucv[it] = *reinterpret_cast<const float2*>(PAM_CHK(a.ub + o, a.ub, fbytes, 8, 95));
-            kvv[it] = *reinterpret_cast<const float2*>(PAM_CHK(kap + m, kap, mbytes, 8, 93));
-            pvv[it] = *reinterpret_cast<const float2*>(PAM_CHK(nxt + o, nxt, fbytes, 8, 96));
-        }
-    }
-#pragma unroll
-    for (int it = 0; it < NUPD; it++) {
-        const int i = tid + it * kAnThreads;
-        const int tz = i / TXP, tx = (i % TXP) * 2;
-        const int z = z0 + tz, x = x0 + tx;
-        const bool zin = z >= 4 && z < g.nz - 4;
-        const bool in0 = zin && x >= 4 && x < g.nx - 4, in1 = zin && x + 1 >= 4 && x + 1 < g.nx - 4;
-        if (!in0 && !in1) continue;
-        const int q = (tz + 4) * kAnQX + (tx + 4);
-        constexpr int s = kAnQX;
-        auto L = [&](const float* f, int off) { return *reinterpret_cast<const float2*>(f + q + off); };
-        float2 op;
-        {
-            const float2 A0 = L(AUs, -4), A1 = L(AUs, -2), A2 = L(AUs, 0), A3 = L(AUs, 2), A4 = L(AUs, 4);
-            const float2 dxx = an_d2(A2, make_float2(A2.y, A3.x), make_float2(A1.y, A2.x), A3, A1,
-                                     make_float2(A3.y, A4.x), make_float2(A0.y, A1.x), A4, A0, a.inv_dx2);
-            const float2 dzz = an_d2(L(BUs, 0), L(BUs, s), L(BUs, -s), L(BUs, 2 * s), L(BUs, -2 * s), L(BUs, 3 * s),
-                                     L(BUs, -3 * s), L(BUs, 4 * s), L(BUs, -4 * s), a.inv_dz2);
-            op = padd2(dxx, dzz);
-        }
-        if (TTI) {
-            // the factorised cross derivative (cpp/Migration.cu:906-928) of HU, per
-            // pair: for each az the rows +az and -az (columns -4 .. +5 around the
-            // pair, five aligned 8-byte loads each) feed the sums of all four ax,
-            // in the order of sum_ax a_ax sum_az a_az (...)
-            const float aa[5] = {0.f, PAM_A1, PAM_A2, PAM_A3, PAM_A4};
-            float2 tax[5] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f),
-                             make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-            for (int az = 1; az <= 4; az++) {
-                float vp[10], vm[10];
-#pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    const float2 hp = L(HUs, az * s - 4 + 2 * k), hm = L(HUs, -az * s - 4 + 2 * k);
-                    vp[2 * k] = hp.x; vp[2 * k + 1] = hp.y;
-                    vm[2 * k] = hm.x; vm[2 * k + 1] = hm.y;
-                }
-#pragma unroll
-                for (int ax = 1; ax <= 4; ax++) {
-                    // H(dz, dx) of the pair = (v[4 + dx], v[5 + dx]) of row dz
-                    const float2 hpa = make_float2(vp[4 + ax], vp[5 + ax]), hma = make_float2(vm[4 + ax], vm[5 + ax]);
-                    const float2 hpb = make_float2(vp[4 - ax], vp[5 - ax]), hmb = make_float2(vm[4 - ax], vm[5 - ax]);
-                    const float2 comb = padd2(fsub2(hpa, hma), fsub2(hmb, hpb));
-                    tax[ax] = pfma2(bc2(aa[az]), comb, tax[ax]);
-                }
-            }
-            float2 dxz = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int ax = 1; ax <= 4; ax++) dxz = pfma2(bc2(aa[ax]), tax[ax], dxz);
-            op = fsub2(op, pmul2(dxz, bc2(a.inv_dx * a.inv_dz)));
-        }
-        {
-            const float2 X0 = L(QXs, -4), X1 = L(QXs, -2), X2 = L(QXs, 0), X3 = L(QXs, 2), X4 = L(QXs, 4);
-            op = fsub2(op, an_d1(make_float2(X2.y, X3.x), make_float2(X1.y, X2.x), X3, X1, make_float2(X3.y, X4.x),
-                                 make_float2(X0.y, X1.x), X4, X0, a.inv_dx));
-            op = fsub2(op, an_d1(L(QZs, s), L(QZs, -s), L(QZs, 2 * s), L(QZs, -2 * s), L(QZs, 3 * s),
-                                 L(QZs, -3 * s), L(QZs, 4 * s), L(QZs, -4 * s), a.inv_dz));
-        }
-        const long long o = (long long)b * g.stride + (long long)z * g.P + x;
-        const float2 uc = ucv[it], kv = kvv[it];
-        float2 prev = pvv[it];
-        if (out_damped) prev = make_float2(damp_apply(g, z, x, prev.x), damp_apply(g, z, x + 1, prev.y));
-        float2 out = pfma2(kv, op, fsub2(padd2(uc, uc), prev));
-        if (out_damped) out = make_float2(damp_apply(g, z, x, out.x), damp_apply(g, z, x + 1, out.y));
-        if (in0 && in1) {
-            *reinterpret_cast<float2*>(PAM_CHK(nxt + o, nxt, fbytes, 8, 96)) = out;
-        } else {
-            if (in0) *PAM_CHK(nxt + o, nxt, fbytes, 4, 96) = out.x;
-            if (in1) *PAM_CHK(nxt + o + 1, nxt, fbytes, 4, 96) = out.y;
-        }
-    }
 }
 
 // ---------------------------------------------------------------- exact discrete adjoint (acoustic)
