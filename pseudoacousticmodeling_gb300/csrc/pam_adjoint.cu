@@ -778,26 +778,38 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         } else if (mode == kFWIRef) {
             // Python loop (src/Migration.py:1030-1049): illumination over every
             // forward step, gradient for t = nt-2 .. 1
-            ilum_sum_kernel<<<gsum, blk, 0, st>>>(Pt, d_grad_ilum, g, nzi, nxi, pstride, nshots);
-            if (t <= nt - 2 && t >= 1) {
+            const bool step = t <= nt - 2 && t >= 1;
+            const float inv_dt2 = 1.0f / (cfg.dt * cfg.dt);
+            auto sums = [&]() {
+                cudaEvent_t pend;
+                prof_begin(t, 4, st, &pend);
+                if (mp && step) {
+                    const float inv_dx = 1.0f / cfg.dx, inv_dz = 1.0f / cfg.dz;
+                    const float inv_dx2 = 1.0f / (cfg.dx * cfg.dx), inv_dz2 = 1.0f / (cfg.dz * cfg.dz);
+                    if (cfg.approximation == PAM_TTI)
+                        mp_grad_kernel<true><<<gsum, blk, 0, st>>>(Pt, Pm1, Pp1, ucur, pstride, d_eps, d_del, d_cth, d_sth,
+                                                                   d_mp, d_mp + interior, d_mp + 2 * interior, d_grad,
+                                                                   d_grad_ilum, g, nzi, nxi, nshots, inv_dx, inv_dz, inv_dx2,
+                                                                   inv_dz2, inv_dt2);
+                    else
+                        mp_grad_kernel<false><<<gsum, blk, 0, st>>>(Pt, Pm1, Pp1, ucur, pstride, d_eps, d_del, d_cth, d_sth,
+                                                                    d_mp, d_mp + interior, nullptr, d_grad, d_grad_ilum, g,
+                                                                    nzi, nxi, nshots, inv_dx, inv_dz, inv_dx2, inv_dz2,
+                                                                    inv_dt2);
+                } else {
+                    fwi_ref_sum_kernel<<<gquad, blk, 0, st>>>(ucur, Pm1, Pt, Pp1, d_grad, d_grad_ilum, g, nzi, nxi, pstride,
+                                                              nshots, inv_dt2, step);
+                }
+                if (pend) cudaEventRecordWithFlags(pend, st, prof_flags);
+            };
+            if (!step) sums();
+            if (step) {
                 if (t >= itlag) {
                     const long long n = (long long)nrec * nshots;
                     inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
                         ucur, d_obs, d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
                 }
-                {
-                    cudaEvent_t pend;
-                    prof_begin(t, 4, st, &pend);
-                    fwi_ref_grad_sum_kernel<<<gsum, blk, 0, st>>>(ucur, Pm1, Pt, Pp1, d_grad, g, nzi, nxi, pstride,
-                                                                  nshots, 1.0f / (cfg.dt * cfg.dt));
-                    if (pend) cudaEventRecordWithFlags(pend, st, prof_flags);
-                }
-                if (mp)
-                    mp_grad_kernel<<<gsum, blk, 0, st>>>(Pt, ucur, pstride, d_eps, d_del, d_cth, d_sth, d_mp,
-                                                         d_mp + interior,
-                                                         cfg.approximation == PAM_TTI ? d_mp + 2 * interior : nullptr,
-                                                         g, nzi, nxi, nshots, 1.0f / cfg.dx, 1.0f / cfg.dz,
-                                                         1.0f / (cfg.dx * cfg.dx), 1.0f / (cfg.dz * cfg.dz));
+                sums();
                 if (cfg.approximation == PAM_ACOUSTIC) {
                     if (cfg.boundary == PAM_CPML)
                         launch_cpml(nshots, ucur, st, d_bpsix, d_bzetax, d_bxaux, d_bpsiz, d_bzetaz, d_bzaux);

@@ -133,39 +133,51 @@ __global__ void imaging_sum_kernel(const float* __restrict__ ub, const float* __
     }
 }
 
-__global__ void fwi_ref_grad_sum_kernel(const float* __restrict__ ub, const float* __restrict__ pp,
-                                        const float* __restrict__ pc, const float* __restrict__ pf,
-                                        float* __restrict__ grad, GridDims g, int nzi, int nxi, long long pstride,
-                                        int B, float inv_dt2)
+// The reference gradient and its illumination in one pass (grad == 0: the
+// illumination alone, of the steps outside the gradient's range), by quads like
+// the imaging condition: the field at t is read once.
+__global__ void fwi_ref_sum_kernel(const float* __restrict__ ub, const float* __restrict__ pp, const float* __restrict__ pc,
+                                   const float* __restrict__ pf, float* __restrict__ grad, float* __restrict__ ilum,
+                                   GridDims g, int nzi, int nxi, long long pstride, int B, float inv_dt2, int with_grad)
 {
-    const int xi = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int zi = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xi >= nxi || zi >= nzi) return;
-    const long long c = (long long)(zi + g.N) * g.P + xi + g.N;
-    float sg = 0.0f;
-#pragma unroll 4
+    const int xf0 = 4 * q;
+    if (zi >= nzi || xf0 >= g.N + nxi || xf0 + 4 <= g.N) return;
+    const long long c = (long long)(zi + g.N) * g.P + xf0;
+    float sg[4] = {0.f, 0.f, 0.f, 0.f}, si[4] = {0.f, 0.f, 0.f, 0.f};
+    auto quad = [&](const float* p, long long o, [[maybe_unused]] long long stride, float (&v)[4]) {
+        const float4 x = *reinterpret_cast<const float4*>(PAM_CHK(p + o, p, (long long)B * stride * 4, 16, 63));
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    };
+#pragma unroll 2
     for (int b = 0; b < B; b++) {
-        const long long pc_ = (long long)b * pstride + c;
-        const float d2 = (pf[pc_] - 2.0f * pc[pc_] + pp[pc_]) * inv_dt2;
-        sg += ub[(long long)b * g.stride + c] * d2;
+        const long long o = (long long)b * pstride + c;
+        float c4[4], f4[4], p4[4], u4[4];
+        quad(pc, o, pstride, c4);
+        if (with_grad) {
+            quad(pf, o, pstride, f4);
+            quad(pp, o, pstride, p4);
+            quad(ub, (long long)b * g.stride + c, g.stride, u4);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            si[j] += c4[j] * c4[j];
+            if (with_grad) {
+                const float d2 = (f4[j] - 2.0f * c4[j] + p4[j]) * inv_dt2;
+                sg[j] += u4[j] * d2;
+            }
+        }
     }
-    grad[(long long)zi * nxi + xi] += sg;
-}
-
-__global__ void ilum_sum_kernel(const float* __restrict__ P_, float* __restrict__ ilum, GridDims g, int nzi, int nxi,
-                                long long pstride, int B)
-{
-    const int xi = blockIdx.x * blockDim.x + threadIdx.x;
-    const int zi = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xi >= nxi || zi >= nzi) return;
-    const long long c = (long long)(zi + g.N) * g.P + xi + g.N;
-    float si = 0.0f;
-#pragma unroll 4
-    for (int b = 0; b < B; b++) {
-        const float p = P_[(long long)b * pstride + c];
-        si += p * p;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int xi = xf0 + j - g.N;
+        if (xi >= 0 && xi < nxi) {
+            const long long i = (long long)zi * nxi + xi;
+            ilum[i] += si[j];
+            if (with_grad) grad[i] += sg[j];
+        }
     }
-    ilum[(long long)zi * nxi + xi] += si;
 }
 
 // Sum per-shot accumulators into the running total: out[i] += sum_b part[b][i]
@@ -258,47 +270,74 @@ __global__ void inject_adjoint_kernel(float* __restrict__ w, const float* __rest
 // are skipped, as the reference's interior arrays do.  One thread per
 // interior cell sums the batch's shots in registers (shots in order) and adds
 // the sums to the running totals [nz][nx] once per step, like the imaging
-// condition; the reference sums each shot over time first.  grid (nx, nz)
-// blocks of 32 x 8.
-__global__ void mp_grad_kernel(const float* __restrict__ P_, const float* __restrict__ ub, long long pstride,
-                               const float* __restrict__ eps, const float* __restrict__ del,
-                               const float* __restrict__ cth, const float* __restrict__ sth,
-                               float* __restrict__ geps, float* __restrict__ gdel, float* __restrict__ gth,
-                               GridDims g, int nzi, int nxi, int B, float inv_dx, float inv_dz, float inv_dx2,
-                               float inv_dz2)
+// condition; the reference sums each shot over time first.  The same pass adds
+// the vp gradient and the illumination of the step (fwi_ref_sum_kernel).  The
+// cross derivative is the x derivative of the z derivative, which the cells of a
+// block pass on through shared memory: 16 loads and 17 operations a cell where
+// the 64-point form took 64 and 84.  grid (nx, nz) blocks of 32 x 8.
+template <bool TTI>
+__global__ void __launch_bounds__(256) mp_grad_kernel(const float* __restrict__ P_, const float* __restrict__ pm,
+                                                      const float* __restrict__ pf, const float* __restrict__ ub,
+                                                      long long pstride, const float* __restrict__ eps,
+                                                      const float* __restrict__ del, const float* __restrict__ cth,
+                                                      const float* __restrict__ sth, float* __restrict__ geps,
+                                                      float* __restrict__ gdel, float* __restrict__ gth,
+                                                      float* __restrict__ grad, float* __restrict__ ilum, GridDims g, int nzi,
+                                                      int nxi, int B, float inv_dx, float inv_dz, float inv_dx2,
+                                                      float inv_dz2, float inv_dt2)
 {
-    const int xi = blockIdx.x * blockDim.x + threadIdx.x;
-    const int zi = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xi < 4 || xi >= nxi - 4 || zi < 4 || zi >= nzi - 4) return;
+    __shared__ float pzs[2][8][40];        // z derivatives of the block's rows, four columns more on each side
+    const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 8;
+    const int xi = x0 + threadIdx.x, zi = z0 + threadIdx.y;
+    const bool cell = xi < nxi && zi < nzi;
+    const bool inner = xi >= 4 && xi < nxi - 4 && zi >= 4 && zi < nzi - 4;
     const long long c = (long long)(zi + g.N) * g.P + xi + g.N;
     const long long s = g.P;
-    const bool tti = gth != nullptr;
-    const float ct = tti ? cth[c] : 1.0f, st = tti ? sth[c] : 0.0f;
-    const float e = eps[c], d = del[c];
+    float ct = 1.0f, st = 0.0f, e = 0.0f, d = 0.0f;
+    if (inner) {
+        if (TTI) {
+            ct = cth[c];
+            st = sth[c];
+        }
+        e = eps[c];
+        d = del[c];
+    }
     const float s2 = 2.0f * st * ct, c2 = ct * ct, sn2 = st * st;
-    float sum_e = 0.0f, sum_d = 0.0f, sum_t = 0.0f;
+    float sum_e = 0.0f, sum_d = 0.0f, sum_t = 0.0f, sum_g = 0.0f, sum_i = 0.0f;
+    auto dz = [&](const float* U) {
+        return (PAM_A1 * (U[s] - U[-s]) + PAM_A2 * (U[2 * s] - U[-2 * s]) + PAM_A3 * (U[3 * s] - U[-3 * s]) +
+                PAM_A4 * (U[4 * s] - U[-4 * s])) * inv_dz;
+    };
+    // the block's outer columns: one cell for each of the first 64 threads
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int hz = z0 + (tid >> 3), hc = tid & 7, hx = x0 + (hc < 4 ? hc - 4 : hc + 28);
+    const bool halo = TTI && tid < 64 && hz >= 4 && hz < nzi - 4 && hx >= 0 && hx < nxi;
+    const long long hcell = (long long)(hz + g.N) * g.P + hx + g.N;
     for (int b = 0; b < B; b++) {
         const float* U = P_ + (long long)b * pstride + c;
-        const float pxx = (PAM_C0 * U[0] + PAM_C1 * (U[1] + U[-1]) + PAM_C2 * (U[2] + U[-2]) +
+        float pz = 0.0f;
+        if (cell && zi >= 4 && zi < nzi - 4) pz = dz(U);
+        if (TTI) {
+            pzs[b & 1][threadIdx.y][threadIdx.x + 4] = pz;
+            if (halo) pzs[b & 1][tid >> 3][hc < 4 ? hc : hc + 32] = dz(P_ + (long long)b * pstride + hcell);
+            __syncthreads();
+        }
+        if (!cell) continue;
+        const float u0 = U[0], a = ub[(long long)b * g.stride + c];
+        sum_i += u0 * u0;
+        sum_g += a * ((pf[(long long)b * pstride + c] - 2.0f * u0 + pm[(long long)b * pstride + c]) * inv_dt2);
+        if (!inner) continue;
+        const float pxx = (PAM_C0 * u0 + PAM_C1 * (U[1] + U[-1]) + PAM_C2 * (U[2] + U[-2]) +
                            PAM_C3 * (U[3] + U[-3]) + PAM_C4 * (U[4] + U[-4])) * inv_dx2;
-        const float pzz = (PAM_C0 * U[0] + PAM_C1 * (U[s] + U[-s]) + PAM_C2 * (U[2 * s] + U[-2 * s]) +
+        const float pzz = (PAM_C0 * u0 + PAM_C1 * (U[s] + U[-s]) + PAM_C2 * (U[2 * s] + U[-2 * s]) +
                            PAM_C3 * (U[3 * s] + U[-3 * s]) + PAM_C4 * (U[4 * s] + U[-4 * s])) * inv_dz2;
         const float px = (PAM_A1 * (U[1] - U[-1]) + PAM_A2 * (U[2] - U[-2]) + PAM_A3 * (U[3] - U[-3]) +
                           PAM_A4 * (U[4] - U[-4])) * inv_dx;
-        const float pz = (PAM_A1 * (U[s] - U[-s]) + PAM_A2 * (U[2 * s] - U[-2 * s]) +
-                          PAM_A3 * (U[3 * s] - U[-3 * s]) + PAM_A4 * (U[4 * s] - U[-4 * s])) * inv_dz;
         float pxz = 0.0f;
-        if (tti) {
-            const float a[4] = {PAM_A1, PAM_A2, PAM_A3, PAM_A4};
-#pragma unroll
-            for (int m = 1; m <= 4; m++) {
-                float t = 0.0f;
-#pragma unroll
-                for (int n = 1; n <= 4; n++)
-                    t += a[n - 1] * (U[n * s + m] - U[-n * s + m] + U[-n * s - m] - U[n * s - m]);
-                pxz += a[m - 1] * t;
-            }
-            pxz *= inv_dx * inv_dz;
+        if (TTI) {
+            const float* v = &pzs[b & 1][threadIdx.y][threadIdx.x + 4];
+            pxz = (PAM_A1 * (v[1] - v[-1]) + PAM_A2 * (v[2] - v[-2]) + PAM_A3 * (v[3] - v[-3]) +
+                   PAM_A4 * (v[4] - v[-4])) * inv_dx;
         }
         float h = px * ct - pz * st, q = px * st + pz * ct;
         const float mh = fmaxf(fabsf(h), fabsf(q));
@@ -312,7 +351,7 @@ __global__ void mp_grad_kernel(const float* __restrict__ P_, const float* __rest
             const float r = 1.0f / (den * den);
             dSe = (-2.0f * t * den - num * 2.0f * h4) * r;
             dSdl = (2.0f * t * den - num * 2.0f * t) * r;
-            if (tti) {
+            if (TTI) {
                 const float w = -2.0f * h * q * q2 + 2.0f * h * h2 * q;
                 const float dnum = -2.0f * (e - d) * w;
                 const float dden =
@@ -320,18 +359,21 @@ __global__ void mp_grad_kernel(const float* __restrict__ P_, const float* __rest
                 dSt = (dnum * den - num * dden) * r;
             }
         }
-        const float a = ub[(long long)b * g.stride + c];
         sum_e += a * (-(2.0f * c2 + dSe) * pxx - (2.0f * sn2 + dSe) * pzz + 2.0f * s2 * pxz);
         sum_d += a * (-dSdl * (pxx + pzz));
-        if (tti) {
+        if (TTI) {
             const float cos2 = c2 - sn2;
             sum_t += a * ((2.0f * e * s2 - dSt) * pxx + (-2.0f * e * s2 - dSt) * pzz + 4.0f * e * cos2 * pxz);
         }
     }
+    if (!cell) return;
     const long long o = (long long)zi * nxi + xi;
+    grad[o] += sum_g;
+    ilum[o] += sum_i;
+    if (!inner) return;
     geps[o] += sum_e;
     gdel[o] += sum_d;
-    if (tti) gth[o] += sum_t;
+    if (TTI) gth[o] += sum_t;
 }
 
 // ---------------------------------------------------------------- boundary saving

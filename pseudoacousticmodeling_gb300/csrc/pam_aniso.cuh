@@ -337,10 +337,9 @@ __global__ void __launch_bounds__(128, aniso_min_blocks<TTI>()) aniso_adjoint_ke
                 op = padd2(dxx, dzz);
             }
             if (TTI) {
-                // the factorised cross derivative (cpp/Migration.cu:906-928) of HU, per
-                // pair: for each az the rows +az and -az (columns -4 .. +5 around the
-                // pair, five aligned 8-byte loads each) feed the sums of all four ax,
-                // in the order of sum_ax a_ax sum_az a_az (...)
+                // the cross derivative (cpp/Migration.cu:906-928) of HU in the order of
+                // sum_ax a_ax sum_az a_az (...): for each az the differences of the rows
+                // +az and -az (columns -4 .. +5 around the pair) feed all four ax
                 const float aa[5] = {0.f, PAM_A1, PAM_A2, PAM_A3, PAM_A4};
                 float2 tax[5] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f),
                                  make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -348,21 +347,15 @@ __global__ void __launch_bounds__(128, aniso_min_blocks<TTI>()) aniso_adjoint_ke
                 for (int az = 1; az <= 4; az++) {
                     const float* const hpr = Hr + ((t - rs + az) & (kAnHRing - 1)) * 64 + 2 * lane;
                     const float* const hmr = Hr + ((t - rs - az) & (kAnHRing - 1)) * 64 + 2 * lane;
-                    float vp[10], vm[10];
+                    float2 v[5];
 #pragma unroll
-                    for (int k = 0; k < 5; k++) {
-                        const float2 hp = at(hpr - 4 + 2 * k), hm = at(hmr - 4 + 2 * k);
-                        vp[2 * k] = hp.x; vp[2 * k + 1] = hp.y;
-                        vm[2 * k] = hm.x; vm[2 * k + 1] = hm.y;
-                    }
-#pragma unroll
-                    for (int ax = 1; ax <= 4; ax++) {
-                        // H(dz, dx) of the pair = (v[4 + dx], v[5 + dx]) of row dz
-                        const float2 hpa = make_float2(vp[4 + ax], vp[5 + ax]), hma = make_float2(vm[4 + ax], vm[5 + ax]);
-                        const float2 hpb = make_float2(vp[4 - ax], vp[5 - ax]), hmb = make_float2(vm[4 - ax], vm[5 - ax]);
-                        const float2 comb = padd2(fsub2(hpa, hma), fsub2(hmb, hpb));
-                        tax[ax] = pfma2(bc2(aa[az]), comb, tax[ax]);
-                    }
+                    for (int k = 0; k < 5; k++) v[k] = fsub2(at(hpr - 4 + 2 * k), at(hmr - 4 + 2 * k));
+                    const float2 p1 = make_float2(v[2].y, v[3].x), m1 = make_float2(v[1].y, v[2].x);
+                    const float2 p3 = make_float2(v[3].y, v[4].x), m3 = make_float2(v[0].y, v[1].x);
+                    tax[1] = pfma2(bc2(aa[az]), fsub2(p1, m1), tax[1]);
+                    tax[2] = pfma2(bc2(aa[az]), fsub2(v[3], v[1]), tax[2]);
+                    tax[3] = pfma2(bc2(aa[az]), fsub2(p3, m3), tax[3]);
+                    tax[4] = pfma2(bc2(aa[az]), fsub2(v[4], v[0]), tax[4]);
                 }
                 float2 dxz = make_float2(0.f, 0.f);
 #pragma unroll
