@@ -60,9 +60,10 @@ __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpre
 //
 // Per row r a warp needs U(t) rows r-4..r+4 (a nine-row register window) and,
 // for its writer lanes, U(t-1) and the model at row r.  The window's leading
-// row r+4, U(t-1) and the model rows arrive through a per-warp ring of kRing
-// shared-memory slots filled by cp.async ring_ahead() rows ahead, so their HBM
-// latency overlaps the arithmetic of earlier rows without costing registers.
+// row r+4, U(t-1) and the model rows arrive through a per-warp ring of
+// ring_slots() shared-memory slots filled by cp.async ring_ahead() rows ahead,
+// so their HBM latency overlaps the arithmetic of earlier rows without costing
+// registers.
 // x neighbours are exchanged through a double-buffered shared row (one
 // 16-byte store and two loads per row).
 
@@ -74,15 +75,19 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-constexpr int kRing = 4;    // ring slots per warp
+// Ring slots per warp.  With three (and one exchange row instead of two) four
+// TTI blocks fit an SM instead of three: 16 shots of 701 x 1601 in 60.6 ms per
+// 793 steps instead of 63.3.  VTI fits its four blocks with four slots; five
+// blocks of 96 registers spill (64 shots of 901 x 2101: 394 ms for 309).
+template <int APPROX>
+__host__ __device__ constexpr int ring_slots() { return APPROX == kTTI ? 3 : 4; }
 
-// Rows in flight ahead of the one being computed (at most kRing - 1: the slot
-// refilled at row r is the one read at row r + ahead - kRing).  The acoustic
-// kernel, with the least arithmetic to hide the latency behind, gains from
-// three; the anisotropic ones run best with two.
+// Rows in flight ahead of the one being computed (at most one less than
+// the slots: the slot refilled at row r is the one read at row r + ahead -
+// slots).  The acoustic kernel, with the least arithmetic to hide the latency
+// behind, gains from three; the anisotropic ones run best with two.
 template <int APPROX>
 __host__ __device__ constexpr int ring_ahead() { return APPROX == kAcoustic ? 3 : 2; }
-static_assert(3 <= kRing - 1, "ring too small for the prefetch distance");
 
 // ring arrays per slot: U(t) leading row (all lanes), then U(t-1), kappa,
 // 1 + 2 eps, -2 (eps - delta), 2 (1 + delta), cos, sin (writer lanes)
@@ -101,13 +106,13 @@ template <int APPROX>
 __host__ __device__ constexpr int slot_quads() { return ring_arrays<APPROX>() * 32 + (fetched_halo<APPROX>() ? 2 : 0); }
 
 // shared exchange entries per warp: U(t) double-buffered (34 quads with the
-// fetched halo), plus the z derivative for the TTI cross term
+// fetched halo); TTI: one row for U(t), one for the z derivative of the cross term
 template <int APPROX>
-__host__ __device__ constexpr int xchg_quads() { return APPROX == kTTI ? 4 * 32 : 2 * 34; }
+__host__ __device__ constexpr int xchg_quads() { return 2 * (APPROX == kTTI ? 32 : 34); }
 
 template <int APPROX>
 __host__ __device__ constexpr int step_smem_bytes() {
-    return kWarpsPerBlock * (kRing * slot_quads<APPROX>() + xchg_quads<APPROX>()) * 16;
+    return kWarpsPerBlock * (ring_slots<APPROX>() * slot_quads<APPROX>() + xchg_quads<APPROX>()) * 16;
 }
 
 // Packed two-wide FP32 arithmetic (sm_100+ FFMA2 / FADD2 / FMUL2), written
@@ -239,14 +244,23 @@ __device__ __forceinline__ float2 update_pair(float2 k, float2 base, float2 pxx,
     return pfma2(hs, pxz, pfma2(az, pzz, pfma2(ax, pxx, base)));   // in written order
 }
 
+// Blocks per SM that the registers are held to.  Acoustic: five (96 registers,
+// no spill) against four: 8 shots of 601 x 2101 migrate in 114.6 ms instead of
+// 118.6, 64 shots of 601 x 1801 model in 124.1 instead of 125.8; six spill (132
+// and 171 ms).
 template <int APPROX>
-__host__ __device__ constexpr int step_min_blocks() { return APPROX == kTTI ? 3 : 4; }
+__host__ __device__ constexpr int step_min_blocks() { return APPROX == kAcoustic ? 5 : 4; }
 
 // Rows per trip of the interior march loop.  The nine-row register window
 // shifts by register moves once per trip (eight quads), so unrolling divides
 // those moves by this factor, as far as the registers allow.
 template <int APPROX>
-__host__ __device__ constexpr int interior_unroll() { return APPROX == kAcoustic ? 2 : 4; }
+__host__ __device__ constexpr int interior_unroll() { return APPROX == kAcoustic ? 2 : APPROX == kVTI ? 4 : 3; }
+
+// The same in the border: two rows a trip gain TTI 1 %, and cost the acoustic
+// and the VTI kernel 2 to 3 % (registers of their interior march).
+template <int APPROX>
+__host__ __device__ constexpr int edge_unroll() { return APPROX == kTTI ? 2 : 1; }
 
 template <int V>
 struct IntTag { static constexpr int value = V; };
@@ -263,8 +277,11 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    float4* __restrict__ ring = smem4 + wib * (kRing * SQ);
-    float4* __restrict__ xbuf = smem4 + kWarpsPerBlock * kRing * SQ + wib * xchg_quads<APPROX>();
+    constexpr int S = ring_slots<APPROX>();
+    float4* __restrict__ ring = smem4 + wib * (S * SQ);
+    float4* __restrict__ xbuf = smem4 + kWarpsPerBlock * S * SQ + wib * xchg_quads<APPROX>();
+    // three slots rotate by one a row (turn[0] is read at the current row)
+    [[maybe_unused]] float4* turn[3] = {ring, ring + SQ, ring + 2 * SQ};
 
     const int warp = blockIdx.x * kWarpsPerBlock + wib;
     const int shot = warp % a.B;
@@ -312,15 +329,15 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
 
     // prefetch ring, kAhead rows ahead: U(t) row r+4 (the queue's leading row)
     // for every lane; U(t-1) and the model arrays at row r for writer lanes.
-    auto issue = [&](int rr) {
-        float4* slot = ring + ((rr - z0) & (kRing - 1)) * SQ + lane;
+    auto issue = [&](int rr, [[maybe_unused]] int ahead) {
+        float4* slot = (S == 4 ? ring + ((rr - z0) & 3) * SQ : turn[ahead]) + lane;
         cp_async16(slot, PAM_CHK(cur + (long long)min(rr + 4, zmax) * P, a.cur, fbytes, 16, 1));
         if (XH && ((lane == 0 && tile > 0) || lane == 31)) {
             // the x halo quads of row rr: columns x0 - 4 (lane 0; tile 0 has no
             // left halo, and only its unwritten columns 0..3 would use it) and
             // x0 + 4 (lane 31)
             const long long ro = (long long)min(rr, zmax) * P;
-            cp_async16(ring + ((rr - z0) & (kRing - 1)) * SQ + NA * 32 + (lane == 0 ? 0 : 1),
+            cp_async16((S == 4 ? ring + ((rr - z0) & 3) * SQ : turn[ahead]) + NA * 32 + (lane == 0 ? 0 : 1),
                        PAM_CHK(cur + ro + (lane == 0 ? -4 : 4), a.cur, fbytes, 16, 2));
         }
         if (writer) {
@@ -340,7 +357,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         cp_async_commit();
     };
 #pragma unroll
-    for (int i = 0; i < kAhead; i++) issue(z0 + i);
+    for (int i = 0; i < kAhead; i++) issue(z0 + i, i);
 
     // One row of the march.  EDGE rows may lie in the absorbing border (Cerjan
     // damping, CPML strip terms, partial stores); interior rows are free of
@@ -349,9 +366,9 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     auto row = [&](auto edge_tag, int r, bool live, float4& Q0, float4& Q1, float4& Q2, float4& Q3, float4& Q4,
                    float4& Q5, float4& Q6, float4& Q7, float4& Q8) {
         constexpr bool EDGE = decltype(edge_tag)::value != 0;
-        issue(r + kAhead);
+        issue(r + kAhead, kAhead);
         cp_async_wait<kAhead>();
-        const float4* slot0 = ring + ((r - z0) & (kRing - 1)) * SQ;
+        const float4* slot0 = S == 4 ? ring + ((r - z0) & 3) * SQ : turn[0];
         const float4* slot = slot0 + lane;
         Q8 = slot[0];
         // CPML strip terms of this row, loaded before its arithmetic so that
@@ -390,7 +407,8 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
             left = xb[lane];
             right = xb[lane + 2];
         } else {
-            float4* xb = xbuf + (r & 1) * 32;
+            // one buffer: the row's second exchange separates its reads from the next row's stores
+            float4* xb = xbuf;
             xb[lane] = center;
             __syncwarp();
             left = xb[(lane + 31) & 31];
@@ -427,7 +445,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         if (APPROX == kTTI) {
             // cross derivative: x derivative of the z derivative (cpp/Modeling.cu:674-693
             // factorised), from the neighbours' pz through the second exchange row
-            float4* zb = xbuf + (2 + (r & 1)) * 32;
+            float4* zb = xbuf + 32;
             zb[lane] = make_float4(pz2v[0].x, pz2v[0].y, pz2v[1].x, pz2v[1].y);
             __syncwarp();
             const float4 pl = zb[(lane + 31) & 31];
@@ -524,6 +542,12 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
                     if (x0 + j >= 4 && x0 + j < a.nx - 4) *PAM_CHK(&nxt[ro + j], a.nxt, fbytes, 4, 17) = out[j];
             }
         }
+        if (S == 3) {
+            float4* const read = turn[0];
+            turn[0] = turn[1];
+            turn[1] = turn[2];
+            turn[2] = read;
+        }
     };
 
     // The march down the segment: register window w[0..7] = rows r-4 .. r+3,
@@ -551,7 +575,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     // border (only those rows carry damping or strip terms, and only x-border
     // tiles have columns outside [4, nx - 4)).
     const bool edge = xborder || z0 < a.N || z1 > a.nz - a.N;
-    if (edge) march(IntTag<1>{}, IntTag<1>{});
+    if (edge) march(IntTag<1>{}, IntTag<edge_unroll<APPROX>()>{});
     else march(IntTag<0>{}, IntTag<interior_unroll<APPROX>()>{});
     cp_async_wait<0>();
 }
