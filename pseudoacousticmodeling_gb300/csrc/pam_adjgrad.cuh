@@ -58,6 +58,7 @@ struct AdjGradArgs {
 
 __global__ void __launch_bounds__(128, 3) adjgrad_kernel(const AdjGradArgs ag)
 {
+    wait_chained();
     const StepArgs& a = ag.s;
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31;

@@ -324,7 +324,7 @@ static int aniso_height(int B, int ntiles, int rows, int resident) {
 }
 
 template <bool TTI>
-static void launch_aniso_t(AnisoArgs aa, float* nxt, const float* kap, cudaStream_t s) {
+static void launch_aniso_t(AnisoArgs aa, float* nxt, const float* kap, cudaStream_t s, bool chain) {
     static bool configured[64] = {};
     static int resident[64] = {};
     constexpr int smem = aniso_smem_bytes<TTI>();
@@ -343,14 +343,15 @@ static void launch_aniso_t(AnisoArgs aa, float* nxt, const float* kap, cudaStrea
     aa.H = aniso_height(aa.B, aa.ntiles, aa.g.nz - 8, resident[d]);
     aa.nseg = (aa.g.nz - 8 + aa.H - 1) / aa.H;
     const long long warps = (long long)aa.B * aa.ntiles * aa.nseg;
-    aniso_adjoint_kernel<TTI><<<(unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock), 32 * kWarpsPerBlock, smem, s>>>(
-        aa, nxt, kap);
+    launch_chained(chain, aniso_adjoint_kernel<TTI>, (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock),
+                   32 * kWarpsPerBlock, smem, s, aa, nxt, kap);
 }
 
-static cudaError_t launch_aniso_adjoint(const AnisoArgs& aa, float* nxt, const float* kap, cudaStream_t s) {
+static cudaError_t launch_aniso_adjoint(const AnisoArgs& aa, float* nxt, const float* kap, cudaStream_t s,
+                                        bool chain) {
     if (!aniso_operands_aligned(aa, nxt, kap)) return cudaErrorMisalignedAddress;
-    if (aa.tti) launch_aniso_t<true>(aa, nxt, kap, s);
-    else launch_aniso_t<false>(aa, nxt, kap, s);
+    if (aa.tti) launch_aniso_t<true>(aa, nxt, kap, s, chain);
+    else launch_aniso_t<false>(aa, nxt, kap, s, chain);
     return cudaSuccess;
 }
 
@@ -383,7 +384,8 @@ static void launch_adjgrad_kernel(const pam_engine* e, const AdjGradArgs& ag, cu
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     const long long warps = (long long)ag.Bp * ag.s.ntiles * ag.s.nseg;
-    adjgrad_kernel<<<(int)(warps / kWarpsPerBlock), 32 * kWarpsPerBlock, adjgrad_smem_bytes(), s>>>(ag);
+    launch_chained(e->chain_launches, adjgrad_kernel, (int)(warps / kWarpsPerBlock), 32 * kWarpsPerBlock,
+                   adjgrad_smem_bytes(), s, ag);
 }
 
 // Segment height of adjgrad_kernel for this batch size: the candidates are
@@ -464,6 +466,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     const TilePlan *ftiles = nullptr, *btiles = nullptr, *rtiles = nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &capturing));
+    chain_launches = capturing == cudaStreamCaptureStatusNone;
     if (capturing == cudaStreamCaptureStatusNone) {
         if (cfg.boundary != PAM_CPML || nseg <= 1) ftiles = tile_plan(nshots, kTileForwardLaunched);
         if (sb || rbc) rtiles = tile_plan(nshots, kTileReverse);
@@ -730,13 +733,14 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             // C++ loop (cpp/Migration.cu:383-390): t = nt-1 .. 0
             if (t >= itlag) {
                 const long long n = (long long)nrec * nshots;
-                inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
-                    ucur, d_obs, d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
+                launch_chained(chain_launches, inject_receivers_kernel, (int)((n + 255) / 256), 256, 0, st, ucur,
+                               d_obs, d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
             }
             {
                 cudaEvent_t pend;
                 prof_begin(t, 4, st, &pend);
-                imaging_sum_kernel<<<gquad, blk, 0, st>>>(ucur, Pt, d_img, d_img_ilum, g, nzi, nxi, pstride, nshots);
+                launch_chained(chain_launches, imaging_sum_kernel, gquad, blk, 0, st, ucur, Pt, d_img, d_img_ilum, g,
+                               nzi, nxi, pstride, nshots);
                 if (pend) cudaEventRecordWithFlags(pend, st, prof_flags);
             }
             if (cfg.approximation == PAM_ACOUSTIC) {
@@ -770,7 +774,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                 {
                     cudaEvent_t pend;
                     prof_begin(t, 3, st, &pend);
-                    if (launch_aniso_adjoint(aa, uprv, d_kap, st) != cudaSuccess) aniso_misaligned = true;
+                    if (launch_aniso_adjoint(aa, uprv, d_kap, st, chain_launches) != cudaSuccess) aniso_misaligned = true;
                     if (pend) cudaEventRecordWithFlags(pend, st, prof_flags);
                 }
             }
@@ -787,18 +791,17 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                     const float inv_dx = 1.0f / cfg.dx, inv_dz = 1.0f / cfg.dz;
                     const float inv_dx2 = 1.0f / (cfg.dx * cfg.dx), inv_dz2 = 1.0f / (cfg.dz * cfg.dz);
                     if (cfg.approximation == PAM_TTI)
-                        mp_grad_kernel<true><<<gsum, blk, 0, st>>>(Pt, Pm1, Pp1, ucur, pstride, d_eps, d_del, d_cth, d_sth,
-                                                                   d_mp, d_mp + interior, d_mp + 2 * interior, d_grad,
-                                                                   d_grad_ilum, g, nzi, nxi, nshots, inv_dx, inv_dz, inv_dx2,
-                                                                   inv_dz2, inv_dt2);
+                        launch_chained(chain_launches, mp_grad_kernel<true>, gsum, blk, 0, st, Pt, Pm1, Pp1, ucur,
+                                       pstride, d_eps, d_del, d_cth, d_sth, d_mp, d_mp + interior, d_mp + 2 * interior,
+                                       d_grad, d_grad_ilum, g, nzi, nxi, nshots, inv_dx, inv_dz, inv_dx2, inv_dz2,
+                                       inv_dt2);
                     else
-                        mp_grad_kernel<false><<<gsum, blk, 0, st>>>(Pt, Pm1, Pp1, ucur, pstride, d_eps, d_del, d_cth, d_sth,
-                                                                    d_mp, d_mp + interior, nullptr, d_grad, d_grad_ilum, g,
-                                                                    nzi, nxi, nshots, inv_dx, inv_dz, inv_dx2, inv_dz2,
-                                                                    inv_dt2);
+                        launch_chained(chain_launches, mp_grad_kernel<false>, gsum, blk, 0, st, Pt, Pm1, Pp1, ucur,
+                                       pstride, d_eps, d_del, d_cth, d_sth, d_mp, d_mp + interior, nullptr, d_grad,
+                                       d_grad_ilum, g, nzi, nxi, nshots, inv_dx, inv_dz, inv_dx2, inv_dz2, inv_dt2);
                 } else {
-                    fwi_ref_sum_kernel<<<gquad, blk, 0, st>>>(ucur, Pm1, Pt, Pp1, d_grad, d_grad_ilum, g, nzi, nxi, pstride,
-                                                              nshots, inv_dt2, step);
+                    launch_chained(chain_launches, fwi_ref_sum_kernel, gquad, blk, 0, st, ucur, Pm1, Pt, Pp1, d_grad,
+                                   d_grad_ilum, g, nzi, nxi, pstride, nshots, inv_dt2, step);
                 }
                 if (pend) cudaEventRecordWithFlags(pend, st, prof_flags);
             };
@@ -806,8 +809,8 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             if (step) {
                 if (t >= itlag) {
                     const long long n = (long long)nrec * nshots;
-                    inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
-                        ucur, d_obs, d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
+                    launch_chained(chain_launches, inject_receivers_kernel, (int)((n + 255) / 256), 256, 0, st, ucur,
+                                   d_obs, d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
                 }
                 sums();
                 if (cfg.approximation == PAM_ACOUSTIC) {
@@ -842,7 +845,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                     {
                         cudaEvent_t pend;
                         prof_begin(t, 3, st, &pend);
-                        if (launch_aniso_adjoint(aa, uprv, d_kap, st) != cudaSuccess) aniso_misaligned = true;
+                        if (launch_aniso_adjoint(aa, uprv, d_kap, st, chain_launches) != cudaSuccess) aniso_misaligned = true;
                         if (pend) cudaEventRecordWithFlags(pend, st, prof_flags);
                     }
                 }
@@ -861,8 +864,8 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             }
             if (t >= itlag) {
                 const long long n = (long long)nrec * nshots;
-                inject_adjoint_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
-                    uprv, d_obs, d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, d_kap, g);
+                launch_chained(chain_launches, inject_adjoint_kernel, (int)((n + 255) / 256), 256, 0, st, uprv, d_obs,
+                               d_rz, d_rx, nrec, nshots, t - itlag, nt_data, rec_per_shot, d_kap, g);
             }
             ubc ^= 1;
         }
@@ -877,8 +880,8 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         const size_t fb = (size_t)field * B, bytes = (size_t)field * nshots * 4;
         if (btiles) {
             const long long n = (long long)nrec * nshots;
-            inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
-                d_ub[0], d_obs, d_rz, d_rx, nrec, nshots, nt - 1 - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
+            launch_chained(chain_launches, inject_receivers_kernel, (int)((n + 255) / 256), 256, 0, st, d_ub[0], d_obs,
+                           d_rz, d_rx, nrec, nshots, nt - 1 - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
         }
         const float *s0 = d_u[(nt - 1) & 1], *s1 = d_u[nt & 1];   // S(t1 - 1), S(t1)
         for (int t1 = nt; t1 > 0; t1 -= kTileSegment) {
@@ -968,8 +971,9 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             if (mode == kRTM && t1 == nt) {
                 // the data of the last step; the tiles inject the next ones
                 const long long n = (long long)nrec * nshots;
-                inject_receivers_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(
-                    d_ub[0], d_obs, d_rz, d_rx, nrec, nshots, nt - 1 - itlag, nt_data, rec_per_shot, inv_dxdz, gnod);
+                launch_chained(chain_launches, inject_receivers_kernel, (int)((n + 255) / 256), 256, 0, st, d_ub[0],
+                               d_obs, d_rz, d_rx, nrec, nshots, nt - 1 - itlag, nt_data, rec_per_shot, inv_dxdz,
+                               gnod);
             }
             if (int rc = tile_adjoint(*btiles, mode == kExact ? kTileExactJob : kTileRtmJob, nshots, t0, t1, slot(t0), t0,
                                       d_obs, inv_dxdz, st))

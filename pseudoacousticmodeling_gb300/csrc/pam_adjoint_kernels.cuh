@@ -49,6 +49,7 @@ __global__ void inject_receivers_kernel(float* __restrict__ field, const float* 
                                         const int* __restrict__ rz, const int* __restrict__ rx, int nrec, int B,
                                         int it, int nt_data, int per_shot, float scale, GridDims g)
 {
+    wait_chained();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)nrec * B) return;
     const int r = (int)(i % nrec);
@@ -103,6 +104,7 @@ __global__ void residual_kernel(const float* __restrict__ dcal, const float* dob
 __global__ void imaging_sum_kernel(const float* __restrict__ ub, const float* __restrict__ P_, float* __restrict__ img,
                                    float* __restrict__ ilum, GridDims g, int nzi, int nxi, long long pstride, int B)
 {
+    wait_chained();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int zi = blockIdx.y * blockDim.y + threadIdx.y;
     const int xf0 = 4 * q;                                   // first field column of the quad
@@ -140,6 +142,7 @@ __global__ void fwi_ref_sum_kernel(const float* __restrict__ ub, const float* __
                                    const float* __restrict__ pf, float* __restrict__ grad, float* __restrict__ ilum,
                                    GridDims g, int nzi, int nxi, long long pstride, int B, float inv_dt2, int with_grad)
 {
+    wait_chained();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int zi = blockIdx.y * blockDim.y + threadIdx.y;
     const int xf0 = 4 * q;
@@ -244,6 +247,7 @@ __global__ void inject_adjoint_kernel(float* __restrict__ w, const float* __rest
                                       const int* __restrict__ rz, const int* __restrict__ rx, int nrec, int B, int it,
                                       int nt_data, int per_shot, const float* __restrict__ kap, GridDims g)
 {
+    wait_chained();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)nrec * B) return;
     const int r = (int)(i % nrec);
@@ -286,6 +290,7 @@ __global__ void __launch_bounds__(256) mp_grad_kernel(const float* __restrict__ 
                                                       int nxi, int B, float inv_dx, float inv_dz, float inv_dx2,
                                                       float inv_dz2, float inv_dt2)
 {
+    wait_chained();
     __shared__ float pzs[2][8][40];        // z derivatives of the block's rows, four columns more on each side
     const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 8;
     const int xi = x0 + threadIdx.x, zi = z0 + threadIdx.y;

@@ -151,6 +151,7 @@ template <bool TTI>
 __global__ void __launch_bounds__(128, aniso_min_blocks<TTI>()) aniso_adjoint_kernel(const AnisoArgs a, float* __restrict__ nxt,
                                                                         const float* __restrict__ kap)
 {
+    wait_chained();
     extern __shared__ float an_sm[];
     const GridDims& g = a.g;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;

@@ -113,6 +113,7 @@ int pam_engine::init(const pam_config& c, int dev) {
     pam_engine* e = this;
     cfg = c;
     device = dev;
+    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sm_count = 152;
     if (c.nz < 1 || c.nx < 1 || c.n_abc < 8 || c.nt < 1 || c.itlag < 0 || c.itlag >= c.nt || c.max_shots < 1)
         return fail(PAM_E_ARG, "invalid config: nz=%d nx=%d n_abc=%d nt=%d itlag=%d max_shots=%d (n_abc must be >= 8)",
                     c.nz, c.nx, c.n_abc, c.nt, c.itlag, c.max_shots);
@@ -440,30 +441,38 @@ int pam_engine::tune_segments(int nshots, cudaStream_t s) {
 
 constexpr int kMaxDevices = 64;
 
-template <int A, int BC>
-static void launch_step_t(const StepArgs& a, cudaStream_t s) {
-    const long long warps = (long long)a.B * a.ntiles * a.nseg;
-    const int blocks = (int)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
+template <int A, int BC, int MIN>
+static void launch_step_t(const StepArgs& a, int blocks, cudaStream_t s, bool chain) {
     constexpr int smem = step_smem_bytes<A>();
     // the shared-memory opt-in is a per-device attribute of the kernel
     static bool configured[kMaxDevices] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices || !configured[dev]) {
-        cudaFuncSetAttribute(step_kernel<A, BC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(step_kernel<A, BC, MIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (dev >= 0 && dev < kMaxDevices) configured[dev] = true;
     }
-    step_kernel<A, BC><<<blocks, 32 * kWarpsPerBlock, smem, s>>>(a);
+    // (after the strips the stream has joined another one: a plain launch)
+    if (BC == kCPML) step_kernel<A, BC, MIN><<<blocks, 32 * kWarpsPerBlock, smem, s>>>(a);
+    else launch_chained(chain, step_kernel<A, BC, MIN>, blocks, 32 * kWarpsPerBlock, smem, s, a);
+}
+
+template <int A, int BC>
+static void launch_step_a(const StepArgs& a, int sms, cudaStream_t s, bool chain) {
+    const long long warps = (long long)a.B * a.ntiles * a.nseg;
+    const int blocks = (int)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    if (A == kAcoustic && blocks > kStepBlocks * sms) launch_step_t<A, BC, A == kAcoustic ? 5 : kStepBlocks>(a, blocks, s, chain);
+    else launch_step_t<A, BC, kStepBlocks>(a, blocks, s, chain);
 }
 
 void pam_engine::launch_step(const StepArgs& a, cudaStream_t s, int boundary) const {
     const int A = cfg.approximation, BC = boundary >= 0 ? boundary : cfg.boundary;
-    if (A == PAM_ACOUSTIC && BC == PAM_CERJAN) launch_step_t<kAcoustic, kCerjan>(a, s);
-    else if (A == PAM_ACOUSTIC) launch_step_t<kAcoustic, kCPML>(a, s);
-    else if (A == PAM_VTI && BC == PAM_CERJAN) launch_step_t<kVTI, kCerjan>(a, s);
-    else if (A == PAM_VTI) launch_step_t<kVTI, kCPML>(a, s);
-    else if (BC == PAM_CERJAN) launch_step_t<kTTI, kCerjan>(a, s);
-    else launch_step_t<kTTI, kCPML>(a, s);
+    if (A == PAM_ACOUSTIC && BC == PAM_CERJAN) launch_step_a<kAcoustic, kCerjan>(a, sm_count, s, chain_launches);
+    else if (A == PAM_ACOUSTIC) launch_step_a<kAcoustic, kCPML>(a, sm_count, s, chain_launches);
+    else if (A == PAM_VTI && BC == PAM_CERJAN) launch_step_a<kVTI, kCerjan>(a, sm_count, s, chain_launches);
+    else if (A == PAM_VTI) launch_step_a<kVTI, kCPML>(a, sm_count, s, chain_launches);
+    else if (BC == PAM_CERJAN) launch_step_a<kTTI, kCerjan>(a, sm_count, s, chain_launches);
+    else launch_step_a<kTTI, kCPML>(a, sm_count, s, chain_launches);
 }
 
 void pam_engine::launch_cpml(int nshots, const float* cur, cudaStream_t s, float* psix, float* zetax, float2* xaux,
@@ -543,7 +552,7 @@ void pam_engine::launch_record(int nshots, const float* cur, float* seis, int it
     r.cerjan_on = cfg.boundary == PAM_CERJAN;
     r.shot_stride = shot_stride;
     const long long n = (long long)nrec * nshots;
-    record_kernel<<<(int)((n + 255) / 256), 256, 0, s>>>(r);
+    launch_chained(chain_launches, record_kernel, (int)((n + 255) / 256), 256, 0, s, r);
 }
 
 // Reset fields and memory variables and inject the step-0 source sample.
@@ -644,6 +653,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     const bool use_graph = std::getenv("PAM_NO_GRAPH") == nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &capturing));
+    chain_launches = capturing == cudaStreamCaptureStatusNone;
     const TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots) : nullptr;
     const int persist_h = use_graph && capturing == cudaStreamCaptureStatusNone && !tiles ? persistent_height(nshots) : 0;
     if (!tiles && !persist_h)   // the persistent paths set their own shapes
@@ -695,7 +705,8 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
         return PAM_OK;
     }
     GraphSet& gs = graph_sets[h_seis ? 1 : 0];
-    if (gs.execs.size() != (size_t)nchunks || gs.shots != nshots || gs.seis != d_seis) {
+    if (gs.execs.size() != (size_t)nchunks || gs.shots != nshots || gs.seis != d_seis ||
+        gs.chained != chain_launches) {
         drop_graphs(gs);
         cudaStream_t cs = capture_stream();
         if (!cs) return fail(PAM_E_CUDA, "could not create the capture stream");
@@ -727,6 +738,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
         }
         gs.shots = nshots;
         gs.seis = d_seis;
+        gs.chained = chain_launches;
     }
     if (!h_seis) {
         CU(cudaGraphLaunch(gs.execs[0], s));

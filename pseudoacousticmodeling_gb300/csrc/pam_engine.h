@@ -17,6 +17,7 @@ struct TileArgs;
 struct pam_engine {
     pam_config cfg{};
     int device = 0;
+    int sm_count = 152;
     bool broken = false;
     std::string err;
     int fail(int code, const char* fmt, ...);
@@ -65,7 +66,9 @@ struct pam_engine {
         std::vector<int> bounds;         // chunk c covers steps [bounds[c], bounds[c+1])
         int shots = -1;
         const float* seis = nullptr;
+        bool chained = false;            // chain_launches at its capture
     };
+    bool chain_launches = true;          // launch_chained(): not into a capture of the caller's
     GraphSet graph_sets[2];
     void drop_graphs(GraphSet& gs);
     cudaStream_t copy_stream = nullptr;  // seismogram downloads overlapping the next chunk,

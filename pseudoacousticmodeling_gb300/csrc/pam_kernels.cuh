@@ -33,6 +33,7 @@
 #include <stdint.h>
 
 #include "pam_check.cuh"
+#include "pam_launch.cuh"
 #include "pam_types.h"
 
 namespace pam {
@@ -244,12 +245,8 @@ __device__ __forceinline__ float2 update_pair(float2 k, float2 base, float2 pxx,
     return pfma2(hs, pxz, pfma2(az, pzz, pfma2(ax, pxx, base)));   // in written order
 }
 
-// Blocks per SM that the registers are held to.  Acoustic: five (96 registers,
-// no spill) against four: 8 shots of 601 x 2101 migrate in 114.6 ms instead of
-// 118.6, 64 shots of 601 x 1801 model in 124.1 instead of 125.8; six spill (132
-// and 171 ms).
-template <int APPROX>
-__host__ __device__ constexpr int step_min_blocks() { return APPROX == kAcoustic ? 5 : 4; }
+// Blocks per SM that the registers of a step are held to.
+constexpr int kStepBlocks = 4;
 
 // Rows per trip of the interior march loop.  The nine-row register window
 // shifts by register moves once per trip (eight quads), so unrolling divides
@@ -580,9 +577,16 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     cp_async_wait<0>();
 }
 
-template <int APPROX, int BC>
-__global__ void __launch_bounds__(128, step_min_blocks<APPROX>()) step_kernel(const StepArgs a)
+// MIN: blocks per SM that the registers are held to.  Acoustic grids of more than
+// kStepBlocks a SM run with five (96 registers, no spill): 8 shots of 601 x 2101
+// migrate in 114.6 ms against 118.6 with four, 64 shots of 601 x 1801 model in
+// 124.1 against 125.8, 16 CPML shots of 600 x 1800 take 70.7 us a step against
+// 73.7; six spill (132 and 171 ms).  Smaller grids have no use for a fifth block:
+// three CPML shots of 500 x 1100 take 13.4 us with its registers, 13.0 without.
+template <int APPROX, int BC, int MIN>
+__global__ void __launch_bounds__(128, MIN) step_kernel(const StepArgs a)
 {
+    wait_chained();
     step_body<APPROX, BC>(a);
 }
 
@@ -957,6 +961,7 @@ __device__ __forceinline__ void record_sample(const RecordArgs& a, long long i)
 
 static __global__ void record_kernel(const RecordArgs a)
 {
+    wait_chained();
     record_sample(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -977,7 +982,7 @@ struct PersistArgs {
 };
 
 template <int APPROX, int BC>
-__global__ void __launch_bounds__(128, step_min_blocks<APPROX>()) step_persistent_kernel(const PersistArgs p)
+__global__ void __launch_bounds__(128, kStepBlocks) step_persistent_kernel(const PersistArgs p)
 {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
