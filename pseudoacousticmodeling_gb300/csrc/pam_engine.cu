@@ -452,9 +452,7 @@ static void launch_step_t(const StepArgs& a, int blocks, cudaStream_t s, bool ch
         cudaFuncSetAttribute(step_kernel<A, BC, MIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (dev >= 0 && dev < kMaxDevices) configured[dev] = true;
     }
-    // (after the strips the stream has joined another one: a plain launch)
-    if (BC == kCPML) step_kernel<A, BC, MIN><<<blocks, 32 * kWarpsPerBlock, smem, s>>>(a);
-    else launch_chained(chain, step_kernel<A, BC, MIN>, blocks, 32 * kWarpsPerBlock, smem, s, a);
+    launch_chained(chain, step_kernel<A, BC, MIN>, blocks, 32 * kWarpsPerBlock, smem, s, a);
 }
 
 template <int A, int BC>
@@ -465,14 +463,33 @@ static void launch_step_a(const StepArgs& a, int sms, cudaStream_t s, bool chain
     else launch_step_t<A, BC, kStepBlocks>(a, blocks, s, chain);
 }
 
+// Largest batch (cells) whose strips go as one chained launch in a stream.  As two
+// kernels on forked streams they cost four event operations a step; as one
+// kernel the x strips get the registers of the z strips, hence fewer warps.
+// CPML migration, us a step, forked -> one launch: 0.87 M cells 37.9 -> 30.7, 2.9 M
+// 69.1 -> 58.3, 8.6 M 142 -> 127, 17 M 233 -> 225, 35 M 421 -> 417.  In a graph the
+// fork costs little and wins at every size (1.7 M cells 12.7 against 13.3 us a
+// step, 121 M VTI 460 against 513).
+constexpr double kChainedStripCells = 4e7;
+
+// Whether a step's strips go as one launch (see kChainedStripCells), the stepping
+// kernel chained behind them.
+bool pam_engine::strips_chained(int nshots, cudaStream_t s) const {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    return chain_launches && (double)nshots * nza * nxa <= kChainedStripCells &&
+           cudaStreamIsCapturing(s, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone;
+}
+
 void pam_engine::launch_step(const StepArgs& a, cudaStream_t s, int boundary) const {
     const int A = cfg.approximation, BC = boundary >= 0 ? boundary : cfg.boundary;
-    if (A == PAM_ACOUSTIC && BC == PAM_CERJAN) launch_step_a<kAcoustic, kCerjan>(a, sm_count, s, chain_launches);
-    else if (A == PAM_ACOUSTIC) launch_step_a<kAcoustic, kCPML>(a, sm_count, s, chain_launches);
-    else if (A == PAM_VTI && BC == PAM_CERJAN) launch_step_a<kVTI, kCerjan>(a, sm_count, s, chain_launches);
-    else if (A == PAM_VTI) launch_step_a<kVTI, kCPML>(a, sm_count, s, chain_launches);
-    else if (BC == PAM_CERJAN) launch_step_a<kTTI, kCerjan>(a, sm_count, s, chain_launches);
-    else launch_step_a<kTTI, kCPML>(a, sm_count, s, chain_launches);
+    // (behind strips on two streams a step follows their join: a plain launch)
+    const bool chain = BC == PAM_CPML ? strips_chained(a.B, s) : chain_launches;
+    if (A == PAM_ACOUSTIC && BC == PAM_CERJAN) launch_step_a<kAcoustic, kCerjan>(a, sm_count, s, chain);
+    else if (A == PAM_ACOUSTIC) launch_step_a<kAcoustic, kCPML>(a, sm_count, s, chain);
+    else if (A == PAM_VTI && BC == PAM_CERJAN) launch_step_a<kVTI, kCerjan>(a, sm_count, s, chain);
+    else if (A == PAM_VTI) launch_step_a<kVTI, kCPML>(a, sm_count, s, chain);
+    else if (BC == PAM_CERJAN) launch_step_a<kTTI, kCerjan>(a, sm_count, s, chain);
+    else launch_step_a<kTTI, kCPML>(a, sm_count, s, chain);
 }
 
 void pam_engine::launch_cpml(int nshots, const float* cur, cudaStream_t s, float* psix, float* zetax, float2* xaux,
@@ -499,35 +516,33 @@ void pam_engine::launch_cpml(int nshots, const float* cur, cudaStream_t s, float
     c.inv_dz = 1.0f / cfg.dz;
     c.inv_dx2 = 1.0f / (cfg.dx * cfg.dx);
     c.inv_dz2 = 1.0f / (cfg.dz * cfg.dz);
+    const bool xpair = N % 2 == 0, zpair = cpml_z_pairs_usable(N);
     const CpmlXShape xs = cpml_x_shape(N);
-    const dim3 xgrid(2, (nza - 8 + xs.rows - 1) / xs.rows, nshots);
+    const CpmlXPairShape xp = cpml_x_pair_shape(N);
+    const int xbx = xpair ? xp.bx : xs.bx, xrows = xpair ? xp.rows : xs.rows, xthreads = xbx * xrows;
+    const int zrows = zpair ? cpml_z_pair_block_rows(N) : cpml_z_block_rows(N);
+    const int zthreads = zrows * (zpair ? kCpmlZCols / 2 : kCpmlZCols);
+    const int nrb = (nza - 8 + xrows - 1) / xrows, nslab = (nxa - 8 + kCpmlZCols - 1) / kCpmlZCols;
+    const size_t xsmem = (size_t)xrows * ((xpair ? 2 * xbx : xbx) + 8) * sizeof(float);
+    const size_t zsmem = (size_t)(zrows * (zpair ? kCpmlZPairRows : kCpmlZRows) + 8) * kCpmlZCols * sizeof(float);
+    if (strips_chained(nshots, s)) {
+        const int xblocks = 2 * nrb * nshots, blocks = xblocks + 2 * nslab * nshots;
+        auto* kernel = xpair ? (zpair ? cpml_strips_kernel<true, true> : cpml_strips_kernel<true, false>)
+                             : (zpair ? cpml_strips_kernel<false, true> : cpml_strips_kernel<false, false>);
+        launch_chained(true, kernel, blocks, std::max(xthreads, zthreads), std::max(xsmem, zsmem), s, c, xblocks, nrb,
+                       nslab);
+        return;
+    }
     // the x and z strips write disjoint arrays and both only read U(t): the
     // x strips (latency-bound, small blocks) run on strip_stream beside the z
     // strips, joined back into s before anything reads the strip terms
     cudaEventRecord(strip_events[0], s);
     cudaStreamWaitEvent(strip_stream, strip_events[0], 0);
-    if (N % 2 == 0) {
-        const CpmlXPairShape xp = cpml_x_pair_shape(N);
-        const dim3 xpgrid(2, (nza - 8 + xp.rows - 1) / xp.rows, nshots);
-        cpml_x_pair_kernel<<<xpgrid, dim3(xp.bx, xp.rows), xp.rows * (2 * xp.bx + 8) * sizeof(float), strip_stream>>>(
-            c);
-    } else {
-        cpml_x_kernel<<<xgrid, dim3(xs.bx, xs.rows), xs.rows * (xs.bx + 8) * sizeof(float), strip_stream>>>(c);
-    }
-    const int nslab = (nxa - 8 + kCpmlZCols - 1) / kCpmlZCols;
-    const dim3 zgrid(nslab, 2, nshots);
-    const int zrows = cpml_z_block_rows(N), R = cpml_z_rows_per_thread(N);
-    const dim3 zblock(kCpmlZCols, zrows);
-    const size_t zsmem = (size_t)(zrows * R + 8) * kCpmlZCols * sizeof(float);
-    if (cpml_z_pairs_usable(N)) {
-        const int zprows = cpml_z_pair_block_rows(N);
-        const size_t zpsmem = (size_t)(zprows * kCpmlZPairRows + 8) * kCpmlZCols * sizeof(float);
-        cpml_z_pair_kernel<<<zgrid, dim3(kCpmlZCols / 2, zprows), zpsmem, s>>>(c);
-    } else if (R == 6) {
-        cpml_z_kernel<6><<<zgrid, zblock, zsmem, s>>>(c);
-    } else {
-        cpml_z_kernel<8><<<zgrid, zblock, zsmem, s>>>(c);
-    }
+    const dim3 xgrid(2, nrb, nshots), zgrid(nslab, 2, nshots);
+    if (xpair) cpml_x_kernel<true><<<xgrid, xthreads, xsmem, strip_stream>>>(c);
+    else cpml_x_kernel<false><<<xgrid, xthreads, xsmem, strip_stream>>>(c);
+    if (zpair) cpml_z_kernel<true><<<zgrid, zthreads, zsmem, s>>>(c);
+    else cpml_z_kernel<false><<<zgrid, zthreads, zsmem, s>>>(c);
     cudaEventRecord(strip_events[1], strip_stream);
     cudaStreamWaitEvent(s, strip_events[1], 0);
 }

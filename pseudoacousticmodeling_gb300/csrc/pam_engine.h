@@ -54,8 +54,8 @@ struct pam_engine {
 
     // streams and graph
     cudaStream_t own_stream = nullptr, stream = nullptr, cap_stream = nullptr;
-    // the CPML x strips run on strip_stream beside the z strips (fork / join
-    // by the two events around each strip update)
+    // the CPML x strips of captured and of large steps run on strip_stream beside
+    // the z strips (fork / join by the two events around each strip update)
     cudaStream_t strip_stream = nullptr;
     cudaEvent_t strip_events[2] = {nullptr, nullptr};
     // the forward time loop as a chain of graphs over consecutive time chunks:
@@ -137,6 +137,7 @@ struct pam_engine {
     void invalidate_graph();
     pam::StepArgs step_args(int k, int nshots, const float* cur, float* nxt, int fwd_src) const;
     void launch_step(const pam::StepArgs& a, cudaStream_t s, int boundary = -1) const;
+    bool strips_chained(int nshots, cudaStream_t s) const;
     void launch_cpml(int nshots, const float* cur, cudaStream_t s, float* psix, float* zetax, float2* xaux,
                      float* psiz, float* zetaz, float2* zaux) const;
     void launch_record(int nshots, const float* cur, float* seis, int it, cudaStream_t s) const;

@@ -613,16 +613,15 @@ __host__ __device__ inline CpmlXShape cpml_x_shape(int N) {
     return CpmlXShape{bx, rows};
 }
 
-static __global__ void __launch_bounds__(256) cpml_x_kernel(const CpmlArgs a)
+__device__ __forceinline__ void cpml_x_strip(const CpmlArgs& a, int side, int rb, int shot)
 {
     extern __shared__ float xsm[];                  // [rows][bx + 8]
-    // grid: (side, row block, shot)
     const CpmlXShape sh = cpml_x_shape(a.N);
     const int W = a.N - 4;
-    const int side = blockIdx.x, rb = blockIdx.y, shot = blockIdx.z;
-    const int i = threadIdx.x, ty = threadIdx.y;
+    const int i = threadIdx.x % sh.bx, ty = threadIdx.x / sh.bx;
     const int z = 4 + rb * sh.rows + ty;
-    const bool valid = i < W && z < a.nz - 4;
+    const bool mine = ty < sh.rows;                 // (the block may have more threads than the strip rows)
+    const bool valid = mine && i < W && z < a.nz - 4;
     float* srow = xsm + ty * (sh.bx + 8);
     const int xbeg = side == 0 ? 4 : a.nx - a.N;    // first strip column
     const int cbeg = side == 0 ? 4 : a.N;           // its index in the [2N] strip row
@@ -648,10 +647,10 @@ static __global__ void __launch_bounds__(256) cpml_x_kernel(const CpmlArgs a)
         const float ps = ab.x * ps_old + ab.y * px;
         *PAM_CHK(&a.psix[so], a.psix, sbytes, 4, 22) = ps;
         srow[i + 4] = ps;
-    } else if (i < sh.bx) {
+    } else if (mine) {
         srow[i + 4] = 0.0f;
     }
-    if (i < 4) { srow[i] = 0.0f; srow[sh.bx + 4 + i] = 0.0f; }
+    if (mine && i < 4) { srow[i] = 0.0f; srow[sh.bx + 4 + i] = 0.0f; }
     __syncthreads();
     if (!valid) return;
     const float* sr = srow + i + 4;
@@ -666,8 +665,8 @@ static __global__ void __launch_bounds__(256) cpml_x_kernel(const CpmlArgs a)
 // even strip-row offsets): one thread per pair of x-adjacent strip cells, so
 // psi, zeta, the (a, b) pairs and the strip terms move as 8- and 16-byte
 // accesses and U's ten taps of the pair are read once; per cell the same
-// expressions as cpml_x_kernel.  A block covers `rows` strip rows of one
-// (shot, side): blockDim = (pairs per row rounded up to 8, rows).
+// expressions as cpml_x_strip.  A block covers `rows` strip rows of one
+// (shot, side), pairs per row rounded up to 8.
 struct CpmlXPairShape {
     int bx, rows;
 };
@@ -679,17 +678,16 @@ __host__ __device__ inline CpmlXPairShape cpml_x_pair_shape(int N) {
     return CpmlXPairShape{bx, rows};
 }
 
-static __global__ void __launch_bounds__(256) cpml_x_pair_kernel(const CpmlArgs a)
+__device__ __forceinline__ void cpml_x_pair_strip(const CpmlArgs& a, int side, int rb, int shot)
 {
     extern __shared__ float xpsm[];                 // [rows][2 bx + 8]
-    // grid: (side, row block, shot)
     const CpmlXPairShape sh = cpml_x_pair_shape(a.N);
     const int pairs = (a.N - 4) / 2;
-    const int side = blockIdx.x, rb = blockIdx.y, shot = blockIdx.z;
-    const int j = threadIdx.x, ty = threadIdx.y;
+    const int j = threadIdx.x % sh.bx, ty = threadIdx.x / sh.bx;
     const int i = 2 * j;                            // first strip column of the pair
     const int z = 4 + rb * sh.rows + ty;
-    const bool valid = j < pairs && z < a.nz - 4;
+    const bool mine = ty < sh.rows;
+    const bool valid = mine && j < pairs && z < a.nz - 4;
     float* srow = xpsm + ty * (2 * sh.bx + 8);
     const int xbeg = side == 0 ? 4 : a.nx - a.N;    // first strip column
     const int cbeg = side == 0 ? 4 : a.N;           // its index in the [2N] strip row
@@ -724,11 +722,11 @@ static __global__ void __launch_bounds__(256) cpml_x_pair_kernel(const CpmlArgs 
         *reinterpret_cast<float2*>(PAM_CHK(&a.psix[so], a.psix, sbytes, 8, 26)) = make_float2(ps0, ps1);
         srow[i + 4] = ps0;
         srow[i + 5] = ps1;
-    } else if (j < sh.bx) {
+    } else if (mine) {
         srow[i + 4] = 0.0f;                         // psi is zero past the strip
         srow[i + 5] = 0.0f;
     }
-    if (j < 4) { srow[j] = 0.0f; srow[2 * sh.bx + 4 + j] = 0.0f; }
+    if (mine && j < 4) { srow[j] = 0.0f; srow[2 * sh.bx + 4 + j] = 0.0f; }
     __syncthreads();
     if (!valid) return;
     const float* sr = srow + i + 4;                 // cell 0 at sr[0], cell 1 at sr[1]
@@ -745,26 +743,22 @@ static __global__ void __launch_bounds__(256) cpml_x_pair_kernel(const CpmlArgs 
 
 // z strips: a block covers 32 columns and the whole strip height of one
 // (shot, side); each thread owns R consecutive strip rows of one column
-// (blockDim = (32, ceil(W / R))), so it reads the R + 8 rows of U its
+// (32 x ceil(W / R) threads), so it reads the R + 8 rows of U its
 // stencils need once.  All loads of a thread are issued before its
 // arithmetic; psi_new goes through shared memory (four zero rows above and
 // below the strip) for its z derivative.
 constexpr int kCpmlZCols = 32;
 
-__host__ __device__ inline int cpml_z_rows_per_thread(int N) { return N - 4 <= 6 * 32 ? 6 : 8; }
-__host__ __device__ inline int cpml_z_block_rows(int N) {
-    const int R = cpml_z_rows_per_thread(N);
-    return (N - 4 + R - 1) / R;
-}
+constexpr int kCpmlZRows = 8;
 
-template <int R>
-__global__ void __launch_bounds__(1024) cpml_z_kernel(const CpmlArgs a)
+__host__ __device__ inline int cpml_z_block_rows(int N) { return (N - 4 + kCpmlZRows - 1) / kCpmlZRows; }
+
+__device__ __forceinline__ void cpml_z_strip(const CpmlArgs& a, int slab, int side, int shot)
 {
+    constexpr int R = kCpmlZRows;
     extern __shared__ float zsm[];                  // [by * R + 8][32]
-    // grid: (column slab, side, shot)
     const int W = a.N - 4;
-    const int slab = blockIdx.x, side = blockIdx.y, shot = blockIdx.z;
-    const int tx = threadIdx.x, ty = threadIdx.y, by = blockDim.y;
+    const int tx = threadIdx.x % kCpmlZCols, ty = threadIdx.x / kCpmlZCols, by = cpml_z_block_rows(a.N);
     const int x = 4 + slab * kCpmlZCols + tx;
     const bool xv = x < a.nx - 4;
     const int zbeg = side == 0 ? 4 : a.nz - a.N;    // first strip row
@@ -831,10 +825,10 @@ __global__ void __launch_bounds__(1024) cpml_z_kernel(const CpmlArgs a)
 
 // z strips in pairs of columns: a block covers 32 columns (16 pairs) and the
 // whole strip height of one (shot, side), each thread 3 consecutive strip
-// rows of one pair of columns (blockDim = (16, ceil(W / 3)), at most 64 rows,
+// rows of one pair of columns (16 x ceil(W / 3) threads, at most 64 rows,
 // so strips up to 192 cells high), reading the 11 rows of U its stencils need
 // as 8-byte pairs; psi, zeta and the strip terms move as 8- and 16-byte
-// accesses.  Per cell the same expressions as cpml_z_kernel.
+// accesses.  Per cell the same expressions as cpml_z_strip.
 constexpr int kCpmlZPairRows = 3;
 
 __host__ __device__ inline int cpml_z_pair_block_rows(int N) {
@@ -842,14 +836,13 @@ __host__ __device__ inline int cpml_z_pair_block_rows(int N) {
 }
 __host__ __device__ inline bool cpml_z_pairs_usable(int N) { return cpml_z_pair_block_rows(N) <= 64; }
 
-static __global__ void __launch_bounds__(1024) cpml_z_pair_kernel(const CpmlArgs a)
+__device__ __forceinline__ void cpml_z_pair_strip(const CpmlArgs& a, int slab, int side, int shot)
 {
     constexpr int R = kCpmlZPairRows;
     extern __shared__ float zpsm[];                 // [by * R + 8][32]
-    // grid: (column slab, side, shot)
     const int W = a.N - 4;
-    const int slab = blockIdx.x, side = blockIdx.y, shot = blockIdx.z;
-    const int tx = threadIdx.x, ty = threadIdx.y, by = blockDim.y;
+    const int tx = threadIdx.x % (kCpmlZCols / 2), ty = threadIdx.x / (kCpmlZCols / 2);
+    const int by = cpml_z_pair_block_rows(a.N);     // (thread rows past it own no strip row)
     const int x = 4 + slab * kCpmlZCols + 2 * tx;   // first column of the pair (even)
     const bool xv0 = x < a.nx - 4, xv1 = x + 1 < a.nx - 4;
     const int zbeg = side == 0 ? 4 : a.nz - a.N;    // first strip row
@@ -931,6 +924,42 @@ static __global__ void __launch_bounds__(1024) cpml_z_pair_kernel(const CpmlArgs
             *PAM_CHK(&a.zetaz[so + k * P], a.zetaz, sbytes, 4, 37) = ze0;
             *PAM_CHK(&a.zaux[so + k * P], a.zaux, 2 * sbytes, 8, 37) = make_float2(dps0, dps0 + ze0);
         }
+    }
+}
+
+// The strips of a step as one kernel each: blocks (side, row block, shot) of the x
+// strips, (column slab, side, shot) of the z strips.
+template <bool PAIR>
+__global__ void __launch_bounds__(256) cpml_x_kernel(const CpmlArgs a)
+{
+    if (PAIR) cpml_x_pair_strip(a, blockIdx.x, blockIdx.y, blockIdx.z);
+    else cpml_x_strip(a, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+template <bool PAIR>
+__global__ void __launch_bounds__(1024) cpml_z_kernel(const CpmlArgs a)
+{
+    if (PAIR) cpml_z_pair_strip(a, blockIdx.x, blockIdx.y, blockIdx.z);
+    else cpml_z_strip(a, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Both strips of a step in one chained launch: the first xblocks blocks (side, row
+// block, shot) are x strips, the others (column slab, side, shot) z strips; they
+// write disjoint arrays and only read U(t).
+template <bool XPAIR, bool ZPAIR>
+__global__ void __launch_bounds__(1024) cpml_strips_kernel(const CpmlArgs a, int xblocks, int nrb, int nslab)
+{
+    wait_chained();
+    int b = blockIdx.x;
+    if (b < xblocks) {
+        const int side = b & 1, rb = (b >> 1) % nrb, shot = (b >> 1) / nrb;
+        if (XPAIR) cpml_x_pair_strip(a, side, rb, shot);
+        else cpml_x_strip(a, side, rb, shot);
+    } else {
+        b -= xblocks;
+        const int slab = b % nslab, side = (b / nslab) & 1, shot = b / (2 * nslab);
+        if (ZPAIR) cpml_z_pair_strip(a, slab, side, shot);
+        else cpml_z_strip(a, slab, side, shot);
     }
 }
 
