@@ -459,8 +459,9 @@ template <int A, int BC>
 static void launch_step_a(const StepArgs& a, int sms, cudaStream_t s, bool chain) {
     const long long warps = (long long)a.B * a.ntiles * a.nseg;
     const int blocks = (int)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    if (A == kAcoustic && blocks > kStepBlocks * sms) launch_step_t<A, BC, A == kAcoustic ? 5 : kStepBlocks>(a, blocks, s, chain);
-    else launch_step_t<A, BC, kStepBlocks>(a, blocks, s, chain);
+    constexpr int kMany = A == kAcoustic ? 5 : 4;
+    if (blocks > 4 * sms) launch_step_t<A, BC, kMany>(a, blocks, s, chain);
+    else launch_step_t<A, BC, 4>(a, blocks, s, chain);
 }
 
 // Largest batch (cells) whose strips go as one chained launch in a stream.  As two
@@ -669,7 +670,9 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &capturing));
     chain_launches = capturing == cudaStreamCaptureStatusNone;
-    const TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots) : nullptr;
+    // (a run into the caller's device buffer returns at once: others may share the GPU)
+    const TileJob job = d_seis == d_seis_own ? kTileForward : kTileForwardAsync;
+    const TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots, job) : nullptr;
     const int persist_h = use_graph && capturing == cudaStreamCaptureStatusNone && !tiles ? persistent_height(nshots) : 0;
     if (!tiles && !persist_h)   // the persistent paths set their own shapes
         if (int rc = tune_segments(nshots, s)) return rc;
@@ -785,7 +788,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
 
 template <int A, int BC>
 static cudaError_t launch_persistent_t(const PersistArgs& p, int blocks, cudaStream_t s) {
-    constexpr int smem = step_smem_bytes<A>();
+    constexpr int smem = step_smem_bytes<A, 4>();
     static bool configured[kMaxDevices] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -805,7 +808,7 @@ static int persistent_capacity() {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    constexpr int smem = step_smem_bytes<A>();
+    constexpr int smem = step_smem_bytes<A, 4>();
     cudaFuncSetAttribute(step_persistent_kernel<A, BC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, step_persistent_kernel<A, BC>, 32 * kWarpsPerBlock,
                                                       smem) != cudaSuccess)

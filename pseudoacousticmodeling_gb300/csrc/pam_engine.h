@@ -165,8 +165,9 @@ struct pam_engine {
         int T = 0, TZ = 0, TX = 0, nty = 0, ntx = 0, R = 0, halo = 4;
         int group = 0;                   // shots per launch
     };
-    enum TileJob { kTileForward = 0, kTileExactJob = 1, kTileRtmJob = 2, kTileReverse = 3, kTileForwardLaunched = 4 };
-    std::map<int, TilePlan> tile_plans[5];
+    enum TileJob { kTileForward = 0, kTileExactJob = 1, kTileRtmJob = 2, kTileReverse = 3, kTileForwardLaunched = 4,
+                   kTileForwardAsync = 5 };
+    std::map<int, TilePlan> tile_plans[6];
     const TilePlan* tile_plan(int nshots, TileJob job = kTileForward);
     int tile_buffers(cudaStream_t s);
     int tile_begin(const TilePlan& p, cudaStream_t s);

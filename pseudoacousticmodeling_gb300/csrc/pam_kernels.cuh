@@ -111,9 +111,9 @@ __host__ __device__ constexpr int slot_quads() { return ring_arrays<APPROX>() * 
 template <int APPROX>
 __host__ __device__ constexpr int xchg_quads() { return 2 * (APPROX == kTTI ? 32 : 34); }
 
-template <int APPROX>
+template <int APPROX, int S = ring_slots<APPROX>()>
 __host__ __device__ constexpr int step_smem_bytes() {
-    return kWarpsPerBlock * (ring_slots<APPROX>() * slot_quads<APPROX>() + xchg_quads<APPROX>()) * 16;
+    return kWarpsPerBlock * (S * slot_quads<APPROX>() + xchg_quads<APPROX>()) * 16;
 }
 
 // Packed two-wide FP32 arithmetic (sm_100+ FFMA2 / FADD2 / FMUL2), written
@@ -245,9 +245,6 @@ __device__ __forceinline__ float2 update_pair(float2 k, float2 base, float2 pxx,
     return pfma2(hs, pxz, pfma2(az, pzz, pfma2(ax, pxx, base)));   // in written order
 }
 
-// Blocks per SM that the registers of a step are held to.
-constexpr int kStepBlocks = 4;
-
 // Rows per trip of the interior march loop.  The nine-row register window
 // shifts by register moves once per trip (eight quads), so unrolling divides
 // those moves by this factor, as far as the registers allow.
@@ -264,7 +261,8 @@ struct IntTag { static constexpr int value = V; };
 
 // One time step of this thread's warp (its shot, tile and segment): the
 // body of step_kernel, also run once per step by step_persistent_kernel.
-template <int APPROX, int BC>
+// EU: rows a trip in the border, S: ring slots.
+template <int APPROX, int BC, int EU = edge_unroll<APPROX>(), int S = ring_slots<APPROX>()>
 __device__ __forceinline__ void step_body(const StepArgs& a)
 {
     constexpr int NA = ring_arrays<APPROX>();
@@ -274,7 +272,6 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    constexpr int S = ring_slots<APPROX>();
     float4* __restrict__ ring = smem4 + wib * (S * SQ);
     float4* __restrict__ xbuf = smem4 + kWarpsPerBlock * S * SQ + wib * xchg_quads<APPROX>();
     // three slots rotate by one a row (turn[0] is read at the current row)
@@ -572,13 +569,13 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     // border (only those rows carry damping or strip terms, and only x-border
     // tiles have columns outside [4, nx - 4)).
     const bool edge = xborder || z0 < a.N || z1 > a.nz - a.N;
-    if (edge) march(IntTag<1>{}, IntTag<edge_unroll<APPROX>()>{});
+    if (edge) march(IntTag<1>{}, IntTag<EU>{});
     else march(IntTag<0>{}, IntTag<interior_unroll<APPROX>()>{});
     cp_async_wait<0>();
 }
 
 // MIN: blocks per SM that the registers are held to.  Acoustic grids of more than
-// kStepBlocks a SM run with five (96 registers, no spill): 8 shots of 601 x 2101
+// four blocks a SM run with five (96 registers, no spill): 8 shots of 601 x 2101
 // migrate in 114.6 ms against 118.6 with four, 64 shots of 601 x 1801 model in
 // 124.1 against 125.8, 16 CPML shots of 600 x 1800 take 70.7 us a step against
 // 73.7; six spill (132 and 171 ms).  Smaller grids have no use for a fifth block:
@@ -1010,8 +1007,11 @@ struct PersistArgs {
     int nt, itlag, k0, k1;
 };
 
+// (Segments of a row or two: one border row a trip and the four-slot ring, three
+// TTI blocks a SM; with the ring and the four blocks of step_kernel four TTI
+// shots of 364 x 464 took 7.7 us a step instead of 6.9.)
 template <int APPROX, int BC>
-__global__ void __launch_bounds__(128, kStepBlocks) step_persistent_kernel(const PersistArgs p)
+__global__ void __launch_bounds__(128, APPROX == kTTI ? 3 : 4) step_persistent_kernel(const PersistArgs p)
 {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(128, kStepBlocks) step_persistent_kernel(const
             r.it = k - p.itlag;
             record_sample(r, gtid);
         }
-        step_body<APPROX, BC>(a);
+        step_body<APPROX, BC, 1, 4>(a);   // (segments of a row or two)
         grid.sync();
     }
 }

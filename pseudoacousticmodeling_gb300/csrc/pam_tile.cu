@@ -41,6 +41,16 @@ constexpr double kTileSumUs[3] = {0.0, 4.0e-4, 1.5e-4};
 // acoustic, 6.9 to 10.3 us VTI, 7.6 to 10.2 us TTI)
 constexpr double kGraphStepUs[3] = {5.5, 6.6, 7.2}, kGraphCellUs[3] = {1.6e-6, 2.1e-6, 3.5e-6};
 
+// ... and of a step of the graph where the callers of three engines keep the GPU
+// busy together, which an asynchronous run (device output) allows and a
+// cooperative launch, taking every SM, does not (three engines in turn, measured:
+// CPML of 0.18 / 0.36 / 0.53 million cells 3.7 / 4.1 / 4.6 us acoustic, 4.1 / 4.9 /
+// 5.6 us VTI, against 4.6 / 9.3 us and 5.3 us as tiles; Cerjan of 1.06 million
+// cells 3.0 us acoustic, 4.2 us VTI against 4.4 and 7.0).  Cerjan batches up to
+// kPersistCells are one cooperative launch either way.
+constexpr double kSharedStepUs[3] = {1.8, 2.1, 2.4}, kSharedCellUs[3] = {1.15e-6, 2.0e-6, 2.8e-6};
+constexpr double kCpmlSharedStepUs[2] = {3.3, 3.6}, kCpmlSharedCellUs[2] = {2.3e-6, 3.3e-6};
+
 constexpr double kCpmlGraphStepUs = 9.6, kCpmlGraphCellUs[2] = {1.9e-6, 3.5e-6};
 // ... and of the one-barrier-per-step persistent loop (0.3 to 0.9 million cells:
 // 3.6 to 4.9 us acoustic, 4.6 to 5.9 us VTI, 5.4 to 8.5 us TTI)
@@ -184,9 +194,12 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
         const double cells_all = nshots * (double)nza * nxa;
         double best_cost = forward ? kGraphStepUs[approx] + kGraphCellUs[approx] * cells_all
                                    : kBackStepUs + kBackCellUs * cells_all;
-        if (job == kTileForward && !cpml && cells_all <= kPersistCells)
+        if ((job == kTileForward || job == kTileForwardAsync) && !cpml && cells_all <= kPersistCells)
             best_cost = std::min(best_cost, kPersistStepUs[approx] + kPersistCellUs[approx] * cells_all);
         if (cpml) best_cost = kCpmlGraphStepUs + kCpmlGraphCellUs[approx] * cells_all + (forward ? 0.0 : kBackStepUs);
+        if (job == kTileForwardAsync && (cpml || cells_all > kPersistCells))
+            best_cost = cpml ? kCpmlSharedStepUs[approx] + kCpmlSharedCellUs[approx] * cells_all
+                             : kSharedStepUs[approx] + kSharedCellUs[approx] * cells_all;
         if (job == kTileForwardLaunched) best_cost += cpml ? kCpmlLaunchUs : kLaunchUs;
         const int halo = cpml ? 8 : 4;
         for (int group = nshots; fits && coop && group >= 1; group = group > 1 ? (group + 1) / 2 : 0) {
