@@ -261,8 +261,9 @@ struct IntTag { static constexpr int value = V; };
 
 // One time step of this thread's warp (its shot, tile and segment): the
 // body of step_kernel, also run once per step by step_persistent_kernel.
-// EU: rows a trip in the border, S: ring slots.
-template <int APPROX, int BC, int EU = edge_unroll<APPROX>(), int S = ring_slots<APPROX>()>
+// EU, IU: rows a trip in the border and inside, S: ring slots.
+template <int APPROX, int BC, int EU = edge_unroll<APPROX>(), int S = ring_slots<APPROX>(),
+          int IU = interior_unroll<APPROX>()>
 __device__ __forceinline__ void step_body(const StepArgs& a)
 {
     constexpr int NA = ring_arrays<APPROX>();
@@ -570,7 +571,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     // tiles have columns outside [4, nx - 4)).
     const bool edge = xborder || z0 < a.N || z1 > a.nz - a.N;
     if (edge) march(IntTag<1>{}, IntTag<EU>{});
-    else march(IntTag<0>{}, IntTag<interior_unroll<APPROX>()>{});
+    else march(IntTag<0>{}, IntTag<IU>{});
     cp_async_wait<0>();
 }
 
@@ -1007,8 +1008,8 @@ struct PersistArgs {
     int nt, itlag, k0, k1;
 };
 
-// (Segments of a row or two: one border row a trip and the four-slot ring, three
-// TTI blocks a SM; with the ring and the four blocks of step_kernel four TTI
+// (Segments of one to eight rows, a power of two: one border row and two or four
+// interior rows a trip, the four-slot ring and three TTI blocks a SM; with the ring and the four blocks of step_kernel four TTI
 // shots of 364 x 464 took 7.7 us a step instead of 6.9.)
 template <int APPROX, int BC>
 __global__ void __launch_bounds__(128, APPROX == kTTI ? 3 : 4) step_persistent_kernel(const PersistArgs p)
@@ -1028,7 +1029,7 @@ __global__ void __launch_bounds__(128, APPROX == kTTI ? 3 : 4) step_persistent_k
             r.it = k - p.itlag;
             record_sample(r, gtid);
         }
-        step_body<APPROX, BC, 1, 4>(a);   // (segments of a row or two)
+        step_body<APPROX, BC, 1, 4, APPROX == kAcoustic ? 2 : 4>(a);
         grid.sync();
     }
 }
