@@ -741,7 +741,7 @@ def rtm_vti_leg(args, local):
     adj_gbs = 16.0 * cells * wl.shots / (adj_launch * 1e-3) / 1e9 if adj_n else None
     return {"leg": "rtm_vti", "workload": wl.name, "nz": wl.nz, "nx": wl.nx, "nt": wl.nt, "shots": wl.shots,
             "ckpt_interval": args.rtm_ckpt, "ms_per_shot": el / wl.shots * 1e3, "hbm_gb_in_use": (total - free) / 1e9,
-            "adjoint_kernel": {"name": "aniso_adjoint_tile_kernel<VTI>", "ms_per_launch": adj_launch,
+            "adjoint_kernel": {"name": "aniso_adjoint_kernel<VTI>", "ms_per_launch": adj_launch,
                                "sampled_launches": adj_n, "alg_bytes_per_cell_shot": 16,
                                "achieved_GBs": adj_gbs, "frac": adj_gbs / peak if adj_gbs else None},
             "imaging_ms_per_launch": img_ms / max(img_n, 1),
