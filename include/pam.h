@@ -71,7 +71,8 @@ int pam_set_models(pam_engine* e, const float* vp, const float* eps, const float
                    const float* theta_deg);
 
 /* Override the source wavelet ([nt] samples, already scaled). Replaces
- * Modeling::createWavelet (cpp/Modeling.cu:84-100). */
+ * Modeling::createWavelet (cpp/Modeling.cu:84-100).  Waits for the work in
+ * flight on the device before replacing the samples. */
 int pam_set_wavelet(pam_engine* e, const float* wavelet);
 
 /* Override the Cerjan damping factors ([n_abc] floats, index 0 at the outer

@@ -958,6 +958,10 @@ int pam_segment_height(const pam_engine* e, int nshots) {
 int pam_set_wavelet(pam_engine* e, const float* w) {
     PAM_GUARD(e);
     if (!w) return e->fail(PAM_E_ARG, "wavelet is NULL");
+    CU(cudaSetDevice(e->device));
+    // the persistent loops read the samples from the device at every step, and
+    // the engine's streams are non-blocking: wait for work that may read them
+    CU(cudaDeviceSynchronize());
     e->wavelet.assign(w, w + e->cfg.nt);
     CU(cudaMemcpy(e->d_wavelet, w, (size_t)e->cfg.nt * sizeof(float), cudaMemcpyHostToDevice));
     e->invalidate_graph();
