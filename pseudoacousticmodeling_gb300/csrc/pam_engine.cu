@@ -589,6 +589,7 @@ int pam_engine::check_numeric() {
 int pam_engine::reset_fields(int nshots, cudaStream_t s) {
     pam_engine* e = this;
     const size_t fb = (size_t)shot_stride * nshots * sizeof(float);
+    tile_held_shots = 0;
     CU(cudaMemsetAsync(d_status, 0, sizeof(int), s));
     CU(cudaMemsetAsync(d_u[0], 0, fb, s));
     CU(cudaMemsetAsync(d_u[1], 0, fb, s));
@@ -716,6 +717,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
             CU(cudaMemcpy2DAsync(h_seis + off, pitch, d_seis + off, pitch, (size_t)(j1 - j0) * nrec * sizeof(float),
                                  nshots, cudaMemcpyDeviceToHost, copy_stream));
         }
+        if (tiles) tile_held_shots = nshots;
         if (h_seis) {
             CU(cudaEventRecord(chunk_events[nchunks], copy_stream));
             CU(cudaStreamWaitEvent(s, chunk_events[nchunks], 0));
@@ -1069,8 +1071,12 @@ int pam_read_seismograms(pam_engine* e, float* out) {
 int pam_read_wavefield(pam_engine* e, int shot, float* out) {
     PAM_GUARD(e);
     if (shot < 0 || shot >= std::max(e->step_shots, 1) || !out) return e->fail(PAM_E_ARG, "bad shot index %d", shot);
-    // U(next_step) lives in buffer next_step & 1
-    const float* src = e->d_u[e->next_step & 1] + (long long)shot * e->shot_stride;
+    // U(next_step) lives in buffer next_step & 1; after a run as tiles, which
+    // publish their state in either set, U(nt) stands for buffer nt & 1 and
+    // U(nt - 1) for the other
+    const float* field = e->d_u[e->next_step & 1];
+    if (shot < e->tile_held_shots) field = e->tile_state((e->next_step ^ e->cfg.nt) & 1);
+    const float* src = field + (long long)shot * e->shot_stride;
     CU(cudaMemcpy2DAsync(out, e->nxa * sizeof(float), src, e->P * sizeof(float), e->nxa * sizeof(float), e->nza,
                          cudaMemcpyDeviceToHost, e->stream));
     CU(cudaStreamSynchronize(e->stream));

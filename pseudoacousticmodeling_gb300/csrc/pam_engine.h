@@ -205,6 +205,7 @@ struct pam_engine {
     bool tile_lists_stale = true;
     int tile_lists_TZ = 0, tile_lists_TX = 0;
     int tile_set = 0;                    // which published state is the current one
+    int tile_held_shots = 0;             // shots whose last fields lie there (a forward run as tiles)
     // The same for the fused adjoint + gradient kernel of the exact gradient
     // (fewer resident warps per SM than the stepping kernel, so its own
     // height); the stepping kernel's until tuned.
