@@ -102,6 +102,14 @@ int pam_forward(pam_engine* e, int nshots, const int* sz, const int* sx, float* 
 int pam_forward_device(pam_engine* e, int nshots, const int* d_sz, const int* d_sx, float* d_seis,
                        void* stream);
 
+/* The blocks of a cooperative launch wait for one another by polling, at most `polls`
+ * times a barrier (2^21 by default, about a second; they are all resident, so
+ * the limit is not met unless it is set far below a step).  A block that gives
+ * up leaves NaN in the samples it has not recorded, and the call (for
+ * pam_forward_device, the engine's next modelling, migration or gradient call)
+ * returns PAM_E_CUDA. */
+int pam_set_barrier_polls(pam_engine* e, int polls);
+
 /* Step-level interface, mirroring Modeling::forward_step(k)
  * (cpp/Modeling.cu:421-431) inside the reference's own loop:
  *   pam_begin(e, n, sz, sx)     reset fields, inject step 0

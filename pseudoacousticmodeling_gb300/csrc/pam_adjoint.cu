@@ -456,6 +456,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                                        "that of the absorbing scheme: use checkpoints");
     if (sb && (cfg.nz < 9 || cfg.nx < 9)) return fail(PAM_E_ARG, "boundary saving needs nz, nx >= 9");
     if (!sb && !rbc && (K <= 0 || K > cfg.nt)) K = cfg.nt;
+    if (int rc = check_gave_up()) return rc;
     CU(cudaSetDevice(device));
     if (int rc = ensure_adjoint(K, store)) return rc;
     const int nseg = adj_nseg;
@@ -700,6 +701,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         std::vector<double> part(blocks);
         CU(cudaMemcpyAsync(part.data(), d_partial, blocks * sizeof(double), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
+        if (int rc = check_gave_up()) return rc;
         for (double v : part) mis += v;
         if (!std::isfinite(mis))
             return fail(PAM_E_NUMERIC, "non-finite misfit: the modelled data overflowed (an unstable dt or grid for "
@@ -1008,20 +1010,11 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         if (mode == kRTM && btiles) tile_fold_image(nshots, d_img, d_img_ilum, st);
         CU(cudaGetLastError());
     }
-    if (mode == kExact) {
-        const size_t n = (size_t)cfg.nz * cfg.nx;
-        std::vector<float> g(n);
-        CU(cudaMemcpyAsync(g.data(), d_grad_b, n * 4, cudaMemcpyDeviceToHost, st));
-        CU(cudaStreamSynchronize(st));
-        for (size_t i = 0; i < n; i++) grad_vp[i] += g[i];
-    }
+    std::vector<float> g_vp(mode == kExact ? interior : 0);
+    if (mode == kExact) CU(cudaMemcpyAsync(g_vp.data(), d_grad_b, interior * 4, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
-    if (ftiles || btiles || rtiles) {
-        // a barrier of the tiles that was given up (a non-finite sample shows in the misfit)
-        int v = 0;
-        CU(cudaMemcpy(&v, d_status, sizeof(int), cudaMemcpyDeviceToHost));
-        if (v & 2) return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
-    }
+    if (int rc = check_gave_up()) return rc;   // (a non-finite sample shows in the misfit)
+    for (size_t i = 0; i < g_vp.size(); i++) grad_vp[i] += g_vp[i];
     if (misfit) *misfit += mis;
     return PAM_OK;
 }

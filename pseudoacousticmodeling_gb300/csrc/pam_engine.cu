@@ -186,6 +186,10 @@ int pam_engine::init(const pam_config& c, int dev) {
     if (dalloc(this, &d_sz, (size_t)B) || dalloc(this, &d_sx, (size_t)B) || dalloc(this, &d_status, (size_t)1))
         return PAM_E_CUDA;
     CU(cudaMemset(d_status, 0, sizeof(int)));
+    CU(cudaHostAlloc((void**)&h_gave_up, sizeof(int), cudaHostAllocMapped));
+    host_allocs.push_back(h_gave_up);
+    *h_gave_up = 0;
+    CU(cudaHostGetDevicePointer((void**)&d_gave_up, h_gave_up, 0));
 
     // Ricker wavelet, float arithmetic of Modeling::createWavelet (cpp/Modeling.cu:84-100)
     wavelet.assign(c.nt, 0.0f);
@@ -579,7 +583,7 @@ int pam_engine::check_numeric() {
     pam_engine* e = this;
     int v = 0;
     CU(cudaMemcpy(&v, d_status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (v & 2) return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
+    if (int rc = check_gave_up()) return rc;
     if (v & 1)
         return fail(PAM_E_NUMERIC, "non-finite values in the seismograms: the scheme is unstable for this model, dt and "
                                    "grid spacing (see pam_check_stability)");
@@ -666,6 +670,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     pam_engine* e = this;
     if (!models_set) return fail(PAM_E_STATE, "pam_set_models has not been called");
     if (nrec < 1) return fail(PAM_E_STATE, "pam_set_receivers has not been called");
+    if (int rc = check_gave_up()) return rc;
     CU(cudaSetDevice(device));
     const bool use_graph = std::getenv("PAM_NO_GRAPH") == nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -948,6 +953,13 @@ int pam_set_random_boundary(pam_engine* e, float dvel, float ratio, unsigned lon
 int pam_autotune(pam_engine* e, int enable) {
     PAM_GUARD(e);
     e->autotune = enable != 0;
+    return PAM_OK;
+}
+
+int pam_set_barrier_polls(pam_engine* e, int polls) {
+    PAM_GUARD(e);
+    if (polls < 1) return e->fail(PAM_E_ARG, "polls=%d is not positive", polls);
+    e->tile_polls = polls;
     return PAM_OK;
 }
 

@@ -199,6 +199,11 @@ struct pam_engine {
     int tile_bset = 0;
     float* d_tile[2] = {nullptr, nullptr};   // [B][stride] the second published state of the tiles
     unsigned* d_tile_bar = nullptr;
+    // set by a block that gives a barrier up (a word of mapped host memory, so
+    // that calls see it without waiting for the device); cleared when reported
+    int *h_gave_up = nullptr, *d_gave_up = nullptr;
+    int tile_polls = 1 << 21;            // of a barrier before that (half a microsecond each)
+    int check_gave_up();
     int* d_tile_beg = nullptr;           // receivers by tile (tile_begin)
     int2* d_tile_ent = nullptr;
     std::vector<int> h_rz, h_rx;

@@ -246,6 +246,14 @@ const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
     return it->second.usable ? &it->second : nullptr;
 }
 
+// PAM_E_CUDA (once) after a run whose blocks left a barrier without the others:
+// the run that has just completed, or an earlier one with device output.
+int pam_engine::check_gave_up() {
+    if (!h_gave_up || !*(volatile int*)h_gave_up) return PAM_OK;
+    *(volatile int*)h_gave_up = 0;
+    return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
+}
+
 int pam_engine::tile_buffers(cudaStream_t s) {
     pam_engine* e = this;
     const size_t field = (size_t)shot_stride * B;
@@ -314,6 +322,8 @@ TileArgs pam_engine::tile_args(const TilePlan& p, int nshots) const {
     t.nt = cfg.nt;
     t.itlag = cfg.itlag;
     t.bar = d_tile_bar;
+    t.polls = tile_polls;
+    t.gave_up = d_gave_up;
     t.status = d_status;
     t.mem_shots = B;
     t.slot_stride = shot_stride * B;

@@ -36,9 +36,6 @@ namespace pam {
 constexpr int kTileThreads = 512;       // at most
 constexpr int kTilePitch = 32;          // quads per row of a shared copy (more than a tile with its halo has)
 constexpr int kTileMaxT = 8;
-// polls of a grid barrier before it is given up (a poll takes about half a
-// microsecond): all blocks are resident, so this is never reached
-constexpr int kTileSpin = 1 << 21;
 
 // model arrays of an approximation: kappa, 1 + 2 eps, -2 (eps - delta),
 // 2 (1 + delta), cos, sin
@@ -75,7 +72,9 @@ struct TileArgs {
     const int2* __restrict__ rec_ent;    // ... as (row << 16 | column, receiver)
     int nt, itlag, k0, k1;
     unsigned* bar;                       // barrier counter, zero at the launch
-    int* status;                         // bit 1 set when a barrier was given up
+    int polls;                           // of a barrier before it is given up
+    int* gave_up;                        // host memory: set to 1 when one was
+    int* status;                         // bit 0 set by a non-finite sample
     // every U(k) kept: U(k) at slots + (k - kslot) * slot_stride; the state before
     // step k0 is U(k0), U(k0 - 1) there, and so is what the tiles exchange
     // (nullptr: the two published sets)
@@ -94,21 +93,31 @@ struct TileArgs {
 
 // Grid-wide barrier of resident blocks: each block's writes before it are
 // visible (through L2) to every block after it.  `want` = blocks x barriers so
-// far.  False when it was given up.
-__device__ __forceinline__ bool tile_barrier(unsigned* bar, unsigned want, int* status, int* flag) {
+// far.  False when it was given up (all blocks are resident, so it is not
+// unless the limit is far below a step): the block then leaves, and so do the
+// others at their next barrier.
+__device__ __forceinline__ bool tile_barrier(const TileArgs& t, unsigned want, int* flag) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-        int left = kTileSpin;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
+        int left = t.polls;
         unsigned v;
         do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.bar) : "memory");
         } while ((int)(v - want) < 0 && --left > 0);
         *flag = left > 0;
-        if (left == 0) atomicOr(status, 2);
+        if (left <= 0) *(volatile int*)t.gave_up = 1;
     }
     __syncthreads();
     return *flag != 0;
+}
+
+// The samples that a block which gave up at step k leaves out: NaN, so that the
+// holder of a device buffer sees it.
+__device__ __forceinline__ void tile_poison(const TileArgs& t, float* seis, int rb, int re, int k) {
+    for (int i = rb + threadIdx.x; i < re; i += blockDim.x)
+        for (int it = max(k - t.itlag, 0); it < t.k1 - t.itlag; it++)
+            seis[(long long)it * t.rec.nrec + t.rec_ent[i].y] = __int_as_float(0x7fc00000);
 }
 
 // A quad of row z, column x (a multiple of 4) of a pitched array; zero outside
@@ -488,7 +497,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_forward_kernel(const Til
         set ^= 1;
         if (left <= 0) break;
         want += gridDim.x;
-        if (!tile_barrier(t.bar, want, t.status, &alive)) return;
+        if (!tile_barrier(t, want, &alive)) {
+            if (!REVERSE) tile_poison(t, seis, rb, re, k);
+            return;
+        }
         // the halo, both fields, from the other tiles
         const unsigned halo = own.valid & ~own.mine;
         if (halo) {
@@ -742,7 +754,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_adjoint_kernel(const Til
         if (k < t.k0) break;
         cp_async_wait<0>();                        // the next group's data (and U)
         want += gridDim.x;
-        if (!tile_barrier(t.bar, want, t.status, &alive)) return;
+        if (!tile_barrier(t, want, &alive)) return;
         const unsigned halo = own.valid & ~own.mine;
         if (halo) {
 #pragma unroll
@@ -1234,7 +1246,10 @@ __global__ void __launch_bounds__(tile_cpml_threads(R), 1) tile_cpml_kernel(cons
         if (left <= 0) break;
         if (ROLE == kTileRtmRole) cp_async_wait<0>();
         want += gridDim.x;
-        if (!tile_barrier(t.bar, want, t.status, &alive)) return;
+        if (!tile_barrier(t, want, &alive)) {
+            if (ROLE == kTileForwardRole) tile_poison(t, seis, rb, re, k);
+            return;
+        }
         const unsigned halo = own.valid & ~own.mine;
         if (halo) {
             float4 px[R], pz[R];

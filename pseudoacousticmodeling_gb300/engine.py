@@ -212,6 +212,10 @@ class Engine:
         """Segment height chosen for a batch of `nshots` (0: not tuned yet)."""
         return int(self.lib.pam_segment_height(self.h, int(nshots)))
 
+    def set_barrier_polls(self, polls):
+        """Most polls of a grid barrier of the persistent tiles before it is given up."""
+        self._check(self.lib.pam_set_barrier_polls(self.h, int(polls)))
+
     def profile_read(self):
         """{class: (total ms, sampled launches)} of the last completed run:
         the forward steps' stepping, CPML-strip and recording kernels, and the
