@@ -464,7 +464,8 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     // rtiles: the source field backwards in time (boundary saving, random border).
     // Forward sweeps that checkpoint CPML memory variables stay with the one-step
     // launches; their backward sweeps do not, so that a sum over time has one order.
-    const TilePlan *ftiles = nullptr, *btiles = nullptr, *rtiles = nullptr;
+    TilePlan *ftiles = nullptr, *rtiles = nullptr;
+    const TilePlan* btiles = nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &capturing));
     chain_launches = capturing == cudaStreamCaptureStatusNone;
@@ -473,7 +474,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         if (sb || rbc) rtiles = tile_plan(nshots, kTileReverse);
         if (sb && !rtiles) ftiles = nullptr;
         if (ftiles)
-            if (int rc = tile_begin(*ftiles, st)) return rc;
+            if (int rc = tile_begin(*ftiles, nshots, st)) return rc;
         if (mode != kFWIRef && (rtiles || !(sb || rbc)))
             if (int rc = tile_adjoint_begin(nshots, mode == kExact ? kTileExactJob : kTileRtmJob, st, &btiles)) return rc;
         if (rtiles) {

@@ -97,6 +97,10 @@ pam_engine::~pam_engine() {
     for (cudaEvent_t ev : strip_events)
         if (ev) cudaEventDestroy(ev);
     if (strip_stream) cudaStreamDestroy(strip_stream);
+    for (auto& plans : tile_plans)
+        for (auto& p : plans)
+            for (TileLists* l : {&p.second.record, &p.second.inject})
+                if (l->uploaded) cudaEventDestroy(l->uploaded);
     for (cudaEvent_t ev : obs_events)
         if (ev) cudaEventDestroy(ev);
     if (copy_stream) cudaStreamDestroy(copy_stream);
@@ -323,7 +327,8 @@ int pam_engine::set_receivers(int n, const int* rz, const int* rx, int per_shot)
     CU(cudaMemcpy(d_rx, rx, cnt * sizeof(int), cudaMemcpyHostToDevice));
     h_rz.assign(rz, rz + cnt);
     h_rx.assign(rx, rx + cnt);
-    tile_lists_stale = tile_inject_stale = true;
+    for (auto& plans : tile_plans)
+        for (auto& p : plans) p.second.record.ready = p.second.inject.ready = false;
     nrec = n;
     rec_per_shot = per_shot ? 1 : 0;
     invalidate_graph();
@@ -678,7 +683,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     chain_launches = capturing == cudaStreamCaptureStatusNone;
     // (a run into the caller's device buffer returns at once: others may share the GPU)
     const TileJob job = d_seis == d_seis_own ? kTileForward : kTileForwardAsync;
-    const TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots, job) : nullptr;
+    TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots, job) : nullptr;
     const int persist_h = use_graph && capturing == cudaStreamCaptureStatusNone && !tiles ? persistent_height(nshots) : 0;
     if (!tiles && !persist_h)   // the persistent paths set their own shapes
         if (int rc = tune_segments(nshots, s)) return rc;
@@ -708,7 +713,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
         }
         const size_t pitch = (size_t)nt_data * nrec * sizeof(float);
         if (tiles)
-            if (int rc = tile_begin(*tiles, s)) return rc;
+            if (int rc = tile_begin(*tiles, nshots, s)) return rc;
         for (int c = 0; c < nchunks; c++) {
             const int rc = tiles ? tile_forward(*tiles, nshots, d_seis, bounds[c], bounds[c + 1], s)
                                  : launch_persistent(nshots, persist_h, d_seis, bounds[c], bounds[c + 1], s);

@@ -160,17 +160,31 @@ struct pam_engine {
     // nullptr for the one-step launches; tile_begin makes the buffers and lists
     // of a plan ready, tile_forward runs steps k0 .. k1-1 from the state that
     // the run's earlier launches left (before the first: d_u[0], d_u[1])
+    // the receivers by tile (or by thread of a tile) of a plan: `count` offsets and
+    // the entries they point into, in one buffer, uploaded in the order of the
+    // run's stream from a pinned copy; made again after set_receivers
+    struct TileLists {
+        bool ready = false, ok = true;   // ok: the plan can take these receivers
+        size_t bytes = 0;                // of both buffers
+        char *d = nullptr, *h = nullptr;
+        size_t entries = 0;              // where these start in d
+        cudaEvent_t uploaded = nullptr;
+        const int* beg() const { return (const int*)d; }
+        const int2* ent() const { return (const int2*)(d + entries); }
+    };
     struct TilePlan {
         bool usable = false;
         int T = 0, TZ = 0, TX = 0, nty = 0, ntx = 0, R = 0, halo = 4;
         int group = 0;                   // shots per launch
+        TileLists record, inject;
     };
     enum TileJob { kTileForward = 0, kTileExactJob = 1, kTileRtmJob = 2, kTileReverse = 3, kTileForwardLaunched = 4,
                    kTileForwardAsync = 5 };
     std::map<int, TilePlan> tile_plans[6];
-    const TilePlan* tile_plan(int nshots, TileJob job = kTileForward);
+    TilePlan* tile_plan(int nshots, TileJob job = kTileForward);
     int tile_buffers(cudaStream_t s);
-    int tile_begin(const TilePlan& p, cudaStream_t s);
+    int tile_begin(TilePlan& p, int nshots, cudaStream_t s);
+    int tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s);
     int tile_undamped(const TilePlan& p, int nshots, const float* kap, cudaStream_t s);
     pam::TileArgs tile_args(const TilePlan& p, int nshots) const;
     // with slots every U(k) goes to slots + (k - kslot) fields and the state
@@ -192,10 +206,6 @@ struct pam_engine {
     void tile_fold_image(int nshots, float* img, float* ilum, cudaStream_t s) const;
     float* d_tile_b[2] = {nullptr, nullptr};     // [B][stride] second published receiver-side state
     float* d_tile_sum[2] = {nullptr, nullptr};   // [B][stride] sums over time: gradient or image, illumination
-    int* d_inj_beg = nullptr;
-    int2* d_inj_ent = nullptr;
-    bool tile_inject_stale = true, tile_inject_ok = false;
-    int tile_inject_shape[4] = {0, 0, 0, 0};
     int tile_bset = 0;
     float* d_tile[2] = {nullptr, nullptr};   // [B][stride] the second published state of the tiles
     unsigned* d_tile_bar = nullptr;
@@ -204,11 +214,7 @@ struct pam_engine {
     int *h_gave_up = nullptr, *d_gave_up = nullptr;
     int tile_polls = 1 << 21;            // of a barrier before that (half a microsecond each)
     int check_gave_up();
-    int* d_tile_beg = nullptr;           // receivers by tile (tile_begin)
-    int2* d_tile_ent = nullptr;
     std::vector<int> h_rz, h_rx;
-    bool tile_lists_stale = true;
-    int tile_lists_TZ = 0, tile_lists_TX = 0;
     int tile_set = 0;                    // which published state is the current one
     int tile_held_shots = 0;             // shots whose last fields lie there (a forward run as tiles)
     // The same for the fused adjoint + gradient kernel of the exact gradient

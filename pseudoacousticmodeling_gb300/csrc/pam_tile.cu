@@ -173,7 +173,7 @@ __global__ void tile_fold_image_kernel(const float* __restrict__ gsum, const flo
 // and the cells of each step's region at the rate one SM updates them; a batch
 // may go in several launches of some shots each.  The tiles are taken where
 // the best of these is below the cost of the one-step launches.
-const pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
+pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
     const int approx = cfg.approximation;
     const bool cpml = cfg.boundary == PAM_CPML && job != kTileReverse;
     if (prof_stride > 0 || std::getenv("PAM_NO_PERSISTENT")) return nullptr;
@@ -266,10 +266,39 @@ int pam_engine::tile_buffers(cudaStream_t s) {
     return PAM_OK;
 }
 
+// The lists of a plan to the device, behind the work queued on s.  Buffers that
+// are large enough are used again: nothing here waits for the device, except to
+// make them larger.
+int pam_engine::tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s) {
+    pam_engine* e = this;
+    l.entries = (beg.size() * sizeof(int) + 15) / 16 * 16;
+    const size_t need = l.entries + ent.size() * sizeof(int2);
+    if (!l.uploaded) CU(cudaEventCreateWithFlags(&l.uploaded, cudaEventDisableTiming));
+    CU(cudaEventSynchronize(l.uploaded));   // the last upload has left the pinned copy
+    if (need > l.bytes) {
+        l.bytes = 0;
+        dfree(l.d);
+        l.d = nullptr;
+        if (l.h) host_allocs.erase(std::find(host_allocs.begin(), host_allocs.end(), (void*)l.h));
+        cudaFreeHost(l.h);
+        l.h = nullptr;
+        if (dalloc_bytes((void**)&l.d, need)) return PAM_E_CUDA;
+        CU(cudaMallocHost((void**)&l.h, need));
+        host_allocs.push_back(l.h);
+        l.bytes = need;
+    }
+    std::copy(beg.begin(), beg.end(), (int*)l.h);
+    std::copy(ent.begin(), ent.end(), (int2*)(l.h + l.entries));
+    CU(cudaMemcpyAsync(l.d, l.h, need, cudaMemcpyHostToDevice, s));
+    CU(cudaEventRecord(l.uploaded, s));
+    l.ready = true;
+    return PAM_OK;
+}
+
 // The buffers of the persistent tiles, and each tile's list of the receivers
 // in it (receivers off the update region, whose samples are zero, go to the
 // nearest tile, which holds those cells in its halo).
-int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
+int pam_engine::tile_begin(TilePlan& p, int nshots, cudaStream_t s) {
     pam_engine* e = this;
     const size_t field = (size_t)shot_stride * B;
     if (int rc = tile_buffers(s)) return rc;
@@ -279,8 +308,8 @@ int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
             if (!d && dalloc_bytes((void**)&d, 4 * field * 4)) return PAM_E_CUDA;
         CU(cudaMemsetAsync(d_tile_mem[0], 0, 4 * field * 4, s));
     }
-    if (!tile_lists_stale && tile_lists_TZ == p.TZ && tile_lists_TX == p.TX) return PAM_OK;
-    const int nt = p.nty * p.ntx, lists = rec_per_shot ? B : 1;
+    if (p.record.ready) return PAM_OK;
+    const int nt = p.nty * p.ntx, lists = rec_per_shot ? nshots : 1;
     std::vector<int> beg((size_t)nt * lists + 1, 0);
     std::vector<int> where((size_t)lists * nrec);
     for (int l = 0; l < lists; l++)
@@ -295,20 +324,7 @@ int pam_engine::tile_begin(const TilePlan& p, cudaStream_t s) {
     std::vector<int> at(beg.begin(), beg.end() - 1);
     std::vector<int2> ent(where.size());
     for (size_t i = 0; i < where.size(); i++) ent[at[where[i]]++] = make_int2(h_rz[i] << 16 | h_rx[i], (int)(i % nrec));
-    dfree(d_tile_beg);
-    dfree(d_tile_ent);
-    d_tile_beg = nullptr;
-    d_tile_ent = nullptr;
-    if (dalloc_bytes((void**)&d_tile_beg, beg.size() * sizeof(int)) ||
-        dalloc_bytes((void**)&d_tile_ent, ent.size() * sizeof(int2)))
-        return PAM_E_CUDA;
-    CU(cudaMemcpyAsync(d_tile_beg, beg.data(), beg.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(d_tile_ent, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
-    CU(cudaStreamSynchronize(s));   // the vectors go out of scope
-    tile_lists_stale = false;
-    tile_lists_TZ = p.TZ;
-    tile_lists_TX = p.TX;
-    return PAM_OK;
+    return tile_upload(p.record, beg, ent, s);
 }
 
 TileArgs pam_engine::tile_args(const TilePlan& p, int nshots) const {
@@ -340,8 +356,8 @@ int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k
     t.ex[1][1] = d_tile[1];
     t.set0 = tile_set;
     t.rec.seis = d_seis;
-    t.rec_beg = d_tile_beg;
-    t.rec_ent = d_tile_ent;
+    t.rec_beg = p.record.beg();
+    t.rec_ent = p.record.ent();
     t.k0 = k0;
     t.k1 = k1;
     t.slots = slots;
@@ -448,58 +464,42 @@ int pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, cons
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &cs));
     if (cfg.approximation != PAM_ACOUSTIC || cs != cudaStreamCaptureStatusNone) return PAM_OK;
-    const TilePlan* p = tile_plan(nshots, job);
+    TilePlan* p = tile_plan(nshots, job);
     if (!p) return PAM_OK;
-    const TileShape g = shape_of(*p);
-    const bool same = !tile_inject_stale && tile_inject_shape[0] == p->T && tile_inject_shape[1] == p->TZ &&
-                      tile_inject_shape[2] == p->TX && tile_inject_shape[3] == p->R;
-    if (!same) {
-        const int nt = p->nty * p->ntx, lists = rec_per_shot ? B : 1, nthr = tile_threads(g);
+    TileLists& l = p->inject;
+    if (!l.ready) {
+        const TileShape g = shape_of(*p);
+        const int nt = p->nty * p->ntx, lists = rec_per_shot ? nshots : 1, nthr = tile_threads(g);
         std::vector<int> beg((size_t)nt * lists * (nthr + 1));
         std::vector<int2> ent;
         std::vector<std::vector<int2>> of(nthr);
-        tile_inject_ok = true;
-        for (size_t i = 0; i < h_rz.size() && tile_inject_ok; i++)
-            tile_inject_ok = h_rz[i] >= 4 && h_rz[i] < nza - 4 && h_rx[i] >= 4 && h_rx[i] < nxa - 4;
-        for (int l = 0; l < lists * nt && tile_inject_ok; l++) {
-            const int tile = l % nt;
+        l.ok = true;
+        for (size_t i = 0; i < (size_t)lists * nrec && l.ok; i++)
+            l.ok = h_rz[i] >= 4 && h_rz[i] < nza - 4 && h_rx[i] >= 4 && h_rx[i] < nxa - 4;
+        for (int t = 0; t < lists * nt && l.ok; t++) {
+            const int tile = t % nt;
             const int ez0 = 4 + (tile / p->ntx) * p->TZ - p->halo * p->T, ex0 = 4 + (tile % p->ntx) * p->TX - p->halo * p->T;
             for (auto& v : of) v.clear();
             for (int r = 0; r < nrec; r++) {
-                const size_t i = (size_t)(l / nt) * nrec + r;
+                const size_t i = (size_t)(t / nt) * nrec + r;
                 const int er = h_rz[i] - ez0, ec = h_rx[i] - ex0;
                 if (er < 0 || er >= g.nrg * g.R || ec < 0 || ec >= 4 * g.EXq) continue;
                 of[(er / g.R) * g.EXq + ec / 4].push_back(make_int2(h_rz[i] << 16 | h_rx[i], r));
             }
             const size_t first = ent.size();
-            int* const b = &beg[(size_t)l * (nthr + 1)];
+            int* const b = &beg[(size_t)t * (nthr + 1)];
             for (int j = 0; j < nthr; j++) {
                 b[j] = (int)ent.size();
                 ent.insert(ent.end(), of[j].begin(), of[j].end());
             }
             b[nthr] = (int)ent.size();
-            if (ent.size() - first > (size_t)kTileInject) tile_inject_ok = false;
+            if (ent.size() - first > (size_t)kTileInject) l.ok = false;
         }
-        if (tile_inject_ok) {
-            dfree(d_inj_beg);
-            dfree(d_inj_ent);
-            d_inj_beg = nullptr;
-            d_inj_ent = nullptr;
-            ent.resize(std::max<size_t>(ent.size(), 1));
-            if (dalloc_bytes((void**)&d_inj_beg, beg.size() * sizeof(int)) ||
-                dalloc_bytes((void**)&d_inj_ent, ent.size() * sizeof(int2)))
-                return PAM_E_CUDA;
-            CU(cudaMemcpyAsync(d_inj_beg, beg.data(), beg.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-            CU(cudaMemcpyAsync(d_inj_ent, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
-            CU(cudaStreamSynchronize(s));   // the vectors go out of scope
-        }
-        tile_inject_stale = false;
-        tile_inject_shape[0] = p->T;
-        tile_inject_shape[1] = p->TZ;
-        tile_inject_shape[2] = p->TX;
-        tile_inject_shape[3] = p->R;
+        if (l.ok)
+            if (int rc = tile_upload(l, beg, ent, s)) return rc;
+        l.ready = true;
     }
-    if (!tile_inject_ok) return PAM_OK;
+    if (!l.ok) return PAM_OK;
     const size_t field = (size_t)shot_stride * B;
     for (float*& d : d_tile_b)
         if (!d) {
@@ -534,8 +534,8 @@ int pam_engine::tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0,
     t.f.k1 = k1;
     t.f.slots = const_cast<float*>(slots);
     t.f.kslot = kslot;
-    t.inj_beg = d_inj_beg;
-    t.inj_ent = d_inj_ent;
+    t.inj_beg = p.inject.beg();
+    t.inj_ent = p.inject.ent();
     t.data = data;
     t.scale = scale;
     t.gsum = d_tile_sum[0];

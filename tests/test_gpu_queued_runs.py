@@ -60,3 +60,54 @@ def test_a_queued_run_keeps_its_wavelet(approx, boundary):
     torch.cuda.synchronize()
     for a, b in zip(alone, queued):
         assert np.array_equal(a, b.cpu().numpy())
+
+
+@pytest.mark.parametrize("per_shot", [False, True])
+def test_batches_of_different_sizes_do_not_wait(per_shot):
+    """A survey's full batches and its smaller last one, in turn and with new
+    receivers in between, are queued while the stream is busy, and give what an
+    engine gives that sees one batch and one set of receivers only."""
+    shots, sizes = 7, (7, 2, 7, 3, 2)
+    st = torch.cuda.Stream()
+
+    def receivers(e, seed):
+        rng = np.random.default_rng(seed)
+        shape = (shots, 25) if per_shot else (25,)
+        e.set_receivers(rng.integers(0, e.cfg.nz_abc, shape).astype(np.int32),
+                        rng.integers(0, e.cfg.nx_abc, shape).astype(np.int32), per_shot=per_shot)
+
+    def queue(e, n):
+        sz, sx = sources(e, n)
+        out = empty_data(e, n)
+        torch.cuda.synchronize()
+        return sz, sx, out
+
+    ref = {}
+    for seed in (1, 2):
+        for n in set(sizes):
+            e, _ = make_engine("acoustic", "cerjan", shots)
+            receivers(e, seed)
+            sz, sx, out = queue(e, n)
+            e.forward_device(sz, sx, out, stream=st.cuda_stream)
+            torch.cuda.synchronize()
+            ref[seed, n] = out.cpu().numpy()
+    assert all(np.abs(v).max() > 0 for v in ref.values())
+    e, _ = make_engine("acoustic", "cerjan", shots)
+    receivers(e, 3)
+    for n in sizes:                      # each batch size's buffers
+        sz, sx, out = queue(e, n)
+        e.forward_device(sz, sx, out, stream=st.cuda_stream)
+    runs = [(seed, n, *queue(e, n)) for seed in (1, 2) for n in sizes]
+    busy = torch.cuda.Event()
+    for i, (seed, n, sz, sx, out) in enumerate(runs):
+        if i % len(sizes) == 0:
+            torch.cuda.synchronize()     # (set_receivers replaces arrays that queued graphs read)
+            receivers(e, seed)
+            with torch.cuda.stream(st):
+                torch.cuda._sleep(WAIT)
+            busy.record(st)
+        e.forward_device(sz, sx, out, stream=st.cuda_stream)
+        assert not busy.query(), (i, n)
+    torch.cuda.synchronize()
+    for seed, n, _, _, out in runs:
+        assert np.array_equal(out.cpu().numpy(), ref[seed, n])
