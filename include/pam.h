@@ -110,6 +110,17 @@ int pam_forward_device(pam_engine* e, int nshots, const int* d_sz, const int* d_
  * returns PAM_E_CUDA. */
 int pam_set_barrier_polls(pam_engine* e, int polls);
 
+/* Small batches run as tiles keep a workspace on the device, sized for the
+ * largest such batch: 2 fields per shot of it (8 more with the matched layer);
+ * migration and gradients 4 more (8 more with the matched layer); boundary
+ * saving and the random border up to 50 more, freed when the strategy or the
+ * interval changes.  None of it is needed: where it does not fit, the run takes
+ * the one-step launches, and the engine's other allocations free it before
+ * they fail.  limit_bytes >= 0 bounds it from here on (0: no tiles); in_use
+ * (may be NULL) receives the bytes now held.  pam_plan_checkpoints does not
+ * count it. */
+int pam_tile_workspace(pam_engine* e, long long limit_bytes, long long* in_use);
+
 /* Step-level interface, mirroring Modeling::forward_step(k)
  * (cpp/Modeling.cu:421-431) inside the reference's own loop:
  *   pam_begin(e, n, sz, sx)     reset fields, inject step 0
@@ -135,7 +146,8 @@ int pam_read_wavefield(pam_engine* e, int shot, float* out);
  * reference's "RBC", src/Migration.py:327-458, 837-959).  The source field
  * runs undamped through a border of random velocities (pam_set_random_boundary)
  * and is rebuilt by running the same undamped scheme backwards in time:
- * nothing is stored.  The receiver field keeps the absorbing border.  For
+ * nothing is stored (small batches keep up to 50 steps at a time in their
+ * workspace, see pam_tile_workspace).  The receiver field keeps the absorbing border.  For
  * pam_rtm and pam_fwi_gradient (whose modelled data then come from an extra
  * forward run with the absorbing border). */
 #define PAM_RANDOM_BOUNDARY (-2)

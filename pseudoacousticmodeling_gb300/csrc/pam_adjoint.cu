@@ -113,6 +113,7 @@ int pam_engine::ensure_adjoint(int K, int store) {
         d_ckpt_cpml = nullptr;
         d_band = nullptr;
         d_band_scale = nullptr;
+        tile_free(&d_tile_slots, tile_slot_count());
         if (K == PAM_RANDOM_BOUNDARY) {
             if (!d_u3 && dalloc_bytes((void**)&d_u3, field * B * 4)) return PAM_E_CUDA;
             if (!d_kap_rbc && dalloc_bytes((void**)&d_kap_rbc, field * 4)) return PAM_E_CUDA;
@@ -241,8 +242,8 @@ int restore_checkpoint(pam_engine* e, int s, int nshots, cudaStream_t st, float*
 }
 
 // Boundary saving: save / write back the band of a source-field buffer; the save
-// takes `times` consecutive fields from the first slot on.
-int save_band(pam_engine* e, const float* field, int slot, int nshots, cudaStream_t st, int times = 1) {
+// takes `times` consecutive fields, fs floats apart, from the first slot on.
+int save_band(pam_engine* e, const float* field, int slot, int nshots, cudaStream_t st, int times = 1, long long fs = 0) {
     const GridDims g = dims(e);
     const long long nb = band_cells(e->cfg.nz, e->cfg.nx);
     const int nchunk = (int)((nb + kBandChunk - 1) / kBandChunk);
@@ -251,7 +252,6 @@ int save_band(pam_engine* e, const float* field, int slot, int nshots, cudaStrea
     float* sc = e->d_band_scale + (size_t)slot * e->B * nchunk;
     if (times < 1) return PAM_OK;
     const dim3 grid(nchunk, nshots, times);
-    const long long fs = e->shot_stride * e->B;
     if (e->adj_store == PAM_STORE_F32)
         band_save_kernel<float><<<grid, kBandChunk, 0, st>>>(field, (float*)dst, sc, g, e->cfg.nz, e->cfg.nx, 0.0f, fs,
                                                              e->B);
@@ -460,10 +460,22 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     CU(cudaSetDevice(device));
     if (int rc = ensure_adjoint(K, store)) return rc;
     const int nseg = adj_nseg;
+    const size_t nseis = (size_t)nshots * nt_data * nrec;
+    if (!d_seis_own || seis_own_nrec < nrec) {
+        if (dalloc_bytes((void**)&d_seis_own, (size_t)B * nt_data * nrec * 4)) return PAM_E_CUDA;
+        seis_own_shots = B;
+        seis_own_nrec = nrec;
+    }
+    if (!d_obs || partial_cap < (nseis + 255) / 256) {
+        if (dalloc_bytes((void**)&d_obs, (size_t)B * nt_data * nrec * 4)) return PAM_E_CUDA;
+        partial_cap = ((size_t)B * nt_data * nrec + 255) / 256;
+        if (dalloc_bytes((void**)&d_partial, partial_cap * sizeof(double))) return PAM_E_CUDA;
+    }
     // small runs: the forward and backward sweeps as persistent tiles (pam_tile.cuh);
     // rtiles: the source field backwards in time (boundary saving, random border).
     // Forward sweeps that checkpoint CPML memory variables stay with the one-step
     // launches; their backward sweeps do not, so that a sum over time has one order.
+    // (After every allocation that the job needs: the tiles' workspace is optional.)
     TilePlan *ftiles = nullptr, *rtiles = nullptr;
     const TilePlan* btiles = nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -472,19 +484,13 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     if (capturing == cudaStreamCaptureStatusNone) {
         if (cfg.boundary != PAM_CPML || nseg <= 1) ftiles = tile_plan(nshots, kTileForwardLaunched);
         if (sb || rbc) rtiles = tile_plan(nshots, kTileReverse);
+        tile_reserve(nshots);
+        if (rtiles && !tile_slots(st)) rtiles = nullptr;
         if (sb && !rtiles) ftiles = nullptr;
-        if (ftiles)
-            if (int rc = tile_begin(*ftiles, nshots, st)) return rc;
+        if (ftiles && !tile_begin(*ftiles, nshots, st)) ftiles = nullptr;
         if (mode != kFWIRef && (rtiles || !(sb || rbc)))
-            if (int rc = tile_adjoint_begin(nshots, mode == kExact ? kTileExactJob : kTileRtmJob, st, &btiles)) return rc;
-        if (rtiles) {
-            if (int rc = tile_buffers(st)) return rc;
-            if (!d_tile_slots) {
-                const size_t n = (size_t)shot_stride * B * (kTileSegment + 2);
-                if (dalloc_bytes((void**)&d_tile_slots, n * 4)) return PAM_E_CUDA;
-                CU(cudaMemsetAsync(d_tile_slots, 0, n * 4, st));   // the outer rows and columns stay zero
-            }
-        }
+            btiles = tile_adjoint_begin(nshots, mode == kExact ? kTileExactJob : kTileRtmJob, st);
+        CU(cudaGetLastError());
     }
     if (!(rbc ? rtiles && (ftiles || mode == kRTM) : ftiles != nullptr) ||
         (!btiles && cfg.approximation == PAM_ACOUSTIC))
@@ -514,17 +520,6 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             }
         CU(cudaMemcpyAsync(d_kap_rbc, kr.data(), kr.size() * 4, cudaMemcpyHostToDevice, st));
         CU(cudaStreamSynchronize(st));
-    }
-    const size_t nseis = (size_t)nshots * nt_data * nrec;
-    if (!d_seis_own || seis_own_nrec < nrec) {
-        if (dalloc_bytes((void**)&d_seis_own, (size_t)B * nt_data * nrec * 4)) return PAM_E_CUDA;
-        seis_own_shots = B;
-        seis_own_nrec = nrec;
-    }
-    if (!d_obs || partial_cap < (nseis + 255) / 256) {
-        if (dalloc_bytes((void**)&d_obs, (size_t)B * nt_data * nrec * 4)) return PAM_E_CUDA;
-        partial_cap = ((size_t)B * nt_data * nrec + 255) / 256;
-        if (dalloc_bytes((void**)&d_partial, partial_cap * sizeof(double))) return PAM_E_CUDA;
     }
     CU(cudaMemcpyAsync(d_sz, sz, nshots * sizeof(int), cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync(d_sx, sx, nshots * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -619,14 +614,15 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         // boundary saving as tiles: segments of fields in the slots (slot j holds
         // U(k0 - 1 + j)), then their bands in one launch
         if (int rc = reset_fields(nshots, st)) return rc;
-        const size_t fb = (size_t)field * B;
+        const long long fb = tile_field();
         CU(cudaMemcpyAsync(d_tile_slots, d_u[1], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
         CU(cudaMemcpyAsync(d_tile_slots + fb, d_u[0], (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
         for (int k0 = 0; k0 < nt; k0 += kTileSegment) {
             const int k1 = std::min(k0 + kTileSegment, nt), n = k1 - k0;
-            if (int rc = tile_forward(*ftiles, nshots, need_data ? d_seis_own : nullptr, k0, k1, st, d_tile_slots + fb, k0))
+            if (int rc = tile_forward(*ftiles, nshots, need_data ? d_seis_own : nullptr, k0, k1, st, d_tile_slots + fb, k0,
+                                      fb))
                 return rc;
-            if (int rc = save_band(this, d_tile_slots + fb, k0, nshots, st, std::min(n, nt - 1 - k0))) return rc;
+            if (int rc = save_band(this, d_tile_slots + fb, k0, nshots, st, std::min(n, nt - 1 - k0), fb)) return rc;
             // the state before step k1 to the front, or, at the end, to the field buffers
             for (int i = 0; i < 2; i++) {
                 float* const to = k1 < nt ? d_tile_slots + i * fb : i == 0 ? d_u[(nt - 1) & 1] : d_u[nt & 1];
@@ -669,7 +665,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         CU(cudaMemcpyAsync(lslot(tl - 1), prev, (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
         CU(cudaMemcpyAsync(lslot(tl), cur, (size_t)field * nshots * 4, cudaMemcpyDeviceToDevice, st));
         if (ftiles) {
-            if (int rc = tile_forward(*ftiles, nshots, seis, tl, nt, st, lslot(tl), tl)) return rc;
+            if (int rc = tile_forward(*ftiles, nshots, seis, tl, nt, st, lslot(tl), tl, field * B)) return rc;
         } else {
             for (int k = tl; k < nt; k++) enqueue_forward_step(k, nshots, seis, st, lslot(k), lslot(k - 1), lslot(k + 1));
         }
@@ -880,7 +876,8 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         // backwards in time into the slots (slot j holds S(t0 - 1 + j)), then the
         // receiver side of the segment
         if (int rc = wait_obs()) return rc;
-        const size_t fb = (size_t)field * B, bytes = (size_t)field * nshots * 4;
+        const long long fb = tile_field();
+        const size_t bytes = (size_t)field * nshots * 4;
         if (btiles) {
             const long long n = (long long)nrec * nshots;
             launch_chained(chain_launches, inject_receivers_kernel, (int)((n + 255) / 256), 256, 0, st, d_ub[0], d_obs,
@@ -896,7 +893,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                 return rc;
             auto slot = [&](int t) { return d_tile_slots + (size_t)(t - t0 + 1) * fb; };
             if (btiles) {
-                if (int rc = tile_adjoint(*btiles, kTileRtmJob, nshots, t0, t1, slot(t0), t0, d_obs, inv_dxdz, st)) return rc;
+                if (int rc = tile_adjoint(*btiles, kTileRtmJob, nshots, t0, t1, slot(t0), t0, fb, d_obs, inv_dxdz, st)) return rc;
             } else {
                 for (int t = t1 - 1; t >= t0; t--) receiver_step(t, t ? slot(t - 1) : slot(0), slot(t), slot(t + 1));
             }
@@ -959,7 +956,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             }
             float* const seis = need_data && nseg == 1 ? d_seis_own : nullptr;
             if (ftiles) {
-                if (int rc = tile_forward(*ftiles, nshots, seis, t0, t1, st, slot(t0), t0)) return rc;
+                if (int rc = tile_forward(*ftiles, nshots, seis, t0, t1, st, slot(t0), t0, field * B)) return rc;
             } else {
                 for (int k = t0; k < t1; k++)
                     enqueue_forward_step(k, nshots, seis, st, slot(k), slot(k - 1), slot(k + 1));
@@ -979,7 +976,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                                gnod);
             }
             if (int rc = tile_adjoint(*btiles, mode == kExact ? kTileExactJob : kTileRtmJob, nshots, t0, t1, slot(t0), t0,
-                                      d_obs, inv_dxdz, st))
+                                      field * B, d_obs, inv_dxdz, st))
                 return rc;
         } else {
             for (int t = t1 - 1; t >= t0; t--) receiver_step(t, slot(t - 1), slot(t), slot(t + 1));

@@ -46,12 +46,7 @@ template <typename T>
 int dalloc(pam_engine* e, T** p, size_t n) {
     *p = nullptr;
     if (n == 0) return PAM_OK;
-    cudaError_t s = cudaMalloc((void**)p, n * sizeof(T));
-    if (s != cudaSuccess)
-        return e->fail(PAM_E_CUDA, "cudaMalloc of %zu bytes failed: %s", n * sizeof(T), cudaGetErrorString(s));
-    e->allocs.push_back((void*)*p);
-    e->bytes_allocated += n * sizeof(T);
-    return PAM_OK;
+    return e->dalloc_bytes((void**)p, n * sizeof(T));
 }
 
 // Edge-replicating padding of Modeling::expandModel (cpp/Modeling.cu:130-182)
@@ -85,6 +80,10 @@ int pam_engine::dalloc_bytes(void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) return PAM_OK;
     cudaError_t s = cudaMalloc(p, bytes);
+    if (s != cudaSuccess && tile_release()) {
+        cudaGetLastError();
+        s = cudaMalloc(p, bytes);
+    }
     if (s != cudaSuccess) return fail(PAM_E_CUDA, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(s));
     allocs.push_back(*p);
     bytes_allocated += bytes;
@@ -684,6 +683,10 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     // (a run into the caller's device buffer returns at once: others may share the GPU)
     const TileJob job = d_seis == d_seis_own ? kTileForward : kTileForwardAsync;
     TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots, job) : nullptr;
+    if (tiles) {
+        tile_reserve(nshots);
+        if (!tile_begin(*tiles, nshots, s)) tiles = nullptr;
+    }
     const int persist_h = use_graph && capturing == cudaStreamCaptureStatusNone && !tiles ? persistent_height(nshots) : 0;
     if (!tiles && !persist_h)   // the persistent paths set their own shapes
         if (int rc = tune_segments(nshots, s)) return rc;
@@ -712,8 +715,6 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
             chunk_events.push_back(ev);
         }
         const size_t pitch = (size_t)nt_data * nrec * sizeof(float);
-        if (tiles)
-            if (int rc = tile_begin(*tiles, nshots, s)) return rc;
         for (int c = 0; c < nchunks; c++) {
             const int rc = tiles ? tile_forward(*tiles, nshots, d_seis, bounds[c], bounds[c + 1], s)
                                  : launch_persistent(nshots, persist_h, d_seis, bounds[c], bounds[c + 1], s);
@@ -965,6 +966,17 @@ int pam_set_barrier_polls(pam_engine* e, int polls) {
     PAM_GUARD(e);
     if (polls < 1) return e->fail(PAM_E_ARG, "polls=%d is not positive", polls);
     e->tile_polls = polls;
+    return PAM_OK;
+}
+
+int pam_tile_workspace(pam_engine* e, long long limit_bytes, long long* in_use) {
+    PAM_GUARD(e);
+    if (limit_bytes >= 0) {
+        e->tile_limit = (size_t)limit_bytes;
+        CU(cudaSetDevice(e->device));
+        if (e->tile_bytes > e->tile_limit) e->tile_release();
+    }
+    if (in_use) *in_use = (long long)e->tile_bytes;
     return PAM_OK;
 }
 

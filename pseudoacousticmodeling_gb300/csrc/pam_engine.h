@@ -119,7 +119,7 @@ struct pam_engine {
     double* d_partial = nullptr;
     size_t partial_cap = 0;
     bool adj_base_ready = false;
-    int dalloc_bytes(void** p, size_t bytes);
+    int dalloc_bytes(void** p, size_t bytes);   // frees the tiles' workspace where it is in the way
     void dfree(void* p);   // free one tracked allocation (implicitly waits for the device)
     int ensure_adjoint(int K, int store);
     int run_adjoint_job(int mode, int nshots, const int* sz, const int* sx, const float* dobs, int K, int store,
@@ -182,32 +182,46 @@ struct pam_engine {
                    kTileForwardAsync = 5 };
     std::map<int, TilePlan> tile_plans[6];
     TilePlan* tile_plan(int nshots, TileJob job = kTileForward);
-    int tile_buffers(cudaStream_t s);
-    int tile_begin(TilePlan& p, int nshots, cudaStream_t s);
-    int tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s);
+    // The tiles' workspace, for the largest batch that took them so far.  All of it
+    // is optional: what does not fit (in tile_limit bytes, or on the device) sends
+    // the run to the one-step launches, and the engine's other allocations free it
+    // before they fail.
+    int tile_shots = 0;                  // shots of every array below
+    size_t tile_bytes = 0, tile_limit = ~(size_t)0;
+    bool tile_tight = false;             // something did not fit
+    void tile_reserve(int nshots);       // sets tile_shots, before anything of a run is allocated
+    bool tile_alloc(float** d, size_t fields, bool zero, cudaStream_t s);
+    void tile_free(float** d, size_t fields);
+    bool tile_release();                 // false: there was nothing to free
+    bool tile_buffers(cudaStream_t s);
+    bool tile_slots(cudaStream_t s);
+    int tile_slot_count() const { return (cfg.nt < kTileSegment ? cfg.nt : kTileSegment) + 2; }
+    long long tile_field() const { return shot_stride * tile_shots; }   // floats of one array of fields
+    bool tile_begin(TilePlan& p, int nshots, cudaStream_t s);
+    bool tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s);
     int tile_undamped(const TilePlan& p, int nshots, const float* kap, cudaStream_t s);
     pam::TileArgs tile_args(const TilePlan& p, int nshots) const;
-    // with slots every U(k) goes to slots + (k - kslot) fields and the state
+    // with slots every U(k) goes to slots + (k - kslot) slot_stride and the state
     // before step k0 is U(k0), U(k0 - 1) there
     int tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s, float* slots = nullptr,
-                     int kslot = 0);
+                     int kslot = 0, long long slot_stride = 0);
     int tile_reverse(const TilePlan& p, int nshots, int k0, int k1, cudaStream_t s, float* slots, int kslot,
                      const float* kap, bool bands);
-    float* d_tile_mem[2] = {nullptr, nullptr};    // [4][B][stride] CPML memory variables as published
+    float* d_tile_mem[2] = {nullptr, nullptr};    // [4][tile_shots][stride] CPML memory variables as published
     float* d_tile_bmem[2] = {nullptr, nullptr};   // ... of the receiver-side field
-    float* d_tile_slots = nullptr;                // [kTileSegment + 2][B][stride] source fields of a segment
+    float* d_tile_slots = nullptr;                // [tile_slot_count()][tile_shots][stride] source fields of a segment
     static constexpr int kTileSegment = 48;       // (boundary saving and the random border)
     const float* tile_state(int i) const { return tile_set ? d_tile[i] : d_u[i]; }   // 0: U(k), 1: U(k-1)
     // backward sweeps of the acoustic jobs: steps t = k1-1 .. k0 of a segment
     // with its source fields in slots, the sums of each shot's cells in d_tile_sum
-    int tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, const TilePlan** out);
+    const TilePlan* tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s);
     int tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0, int k1, const float* slots, int kslot,
-                     const float* data, float scale, cudaStream_t s);
+                     long long slot_stride, const float* data, float scale, cudaStream_t s);
     void tile_fold_image(int nshots, float* img, float* ilum, cudaStream_t s) const;
-    float* d_tile_b[2] = {nullptr, nullptr};     // [B][stride] second published receiver-side state
-    float* d_tile_sum[2] = {nullptr, nullptr};   // [B][stride] sums over time: gradient or image, illumination
+    float* d_tile_b[2] = {nullptr, nullptr};     // [tile_shots][stride] second published receiver-side state
+    float* d_tile_sum[2] = {nullptr, nullptr};   // [tile_shots][stride] sums over time: gradient or image, illumination
     int tile_bset = 0;
-    float* d_tile[2] = {nullptr, nullptr};   // [B][stride] the second published state of the tiles
+    float* d_tile[2] = {nullptr, nullptr};   // [tile_shots][stride] the second published state of the tiles
     unsigned* d_tile_bar = nullptr;
     // set by a block that gives a barrier up (a word of mapped host memory, so
     // that calls see it without waiting for the device); cleared when reported

@@ -254,27 +254,77 @@ int pam_engine::check_gave_up() {
     return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
 }
 
-int pam_engine::tile_buffers(cudaStream_t s) {
-    pam_engine* e = this;
-    const size_t field = (size_t)shot_stride * B;
-    for (float*& d : d_tile)
-        if (!d) {
-            if (dalloc_bytes((void**)&d, field * 4)) return PAM_E_CUDA;
-            CU(cudaMemsetAsync(d, 0, field * 4, s));
+// One array of the workspace: `fields` fields of every shot of it.
+bool pam_engine::tile_alloc(float** d, size_t fields, bool zero, cudaStream_t s) {
+    if (*d) return true;
+    const size_t bytes = fields * (size_t)tile_field() * 4;
+    tile_tight = true;
+    if (bytes > tile_limit || tile_bytes > tile_limit - bytes) return false;
+    if (cudaMalloc((void**)d, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        *d = nullptr;
+        return false;
+    }
+    tile_tight = false;
+    allocs.push_back(*d);
+    tile_bytes += bytes;
+    if (zero) cudaMemsetAsync(*d, 0, bytes, s);   // (its error is the caller's next one)
+    return true;
+}
+
+void pam_engine::tile_free(float** d, size_t fields) {
+    if (!*d) return;
+    dfree(*d);
+    *d = nullptr;
+    tile_bytes -= fields * (size_t)tile_field() * 4;
+}
+
+bool pam_engine::tile_release() {
+    if (!tile_bytes) return false;
+    for (float** d : {d_tile, d_tile_b, d_tile_sum})
+        for (int i = 0; i < 2; i++) tile_free(d + i, 1);
+    for (float** d : {d_tile_mem, d_tile_bmem})
+        for (int i = 0; i < 2; i++) tile_free(d + i, 4);
+    tile_free(&d_tile_slots, tile_slot_count());
+    tile_held_shots = 0;
+    return true;
+}
+
+// The workspace grows with the batch; where the larger one has not fitted, it is
+// made anew for the smaller.
+void pam_engine::tile_reserve(int nshots) {
+    if (nshots <= tile_shots && !(nshots < tile_shots && tile_tight)) return;
+    tile_release();
+    tile_shots = nshots;
+    tile_tight = false;
+}
+
+// The second published state.
+bool pam_engine::tile_buffers(cudaStream_t s) {
+    if (!d_tile_bar) {
+        if (cudaMalloc((void**)&d_tile_bar, 128) != cudaSuccess) {
+            cudaGetLastError();
+            d_tile_bar = nullptr;
+            return false;
         }
-    if (!d_tile_bar && dalloc_bytes((void**)&d_tile_bar, 128)) return PAM_E_CUDA;
-    return PAM_OK;
+        allocs.push_back(d_tile_bar);
+    }
+    return tile_alloc(&d_tile[0], 1, true, s) && tile_alloc(&d_tile[1], 1, true, s);
+}
+
+// The source fields of a segment (their outer rows and columns stay zero).
+bool pam_engine::tile_slots(cudaStream_t s) {
+    return tile_buffers(s) && tile_alloc(&d_tile_slots, tile_slot_count(), true, s);
 }
 
 // The lists of a plan to the device, behind the work queued on s.  Buffers that
 // are large enough are used again: nothing here waits for the device, except to
 // make them larger.
-int pam_engine::tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s) {
-    pam_engine* e = this;
+bool pam_engine::tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s) {
     l.entries = (beg.size() * sizeof(int) + 15) / 16 * 16;
     const size_t need = l.entries + ent.size() * sizeof(int2);
-    if (!l.uploaded) CU(cudaEventCreateWithFlags(&l.uploaded, cudaEventDisableTiming));
-    CU(cudaEventSynchronize(l.uploaded));   // the last upload has left the pinned copy
+    if (!l.uploaded && cudaEventCreateWithFlags(&l.uploaded, cudaEventDisableTiming) != cudaSuccess) return false;
+    cudaEventSynchronize(l.uploaded);   // the last upload has left the pinned copy
     if (need > l.bytes) {
         l.bytes = 0;
         dfree(l.d);
@@ -282,33 +332,41 @@ int pam_engine::tile_upload(TileLists& l, const std::vector<int>& beg, const std
         if (l.h) host_allocs.erase(std::find(host_allocs.begin(), host_allocs.end(), (void*)l.h));
         cudaFreeHost(l.h);
         l.h = nullptr;
-        if (dalloc_bytes((void**)&l.d, need)) return PAM_E_CUDA;
-        CU(cudaMallocHost((void**)&l.h, need));
+        if (cudaMalloc((void**)&l.d, need) != cudaSuccess) {
+            l.d = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        allocs.push_back(l.d);
+        if (cudaMallocHost((void**)&l.h, need) != cudaSuccess) {
+            l.h = nullptr;
+            cudaGetLastError();
+            return false;
+        }
         host_allocs.push_back(l.h);
         l.bytes = need;
     }
     std::copy(beg.begin(), beg.end(), (int*)l.h);
     std::copy(ent.begin(), ent.end(), (int2*)(l.h + l.entries));
-    CU(cudaMemcpyAsync(l.d, l.h, need, cudaMemcpyHostToDevice, s));
-    CU(cudaEventRecord(l.uploaded, s));
-    l.ready = true;
-    return PAM_OK;
+    l.ready = cudaMemcpyAsync(l.d, l.h, need, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+              cudaEventRecord(l.uploaded, s) == cudaSuccess;
+    return l.ready;
 }
 
 // The buffers of the persistent tiles, and each tile's list of the receivers
 // in it (receivers off the update region, whose samples are zero, go to the
-// nearest tile, which holds those cells in its halo).
-int pam_engine::tile_begin(TilePlan& p, int nshots, cudaStream_t s) {
-    pam_engine* e = this;
-    const size_t field = (size_t)shot_stride * B;
-    if (int rc = tile_buffers(s)) return rc;
+// nearest tile, which holds those cells in its halo).  False: there is no room
+// for them.
+bool pam_engine::tile_begin(TilePlan& p, int nshots, cudaStream_t s) {
+    if (!tile_buffers(s)) return false;
     tile_set = 0;
     if (p.halo == 8) {
-        for (float*& d : d_tile_mem)
-            if (!d && dalloc_bytes((void**)&d, 4 * field * 4)) return PAM_E_CUDA;
-        CU(cudaMemsetAsync(d_tile_mem[0], 0, 4 * field * 4, s));
+        if (!tile_alloc(&d_tile_mem[0], 4, false, s) || !tile_alloc(&d_tile_mem[1], 4, false, s)) return false;
+        // (what is published into the other set covers all that is read from it)
+        for (int i = 0; i < 4; i++)
+            cudaMemsetAsync(d_tile_mem[0] + i * tile_field(), 0, (size_t)shot_stride * nshots * 4, s);
     }
-    if (p.record.ready) return PAM_OK;
+    if (p.record.ready) return true;
     const int nt = p.nty * p.ntx, lists = rec_per_shot ? nshots : 1;
     std::vector<int> beg((size_t)nt * lists + 1, 0);
     std::vector<int> where((size_t)lists * nrec);
@@ -341,13 +399,12 @@ TileArgs pam_engine::tile_args(const TilePlan& p, int nshots) const {
     t.polls = tile_polls;
     t.gave_up = d_gave_up;
     t.status = d_status;
-    t.mem_shots = B;
-    t.slot_stride = shot_stride * B;
+    t.mem_shots = tile_shots;
     return t;
 }
 
 int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k0, int k1, cudaStream_t s, float* slots,
-                             int kslot) {
+                             int kslot, long long slot_stride) {
     if (k1 <= k0) return PAM_OK;
     TileArgs t = tile_args(p, nshots);
     t.ex[0][0] = d_u[0];
@@ -362,6 +419,7 @@ int pam_engine::tile_forward(const TilePlan& p, int nshots, float* d_seis, int k
     t.k1 = k1;
     t.slots = slots;
     t.kslot = kslot;
+    t.slot_stride = slot_stride;
     const size_t smem = smem_of(t.g, cfg.approximation, kTileForward);
     for (int b = 0; b < nshots; b += p.group) {
         t.shot0 = b;
@@ -399,8 +457,10 @@ int pam_engine::tile_reverse(const TilePlan& p, int nshots, int k0, int k1, cuda
     t.k1 = k1;
     t.slots = slots;
     t.kslot = kslot;
+    t.slot_stride = tile_field();
     if (bands) {
         t.band = d_band;
+        t.band_shots = B;
         t.band_scale = d_band_scale;
         t.band_store = adj_store;
         t.nzi = cfg.nz;
@@ -454,18 +514,14 @@ int pam_engine::tile_undamped(const TilePlan& p, int nshots, const float* kap, c
 
 // ---------------------------------------------------------------- backward sweeps
 
-// The plan of a backward sweep, its buffers and each thread's receivers; nullptr
-// in *out for the one-step launches.  Receivers off the update region, which
-// the one-step kernels inject into cells that no step writes, and lists too
-// long for shared memory stay with those.
-int pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, const TilePlan** out) {
-    pam_engine* e = this;
-    *out = nullptr;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CU(cudaStreamIsCapturing(s, &cs));
-    if (cfg.approximation != PAM_ACOUSTIC || cs != cudaStreamCaptureStatusNone) return PAM_OK;
+// The plan of a backward sweep, with its buffers and each thread's receivers
+// ready; nullptr for the one-step launches.  Receivers off the update region,
+// which the one-step kernels inject into cells that no step writes, and lists
+// too long for shared memory stay with those.
+const pam_engine::TilePlan* pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s) {
+    if (cfg.approximation != PAM_ACOUSTIC) return nullptr;
     TilePlan* p = tile_plan(nshots, job);
-    if (!p) return PAM_OK;
+    if (!p) return nullptr;
     TileLists& l = p->inject;
     if (!l.ready) {
         const TileShape g = shape_of(*p);
@@ -495,33 +551,25 @@ int pam_engine::tile_adjoint_begin(int nshots, TileJob job, cudaStream_t s, cons
             b[nthr] = (int)ent.size();
             if (ent.size() - first > (size_t)kTileInject) l.ok = false;
         }
-        if (l.ok)
-            if (int rc = tile_upload(l, beg, ent, s)) return rc;
+        if (l.ok && !tile_upload(l, beg, ent, s)) return nullptr;
         l.ready = true;
     }
-    if (!l.ok) return PAM_OK;
-    const size_t field = (size_t)shot_stride * B;
-    for (float*& d : d_tile_b)
-        if (!d) {
-            if (dalloc_bytes((void**)&d, field * 4)) return PAM_E_CUDA;
-            CU(cudaMemsetAsync(d, 0, field * 4, s));
-        }
-    for (float*& d : d_tile_sum)
-        if (!d && dalloc_bytes((void**)&d, field * 4)) return PAM_E_CUDA;
-    if (!d_tile_bar && dalloc_bytes((void**)&d_tile_bar, 128)) return PAM_E_CUDA;
-    for (float* d : d_tile_sum) CU(cudaMemsetAsync(d, 0, (size_t)shot_stride * nshots * 4, s));
-    if (p->halo == 8) {
-        for (float*& d : d_tile_bmem)
-            if (!d && dalloc_bytes((void**)&d, 4 * field * 4)) return PAM_E_CUDA;
-        CU(cudaMemsetAsync(d_tile_bmem[0], 0, 4 * field * 4, s));
-    }
+    if (!l.ok) return nullptr;
+    if (!tile_buffers(s)) return nullptr;
+    for (int i = 0; i < 2; i++)
+        if (!tile_alloc(&d_tile_b[i], 1, true, s) || !tile_alloc(&d_tile_sum[i], 1, false, s) ||
+            (p->halo == 8 && !tile_alloc(&d_tile_bmem[i], 4, false, s)))
+            return nullptr;
+    const size_t bytes = (size_t)shot_stride * nshots * 4;
+    for (float* d : d_tile_sum) cudaMemsetAsync(d, 0, bytes, s);
+    if (p->halo == 8)
+        for (int i = 0; i < 4; i++) cudaMemsetAsync(d_tile_bmem[0] + i * tile_field(), 0, bytes, s);
     tile_bset = 0;
-    *out = p;
-    return PAM_OK;
+    return p;
 }
 
 int pam_engine::tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0, int k1, const float* slots, int kslot,
-                             const float* data, float scale, cudaStream_t s) {
+                             long long slot_stride, const float* data, float scale, cudaStream_t s) {
     if (k1 <= k0) return PAM_OK;
     TileAdjArgs t{};
     t.f = tile_args(p, nshots);
@@ -534,6 +582,7 @@ int pam_engine::tile_adjoint(const TilePlan& p, TileJob job, int nshots, int k0,
     t.f.k1 = k1;
     t.f.slots = const_cast<float*>(slots);
     t.f.kslot = kslot;
+    t.f.slot_stride = slot_stride;
     t.inj_beg = p.inject.beg();
     t.inj_ent = p.inject.ent();
     t.data = data;

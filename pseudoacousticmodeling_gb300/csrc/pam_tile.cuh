@@ -88,7 +88,7 @@ struct TileArgs {
     // saved band of time t-1 written over it (band == nullptr: none)
     const void* band;                    // [nt-1][B][nb] in the storage type
     const float* __restrict__ band_scale;   // [nt-1][B][chunks]
-    int band_store, nzi, nxi;
+    int band_shots, band_store, nzi, nxi;   // (the bands are kept for max_shots)
 };
 
 // Grid-wide barrier of resident blocks: each block's writes before it are
@@ -303,7 +303,7 @@ __device__ __forceinline__ int tile_band_index(int zi, int xi, int nzi, int nxi)
 __device__ __forceinline__ float tile_band_value(const TileArgs& t, int shot, int tt, int i) {
     const long long nb = band_cells(t.nzi, t.nxi);
     const long long nchunk = (nb + kBandChunk - 1) / kBandChunk;
-    const long long row = (long long)tt * t.mem_shots + shot;
+    const long long row = (long long)tt * t.band_shots + shot;
     if (t.band_store == 0) return reinterpret_cast<const float*>(t.band)[row * nb + i];
     const float v = t.band_store == 1 ? band_unpack(reinterpret_cast<const __nv_bfloat16*>(t.band)[row * nb + i])
                                       : band_unpack(reinterpret_cast<const __half*>(t.band)[row * nb + i]);

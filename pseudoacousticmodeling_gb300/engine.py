@@ -216,6 +216,13 @@ class Engine:
         """Most polls of a grid barrier of the persistent tiles before it is given up."""
         self._check(self.lib.pam_set_barrier_polls(self.h, int(polls)))
 
+    def tile_workspace(self, limit_bytes=-1):
+        """Bytes of the persistent tiles' workspace now held; limit_bytes >= 0
+        bounds it from here on (pam_tile_workspace)."""
+        n = ctypes.c_longlong()
+        self._check(self.lib.pam_tile_workspace(self.h, int(limit_bytes), ctypes.byref(n)))
+        return n.value
+
     def profile_read(self):
         """{class: (total ms, sampled launches)} of the last completed run:
         the forward steps' stepping, CPML-strip and recording kernels, and the
