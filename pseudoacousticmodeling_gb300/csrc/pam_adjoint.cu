@@ -492,9 +492,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
             btiles = tile_adjoint_begin(nshots, mode == kExact ? kTileExactJob : kTileRtmJob, st);
         CU(cudaGetLastError());
     }
-    if (!(rbc ? rtiles && (ftiles || mode == kRTM) : ftiles != nullptr) ||
-        (!btiles && cfg.approximation == PAM_ACOUSTIC))
-        if (int rc = tune_segments(nshots, st)) return rc;
+    if (int rc = tune_segments(nshots, st)) return rc;   // (with tiles too: see run_forward)
     if (mode == kExact && !btiles)
         if (int rc = tune_adjgrad(nshots, st)) return rc;
     if (rbc) {

@@ -687,8 +687,10 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
         tile_reserve(nshots);
         if (!tile_begin(*tiles, nshots, s)) tiles = nullptr;
     }
-    const int persist_h = use_graph && capturing == cudaStreamCaptureStatusNone && !tiles ? persistent_height(nshots) : 0;
-    if (!tiles && !persist_h)   // the persistent paths set their own shapes
+    // the one-barrier-per-step loop sets its own height; the tiles have none, but a
+    // later call of this batch size into a capture, which cannot tune, needs it
+    const int persist_h = use_graph && capturing == cudaStreamCaptureStatusNone ? persistent_height(nshots) : 0;
+    if (!persist_h)
         if (int rc = tune_segments(nshots, s)) return rc;
     if (int rc = reset_fields(nshots, s)) return rc;
     if (!use_graph) {
