@@ -121,6 +121,16 @@ int pam_set_barrier_polls(pam_engine* e, int polls);
  * count it. */
 int pam_tile_workspace(pam_engine* e, long long limit_bytes, long long* in_use);
 
+/* Which loop a batch of nshots takes (outside a stream capture, with room for
+ * the workspace): 0 one-step launches, 1 the cooperative launch with a barrier
+ * after every step, 2 tiles; <0 on error.  sweep: 0 pam_forward, 1 the backward
+ * sweep of the exact gradient, 2 that of acoustic migration, 3 the source field
+ * backwards in time (boundary saving, random border), 4 the forward sweep of a
+ * migration or gradient, 5 pam_forward_device.  plan[6] (may be NULL) receives for
+ * tiles: steps between barriers, rows and columns of a tile, rows per thread,
+ * halo cells per step, shots per launch. */
+int pam_time_loop(pam_engine* e, int nshots, int sweep, int* plan);
+
 /* Step-level interface, mirroring Modeling::forward_step(k)
  * (cpp/Modeling.cu:421-431) inside the reference's own loop:
  *   pam_begin(e, n, sz, sx)     reset fields, inject step 0

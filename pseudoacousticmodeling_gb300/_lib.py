@@ -61,6 +61,7 @@ SIGNATURES = {
                                  ctypes.c_float, ctypes.c_ulonglong, _p]),
     "pam_segment_height": (_i, [_p, _i]),
     "pam_set_barrier_polls": (_i, [_p, _i]),
+    "pam_time_loop": (_i, [_p, _i, _i, _pi]),
     "pam_tile_workspace": (_i, [_p, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]),
     "pam_profile_enable": (_i, [_p, _i]),
     "pam_profile_read": (_i, [_p, _pd, _pi, _i]),

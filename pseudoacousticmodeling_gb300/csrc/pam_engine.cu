@@ -982,6 +982,25 @@ int pam_tile_workspace(pam_engine* e, long long limit_bytes, long long* in_use) 
     return PAM_OK;
 }
 
+int pam_time_loop(pam_engine* e, int nshots, int sweep, int* plan) {
+    PAM_GUARD(e);
+    if (nshots < 1 || nshots > e->B) return e->fail(PAM_E_ARG, "nshots=%d outside [1, %d]", nshots, e->B);
+    if (sweep < pam_engine::kTileForward || sweep > pam_engine::kTileForwardAsync)
+        return e->fail(PAM_E_ARG, "unknown sweep %d", sweep);
+    CU(cudaSetDevice(e->device));
+    const auto job = (pam_engine::TileJob)sweep;
+    const bool modelling = job == pam_engine::kTileForward || job == pam_engine::kTileForwardAsync;
+    const bool backward = job == pam_engine::kTileExactJob || job == pam_engine::kTileRtmJob;
+    if (modelling && std::getenv("PAM_NO_GRAPH")) return 0;
+    if (backward && e->cfg.approximation != PAM_ACOUSTIC) return 0;
+    if (const auto* p = e->tile_plan(nshots, job)) {
+        const int v[6] = {p->T, p->TZ, p->TX, p->R, p->halo, p->group};
+        if (plan) std::copy(v, v + 6, plan);
+        return 2;
+    }
+    return modelling && e->persistent_height(nshots) ? 1 : 0;
+}
+
 int pam_segment_height(const pam_engine* e, int nshots) {
     if (!e) return PAM_E_ARG;
     const auto it = e->seg_height_by_shots.find(nshots);

@@ -15,6 +15,7 @@ MISFIT_NOALLOC_MAX_SAMPLES = 134217728   # PAM_MISFIT_NOALLOC_MAX_SAMPLES
 APPROX = {"acoustic": 0, "VTI": 1, "TTI": 2}
 BOUNDARY = {"cerjan": 0, "CPML": 1}
 STORE = {"f32": 0, "bf16": 1, "f16": 2}
+SWEEPS = ("forward", "exact", "rtm", "reverse", "job forward", "forward_device")   # of pam_time_loop
 BOUNDARY_SAVING = -1    # ckpt_interval value: rebuild the source field from saved boundary bands
 RANDOM_BOUNDARY = -2    # ckpt_interval value: undamped source field through a random border, run backwards
 NORM = {"none": 0, "cpp": 1, "py": 2}
@@ -222,6 +223,13 @@ class Engine:
         n = ctypes.c_longlong()
         self._check(self.lib.pam_tile_workspace(self.h, int(limit_bytes), ctypes.byref(n)))
         return n.value
+
+    def time_loop(self, nshots, sweep="forward"):
+        """(loop, plan) of a batch: "launches", "persistent" or "tiles", and for
+        tiles a dict of the cut (pam_time_loop)."""
+        v = (ctypes.c_int * 6)()
+        loop = self._check(self.lib.pam_time_loop(self.h, int(nshots), SWEEPS.index(sweep), v))
+        return ("launches", "persistent", "tiles")[loop], dict(zip(("T", "TZ", "TX", "R", "halo", "group"), v))
 
     def profile_read(self):
         """{class: (total ms, sampled launches)} of the last completed run:
