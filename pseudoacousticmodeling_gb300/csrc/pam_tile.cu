@@ -85,7 +85,7 @@ size_t smem_of(const TileShape& g, int approx, int job) {
     return forward ? tile_smem_bytes(g, models_of(approx)) : tile_adj_smem_bytes(g);
 }
 
-int threads_of(const TileShape& g) { return g.halo == 8 ? tile_cpml_threads(g.R) : kTileThreads; }
+int threads_of(const TileShape& g) { return g.halo == 8 ? kTileCpmlThreads : kTileThreads; }
 
 // A cooperative launch; the shared-memory opt-in is a per-device attribute of
 // the kernel.
@@ -124,15 +124,10 @@ cudaError_t launch_forward(int approx, const TileArgs& t, int blocks, size_t sme
                                   : launch_forward<kTTI, REVERSE>(t, blocks, smem, s);
 }
 
-template <int A, int R, int ROLE>
-cudaError_t launch_cpml(const TileCpmlArgs& t, int blocks, size_t smem, cudaStream_t s) {
-    static bool configured[kMaxDevices] = {};
-    return launch<TileCpmlArgs>(tile_cpml_kernel<A, R, ROLE>, configured, t, blocks, tile_threads(t.r.f.g), smem, s);
-}
-
 template <int A, int ROLE>
 cudaError_t launch_cpml(const TileCpmlArgs& t, int blocks, size_t smem, cudaStream_t s) {
-    return t.r.f.g.R == 1 ? launch_cpml<A, 1, ROLE>(t, blocks, smem, s) : launch_cpml<A, 2, ROLE>(t, blocks, smem, s);
+    static bool configured[kMaxDevices] = {};
+    return launch<TileCpmlArgs>(tile_cpml_kernel<A, ROLE>, configured, t, blocks, tile_threads(t.r.f.g), smem, s);
 }
 
 template <int MODE, int R>
@@ -209,7 +204,7 @@ pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
                 const int nty0 = std::min(sms / (ntx * group), rows);
                 if (nty0 < 1) break;
                 const int TZ = (rows + nty0 - 1) / nty0, nty = (rows + TZ - 1) / TZ;
-                for (int R = cpml ? 1 : 2; R <= (cpml ? 2 : 4); R++)
+                for (int R = cpml ? kTileCpmlRows : 2; R <= (cpml ? kTileCpmlRows : 4); R++)
                     for (int T = 1; T <= kTileMaxT; T++) {
                         TilePlan p;
                         p.usable = true;

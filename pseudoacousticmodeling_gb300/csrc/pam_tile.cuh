@@ -842,12 +842,15 @@ __device__ __forceinline__ void d1_quad(const float4& l, const float4& c, const 
     d[1] = d1_pair_ref(O3, O2, P4, P2, O4, O1, P5, P1, inv);
 }
 
-// threads of a block at most, by rows per thread: one row in 64 registers, two in 168
-__host__ __device__ constexpr int tile_cpml_threads(int R) { return R == 1 ? 1024 : 384; }
+// One row per thread, in 64 registers: a cut that fits with two rows in twice the
+// registers (384 threads at most) fits with one too, in no more shared memory and
+// with a cheaper exchange.
+constexpr int kTileCpmlRows = 1, kTileCpmlThreads = 1024;
 
-template <int APPROX, int R, int ROLE>
-__global__ void __launch_bounds__(tile_cpml_threads(R), 1) tile_cpml_kernel(const TileCpmlArgs tc)
+template <int APPROX, int ROLE>
+__global__ void __launch_bounds__(kTileCpmlThreads, 1) tile_cpml_kernel(const TileCpmlArgs tc)
 {
+    constexpr int R = kTileCpmlRows;
     extern __shared__ float4 tsm[];
     __shared__ int alive;
     const TileAdjArgs& ta = tc.r;
