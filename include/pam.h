@@ -106,8 +106,8 @@ int pam_forward_device(pam_engine* e, int nshots, const int* d_sz, const int* d_
  * times a barrier (2^21 by default, about a second; they are all resident, so
  * the limit is not met unless it is set far below a step).  A block that gives
  * up leaves NaN in the samples it has not recorded, and the call (for
- * pam_forward_device, the engine's next modelling, migration or gradient call)
- * returns PAM_E_CUDA. */
+ * pam_forward_device, the engine's next call that waits for its run) returns
+ * PAM_E_CUDA. */
 int pam_set_barrier_polls(pam_engine* e, int polls);
 
 /* Small batches run as tiles keep a workspace on the device, sized for the

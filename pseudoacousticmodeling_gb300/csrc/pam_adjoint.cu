@@ -456,7 +456,6 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
                                        "that of the absorbing scheme: use checkpoints");
     if (sb && (cfg.nz < 9 || cfg.nx < 9)) return fail(PAM_E_ARG, "boundary saving needs nz, nx >= 9");
     if (!sb && !rbc && (K <= 0 || K > cfg.nt)) K = cfg.nt;
-    if (int rc = check_gave_up()) return rc;
     CU(cudaSetDevice(device));
     if (int rc = ensure_adjoint(K, store)) return rc;
     const int nseg = adj_nseg;
@@ -696,8 +695,9 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         std::vector<double> part(blocks);
         CU(cudaMemcpyAsync(part.data(), d_partial, blocks * sizeof(double), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
-        if (int rc = check_gave_up()) return rc;
         for (double v : part) mis += v;
+        if (!std::isfinite(mis))
+            if (int rc = check_status(false)) return rc;   // samples left out
         if (!std::isfinite(mis))
             return fail(PAM_E_NUMERIC, "non-finite misfit: the modelled data overflowed (an unstable dt or grid for "
                                        "this model, see pam_check_stability) or the observed data hold NaN/Inf");
@@ -1009,7 +1009,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     std::vector<float> g_vp(mode == kExact ? interior : 0);
     if (mode == kExact) CU(cudaMemcpyAsync(g_vp.data(), d_grad_b, interior * 4, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
-    if (int rc = check_gave_up()) return rc;   // (a non-finite sample shows in the misfit)
+    if (int rc = check_status(false)) return rc;   // (a non-finite sample shows in the misfit)
     for (size_t i = 0; i < g_vp.size(); i++) grad_vp[i] += g_vp[i];
     if (misfit) *misfit += mis;
     return PAM_OK;

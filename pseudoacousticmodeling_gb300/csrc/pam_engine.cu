@@ -186,13 +186,9 @@ int pam_engine::init(const pam_config& c, int dev) {
             dalloc(this, &d_cxab, (size_t)xs_stride) || dalloc(this, &d_czab, (size_t)zs_stride))
             return PAM_E_CUDA;
     }
-    if (dalloc(this, &d_sz, (size_t)B) || dalloc(this, &d_sx, (size_t)B) || dalloc(this, &d_status, (size_t)1))
+    if (dalloc(this, &d_sz, (size_t)B) || dalloc(this, &d_sx, (size_t)B) || dalloc(this, &d_status, (size_t)2))
         return PAM_E_CUDA;
-    CU(cudaMemset(d_status, 0, sizeof(int)));
-    CU(cudaHostAlloc((void**)&h_gave_up, sizeof(int), cudaHostAllocMapped));
-    host_allocs.push_back(h_gave_up);
-    *h_gave_up = 0;
-    CU(cudaHostGetDevicePointer((void**)&d_gave_up, h_gave_up, 0));
+    CU(cudaMemset(d_status, 0, 2 * sizeof(int)));
 
     // Ricker wavelet, float arithmetic of Modeling::createWavelet (cpp/Modeling.cu:84-100)
     wavelet.assign(c.nt, 0.0f);
@@ -579,21 +575,24 @@ void pam_engine::launch_record(int nshots, const float* cur, float* seis, int it
     launch_chained(chain_launches, record_kernel, (int)((n + 255) / 256), 256, 0, s, r);
 }
 
-// Reset fields and memory variables and inject the step-0 source sample.
-// After a modelling run has completed: PAM_E_NUMERIC if the recording saw a
-// non-finite value (an unstable time step or grid for the model overflows the
-// fields within a few dozen steps).
-int pam_engine::check_numeric() {
+// The recording sees a non-finite value when an unstable time step or grid for
+// the model overflows the fields, within a few dozen steps.
+int pam_engine::check_status(bool numeric) {
     pam_engine* e = this;
-    int v = 0;
-    CU(cudaMemcpy(&v, d_status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (int rc = check_gave_up()) return rc;
-    if (v & 1)
+    int v[2] = {0, 0};
+    CU(cudaMemcpy(v, d_status, sizeof(v), cudaMemcpyDeviceToHost));
+    if (v[1]) {
+        // this run, or an earlier one with device output
+        CU(cudaMemset(d_status + 1, 0, sizeof(int)));
+        return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
+    }
+    if (numeric && (v[0] & 1))
         return fail(PAM_E_NUMERIC, "non-finite values in the seismograms: the scheme is unstable for this model, dt and "
                                    "grid spacing (see pam_check_stability)");
     return PAM_OK;
 }
 
+// Reset fields and memory variables and inject the step-0 source sample.
 int pam_engine::reset_fields(int nshots, cudaStream_t s) {
     pam_engine* e = this;
     const size_t fb = (size_t)shot_stride * nshots * sizeof(float);
@@ -674,7 +673,6 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     pam_engine* e = this;
     if (!models_set) return fail(PAM_E_STATE, "pam_set_models has not been called");
     if (nrec < 1) return fail(PAM_E_STATE, "pam_set_receivers has not been called");
-    if (int rc = check_gave_up()) return rc;
     CU(cudaSetDevice(device));
     const bool use_graph = std::getenv("PAM_NO_GRAPH") == nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -1075,7 +1073,7 @@ int pam_forward(pam_engine* e, int nshots, const int* sz, const int* sx, float* 
         CU(cudaMemcpyAsync(seis, e->d_seis_own, bytes, cudaMemcpyDeviceToHost, s));
     }
     CU(cudaStreamSynchronize(s));
-    return e->check_numeric();
+    return e->check_status(true);
 }
 
 int pam_begin(pam_engine* e, int nshots, const int* sz, const int* sx) {
@@ -1115,7 +1113,7 @@ int pam_read_seismograms(pam_engine* e, float* out) {
     CU(cudaMemcpyAsync(out, e->d_seis_own, (size_t)e->step_shots * e->nt_data * e->nrec * sizeof(float),
                        cudaMemcpyDeviceToHost, e->stream));
     CU(cudaStreamSynchronize(e->stream));
-    return e->check_numeric();
+    return e->check_status(true);
 }
 
 int pam_read_wavefield(pam_engine* e, int shot, float* out) {

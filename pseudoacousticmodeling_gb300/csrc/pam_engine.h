@@ -43,8 +43,12 @@ struct pam_engine {
     size_t rec_cap = 0;
     int nrec = 0, rec_per_shot = 0;
     float* d_seis_own = nullptr;
-    int* d_status = nullptr;             // bit 0: a non-finite seismogram sample was recorded
-    int check_numeric();                 // PAM_E_NUMERIC (with a message) if that bit is set
+    // [0]: bit 0, a non-finite seismogram sample was recorded (of a run); [1]: a
+    // block gave a barrier up (until it is reported)
+    int* d_status = nullptr;
+    // after the stream has been waited for: PAM_E_CUDA for the second, PAM_E_NUMERIC
+    // (numeric) for the first, with a message
+    int check_status(bool numeric);
     int seis_own_shots = 0, seis_own_nrec = 0;
     std::vector<float> wavelet;
     float* d_wavelet = nullptr;          // [nt], the persistent tiles' source samples
@@ -223,11 +227,7 @@ struct pam_engine {
     int tile_bset = 0;
     float* d_tile[2] = {nullptr, nullptr};   // [tile_shots][stride] the second published state of the tiles
     unsigned* d_tile_bar = nullptr;
-    // set by a block that gives a barrier up (a word of mapped host memory, so
-    // that calls see it without waiting for the device); cleared when reported
-    int *h_gave_up = nullptr, *d_gave_up = nullptr;
-    int tile_polls = 1 << 21;            // of a barrier before that (half a microsecond each)
-    int check_gave_up();
+    int tile_polls = 1 << 21;            // of a barrier before it is given up (half a microsecond each)
     std::vector<int> h_rz, h_rx;
     int tile_set = 0;                    // which published state is the current one
     int tile_held_shots = 0;             // shots whose last fields lie there (a forward run as tiles)

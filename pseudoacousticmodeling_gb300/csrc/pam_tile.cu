@@ -241,14 +241,6 @@ pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
     return it->second.usable ? &it->second : nullptr;
 }
 
-// PAM_E_CUDA (once) after a run whose blocks left a barrier without the others:
-// the run that has just completed, or an earlier one with device output.
-int pam_engine::check_gave_up() {
-    if (!h_gave_up || !*(volatile int*)h_gave_up) return PAM_OK;
-    *(volatile int*)h_gave_up = 0;
-    return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
-}
-
 // One array of the workspace: `fields` fields of every shot of it.
 bool pam_engine::tile_alloc(float** d, size_t fields, bool zero, cudaStream_t s) {
     if (*d) return true;
@@ -392,7 +384,6 @@ TileArgs pam_engine::tile_args(const TilePlan& p, int nshots) const {
     t.itlag = cfg.itlag;
     t.bar = d_tile_bar;
     t.polls = tile_polls;
-    t.gave_up = d_gave_up;
     t.status = d_status;
     t.mem_shots = tile_shots;
     return t;

@@ -73,8 +73,7 @@ struct TileArgs {
     int nt, itlag, k0, k1;
     unsigned* bar;                       // barrier counter, zero at the launch
     int polls;                           // of a barrier before it is given up
-    int* gave_up;                        // host memory: set to 1 when one was
-    int* status;                         // bit 0 set by a non-finite sample
+    int* status;                         // [0] bit 0 set by a non-finite sample, [1] by a barrier given up
     // every U(k) kept: U(k) at slots + (k - kslot) * slot_stride; the state before
     // step k0 is U(k0), U(k0 - 1) there, and so is what the tiles exchange
     // (nullptr: the two published sets)
@@ -106,7 +105,7 @@ __device__ __forceinline__ bool tile_barrier(const TileArgs& t, unsigned want, i
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.bar) : "memory");
         } while ((int)(v - want) < 0 && --left > 0);
         *flag = left > 0;
-        if (left <= 0) *(volatile int*)t.gave_up = 1;
+        if (left <= 0) t.status[1] = 1;
     }
     __syncthreads();
     return *flag != 0;
