@@ -94,10 +94,12 @@ int pam_set_receivers(pam_engine* e, int nrec, const int* rz, const int* rx, int
  * once (source cells sz[i], sx[i]).  seis receives [nshots][nt_data][nrec].
  * pam_forward takes host arrays and copies inside; pam_forward_device takes
  * device arrays (sz, sx, seis all on the device).  The loop runs as a CUDA
- * graph of one-step launches, or, for small Cerjan batches (up to about a
- * million cell updates per step) on a stream that is not being captured, as one
- * cooperative launch per time chunk whose blocks keep their tile of the grid on
- * chip and exchange halos every few steps; the seismograms are the same bit for bit. */
+ * graph of one-step launches, or, for small batches (up to about a million cell
+ * updates per step; with the matched layer acoustic and VTI ones) on a stream
+ * that is not being captured, as one cooperative launch per time chunk whose
+ * blocks keep their tile of the grid on chip and exchange halos every few steps;
+ * the seismograms are the same bit for bit (acoustic with the matched layer: as
+ * those of segment height 8, see pam_autotune). */
 int pam_forward(pam_engine* e, int nshots, const int* sz, const int* sx, float* seis, void* stream);
 int pam_forward_device(pam_engine* e, int nshots, const int* d_sz, const int* d_sx, float* d_seis,
                        void* stream);
@@ -288,9 +290,13 @@ int pam_misfit_noalloc(const float* d_dcal, const float* d_dobs, long long n, do
  * fixed 2-D blocks: cpp/Modeling.cu:448-449).  The first modelling, migration
  * or gradient call for a batch size times the stepping kernel with every
  * candidate segment height (the rows one warp marches: 8 ... 128) and keeps
- * the fastest; results do not depend on the choice.  pam_autotune(e, 0)
- * keeps the default height of 64 for batch sizes not yet tuned.
- * pam_segment_height returns the height chosen for `nshots`, 0 if none yet. */
+ * the fastest (small Cerjan batches that run with a barrier per step excepted).
+ * Results do not depend on the choice, except with the acoustic operator and
+ * the matched layer: there a segment clear of the border contracts the sum of
+ * the second derivatives into one operation, so the height moves the last bits.
+ * pam_autotune(e, 0) keeps the default height of 64 for batch sizes not yet
+ * tuned.  pam_segment_height returns the height chosen for `nshots`, 0 if none
+ * yet. */
 int pam_autotune(pam_engine* e, int enable);
 int pam_segment_height(const pam_engine* e, int nshots);
 

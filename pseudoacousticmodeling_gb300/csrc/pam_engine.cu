@@ -402,8 +402,11 @@ int pam_engine::seg_height(int nshots) const {
 // with events; the fastest is kept for this batch size.  Short segments give
 // more warps and shorter dependency chains (small batches), long ones less
 // halo re-reading (large batches).  The arithmetic per cell does not depend on
-// the height, so results are bitwise identical whatever is chosen.  The
-// buffers hold garbage afterwards: callers tune before resetting the fields.
+// the height, so results are bitwise identical whatever is chosen; except
+// acoustic CPML, where the march of the segments clear of the border contracts
+// the sum of the second derivatives into one operation, so that the height moves
+// the last bits.  The buffers hold garbage afterwards: callers tune before
+// resetting the fields.
 // Skipped (default height) while the stream is being captured into a graph.
 int pam_engine::tune_segments(int nshots, cudaStream_t s) {
     pam_engine* e = this;

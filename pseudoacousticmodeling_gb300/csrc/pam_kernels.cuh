@@ -117,9 +117,11 @@ __host__ __device__ constexpr int step_smem_bytes() {
 }
 
 // Packed two-wide FP32 arithmetic (sm_100+ FFMA2 / FADD2 / FMUL2), written
-// as inline PTX: every operation rounds exactly as written, whichever kernel
-// and code path it is inlined into, so that kernels evaluating the same
-// update (one step per launch, two steps per launch) agree bit for bit.
+// as inline PTX: the operations are those written, whichever kernel and code path
+// they are inlined into, so that kernels evaluating the same update agree bit for
+// bit.  (The assembler contracts a product and a sum that follow each other in
+// straight-line code into one operation; a branch between them, as around the
+// CPML strip terms, keeps them apart.)
 __device__ __forceinline__ unsigned long long f2bits(float2 v) { return *reinterpret_cast<unsigned long long*>(&v); }
 __device__ __forceinline__ float2 bits2f(unsigned long long b) { return *reinterpret_cast<float2*>(&b); }
 __device__ __forceinline__ float2 padd2(float2 a, float2 b) {
@@ -547,9 +549,10 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
 
     // The march down the segment: register window w[0..7] = rows r-4 .. r+3,
     // row r+4 arriving through the ring; U rows per trip, then the window
-    // shifts by U rows.  The rows past z1 in the last trip (at most U - 1;
-    // interior marches only, so no damping or strip reads) read only the ring,
-    // whose addresses are clamped to the field, and are not stored.
+    // shifts by U rows.  The rows past z1 in the last trip (at most U - 1) read
+    // the ring, whose addresses are clamped to the field, and, in the border
+    // march of TTI (one such row), the damping factor or strip terms of a row that
+    // still lies on the grid (z1 <= nz - 4); they are not stored.
     auto march = [&](auto edge_tag, auto unroll_tag) {
         constexpr int U = decltype(unroll_tag)::value;
         static_assert(U >= 1 && U <= 8, "rows per trip");
@@ -1008,9 +1011,10 @@ struct PersistArgs {
     int nt, itlag, k0, k1;
 };
 
-// (Segments of one to eight rows, a power of two: one border row and two or four
-// interior rows a trip, the four-slot ring and three TTI blocks a SM; with the ring and the four blocks of step_kernel four TTI
-// shots of 364 x 464 took 7.7 us a step instead of 6.9.)
+// (Segments of 1 to 64 rows, the shortest power of two whose blocks all fit at
+// once; one border row and two or four interior rows a trip, the four-slot ring
+// and three TTI blocks a SM: with the ring and the four blocks of step_kernel four
+// TTI shots of 364 x 464 took 7.7 us a step instead of 6.9.)
 template <int APPROX, int BC>
 __global__ void __launch_bounds__(128, APPROX == kTTI ? 3 : 4) step_persistent_kernel(const PersistArgs p)
 {

@@ -43,10 +43,14 @@ constexpr double kGraphStepUs[3] = {5.5, 6.6, 7.2}, kGraphCellUs[3] = {1.6e-6, 2
 
 // ... and of a step of the graph where the callers of three engines keep the GPU
 // busy together, which an asynchronous run (device output) allows and a
-// cooperative launch, taking every SM, does not (three engines in turn, measured:
+// cooperative launch, taking every SM, does not.  Every such run is weighed with
+// these figures, since the engine cannot know who else uses the GPU: one engine
+// that waits after each batch would do better as tiles (eight acoustic shots of
+// 301 x 501: 5.3 against 7.4 us a step by the figures above), as before there
+// were tiles.  (Three engines in turn, measured:
 // CPML of 0.18 / 0.36 / 0.53 million cells 3.7 / 4.1 / 4.6 us acoustic, 4.1 / 4.9 /
 // 5.6 us VTI, against 4.6 / 9.3 us and 5.3 us as tiles; Cerjan of 1.06 million
-// cells 3.0 us acoustic, 4.2 us VTI against 4.4 and 7.0).  Cerjan batches up to
+// cells 3.0 us acoustic, 4.2 us VTI against 4.4 and 7.0.)  Cerjan batches up to
 // kPersistCells are one cooperative launch either way.
 constexpr double kSharedStepUs[3] = {1.8, 2.1, 2.4}, kSharedCellUs[3] = {1.15e-6, 2.0e-6, 2.8e-6};
 constexpr double kCpmlSharedStepUs[2] = {3.3, 3.6}, kCpmlSharedCellUs[2] = {2.3e-6, 3.3e-6};

@@ -10,7 +10,8 @@
 // that the last one ends on the tile itself; then it publishes the tile's two
 // fields, waits for the other blocks and reads the halo back from L2.  The
 // halo cells are computed by several blocks, from the same values by the same
-// operations, so the results are those of the one-step kernels bit for bit.
+// operations, so the results are those of the one-step kernels bit for bit
+// (acoustic with the matched layer: of those with segments of eight rows).
 //
 // A thread owns one quad of columns and R rows of the tile with its halo:
 // U(t) and U(t-1) of those cells stay in its registers, and two copies of U in
