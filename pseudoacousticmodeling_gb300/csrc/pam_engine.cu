@@ -438,6 +438,7 @@ int pam_engine::tune_segments(int nshots, cudaStream_t s) {
             return fail(PAM_E_CUDA, "segment tuning failed: %s", cudaGetErrorString(err));
         }
         if (ms < best_ms) { best_ms = ms; best = h; }
+        if (ms > 1.5f * best_ms) break;          // (too few warps by now: taller ones are slower still)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
