@@ -249,14 +249,13 @@ pam_engine::TilePlan* pam_engine::tile_plan(int nshots, TileJob job) {
 bool pam_engine::tile_alloc(float** d, size_t fields, bool zero, cudaStream_t s) {
     if (*d) return true;
     const size_t bytes = fields * (size_t)tile_field() * 4;
-    tile_tight = true;
-    if (bytes > tile_limit || tile_bytes > tile_limit - bytes) return false;
-    if (cudaMalloc((void**)d, bytes) != cudaSuccess) {
-        cudaGetLastError();
+    const bool allowed = bytes <= tile_limit && tile_bytes <= tile_limit - bytes;
+    if (!allowed || cudaMalloc((void**)d, bytes) != cudaSuccess) {
+        if (allowed) cudaGetLastError();
         *d = nullptr;
+        tile_tight = true;   // until tile_reserve makes room
         return false;
     }
-    tile_tight = false;
     allocs.push_back(*d);
     tile_bytes += bytes;
     if (zero) cudaMemsetAsync(*d, 0, bytes, s);   // (its error is the caller's next one)

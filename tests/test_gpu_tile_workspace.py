@@ -122,3 +122,19 @@ def test_batches_that_grow_and_shrink(approx, abc):
         jobs(e, case, n, approx, abc)
     same(jobs(e, case, 1, approx, abc), ref[1])
     assert e.tile_workspace() <= 72 * e.field_bytes()
+
+
+def test_a_batch_that_has_not_fitted_keeps_no_smaller_one_out():
+    """Room for the segment's fields of one shot, not of three: three shots migrate
+    with the rest of the workspace, and one shot then gets its own."""
+    case = case_for()
+    e = engine_for(case)
+    e.set_random_boundary(400.0, 30.0, 3)
+    e.tile_workspace(limit_bytes=80 * e.field_bytes())
+    d = e.forward(case["sz"], case["sx"])
+    e.rtm(case["sz"], case["sx"], d, ckpt_interval=BOUNDARY_SAVING)
+    e.rtm(case["sz"], case["sx"], d, ckpt_interval=0)    # (fits: two arrays more for the receiver side)
+    assert e.tile_workspace() == 3 * 6 * e.field_bytes()
+    sz, sx = shots(case, 1)
+    e.rtm(sz, sx, d[:1], ckpt_interval=RANDOM_BOUNDARY)
+    assert e.tile_workspace() == 56 * e.field_bytes()
