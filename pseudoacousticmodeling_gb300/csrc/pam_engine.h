@@ -164,9 +164,9 @@ struct pam_engine {
     // nullptr for the one-step launches; tile_begin makes the buffers and lists
     // of a plan ready, tile_forward runs steps k0 .. k1-1 from the state that
     // the run's earlier launches left (before the first: d_u[0], d_u[1])
-    // the receivers by tile (or by thread of a tile) of a plan: `count` offsets and
-    // the entries they point into, in one buffer, uploaded in the order of the
-    // run's stream from a pinned copy; made again after set_receivers
+    // the receivers by tile (or by thread of a tile) of a plan: offsets and the
+    // entries they point into, in one buffer, uploaded in the order of the run's
+    // stream from a pinned copy; made again after set_receivers
     struct TileLists {
         bool ready = false, ok = true;   // ok: the plan can take these receivers
         size_t bytes = 0;                // of both buffers

@@ -308,8 +308,9 @@ bool pam_engine::tile_slots(cudaStream_t s) {
 }
 
 // The lists of a plan to the device, behind the work queued on s.  Buffers that
-// are large enough are used again: nothing here waits for the device, except to
-// make them larger.
+// are large enough are used again; what is waited for is the plan's last upload
+// (still queued only if the receivers changed twice meanwhile), and the device
+// where the buffers have to grow.
 bool pam_engine::tile_upload(TileLists& l, const std::vector<int>& beg, const std::vector<int2>& ent, cudaStream_t s) {
     l.entries = (beg.size() * sizeof(int) + 15) / 16 * 16;
     const size_t need = l.entries + ent.size() * sizeof(int2);
