@@ -480,6 +480,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &capturing));
     chain_launches = capturing == cudaStreamCaptureStatusNone;
+    wavelet_read = true;
     if (capturing == cudaStreamCaptureStatusNone) {
         if (cfg.boundary != PAM_CPML || nseg <= 1) ftiles = tile_plan(nshots, kTileForwardLaunched);
         if (sb || rbc) rtiles = tile_plan(nshots, kTileReverse);
@@ -697,7 +698,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
         CU(cudaStreamSynchronize(st));
         for (double v : part) mis += v;
         if (!std::isfinite(mis))
-            if (int rc = check_status(false)) return rc;   // samples left out
+            if (int rc = check_status(false, st)) return rc;   // samples left out
         if (!std::isfinite(mis))
             return fail(PAM_E_NUMERIC, "non-finite misfit: the modelled data overflowed (an unstable dt or grid for "
                                        "this model, see pam_check_stability) or the observed data hold NaN/Inf");
@@ -1008,8 +1009,7 @@ int pam_engine::run_adjoint_job(int mode, int nshots, const int* sz, const int* 
     }
     std::vector<float> g_vp(mode == kExact ? interior : 0);
     if (mode == kExact) CU(cudaMemcpyAsync(g_vp.data(), d_grad_b, interior * 4, cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    if (int rc = check_status(false)) return rc;   // (a non-finite sample shows in the misfit)
+    if (int rc = check_status(false, st)) return rc;   // (a non-finite sample shows in the misfit)
     for (size_t i = 0; i < g_vp.size(); i++) grad_vp[i] += g_vp[i];
     if (misfit) *misfit += mis;
     return PAM_OK;

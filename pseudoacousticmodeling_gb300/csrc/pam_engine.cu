@@ -581,13 +581,14 @@ void pam_engine::launch_record(int nshots, const float* cur, float* seis, int it
 
 // The recording sees a non-finite value when an unstable time step or grid for
 // the model overflows the fields, within a few dozen steps.
-int pam_engine::check_status(bool numeric) {
+int pam_engine::check_status(bool numeric, cudaStream_t s) {
     pam_engine* e = this;
     int v[2] = {0, 0};
-    CU(cudaMemcpy(v, d_status, sizeof(v), cudaMemcpyDeviceToHost));
+    CU(cudaMemcpyAsync(v, d_status, sizeof(v), cudaMemcpyDeviceToHost, s));
+    CU(cudaStreamSynchronize(s));
     if (v[1]) {
         // this run, or an earlier one with device output
-        CU(cudaMemset(d_status + 1, 0, sizeof(int)));
+        CU(cudaMemsetAsync(d_status + 1, 0, sizeof(int), s));
         return fail(PAM_E_CUDA, "a grid barrier of the persistent time loop was given up");
     }
     if (numeric && (v[0] & 1))
@@ -682,6 +683,7 @@ int pam_engine::run_forward(int nshots, float* d_seis, cudaStream_t s, float* h_
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &capturing));
     chain_launches = capturing == cudaStreamCaptureStatusNone;
+    wavelet_read = true;
     // (a run into the caller's device buffer returns at once: others may share the GPU)
     const TileJob job = d_seis == d_seis_own ? kTileForward : kTileForwardAsync;
     TilePlan* tiles = use_graph && capturing == cudaStreamCaptureStatusNone ? tile_plan(nshots, job) : nullptr;
@@ -1014,8 +1016,9 @@ int pam_set_wavelet(pam_engine* e, const float* w) {
     if (!w) return e->fail(PAM_E_ARG, "wavelet is NULL");
     CU(cudaSetDevice(e->device));
     // the persistent loops read the samples from the device at every step, and
-    // the engine's streams are non-blocking: wait for work that may read them
-    CU(cudaDeviceSynchronize());
+    // the engine's streams are non-blocking: wait for runs that may read them
+    if (e->wavelet_read) CU(cudaDeviceSynchronize());
+    e->wavelet_read = false;
     e->wavelet.assign(w, w + e->cfg.nt);
     CU(cudaMemcpy(e->d_wavelet, w, (size_t)e->cfg.nt * sizeof(float), cudaMemcpyHostToDevice));
     e->invalidate_graph();
@@ -1076,8 +1079,7 @@ int pam_forward(pam_engine* e, int nshots, const int* sz, const int* sx, float* 
         const size_t bytes = (size_t)nshots * e->nt_data * e->nrec * sizeof(float);
         CU(cudaMemcpyAsync(seis, e->d_seis_own, bytes, cudaMemcpyDeviceToHost, s));
     }
-    CU(cudaStreamSynchronize(s));
-    return e->check_status(true);
+    return e->check_status(true, s);
 }
 
 int pam_begin(pam_engine* e, int nshots, const int* sz, const int* sx) {
@@ -1116,8 +1118,7 @@ int pam_read_seismograms(pam_engine* e, float* out) {
     if (e->step_shots < 1 || !out) return e->fail(PAM_E_STATE, "no shots in flight");
     CU(cudaMemcpyAsync(out, e->d_seis_own, (size_t)e->step_shots * e->nt_data * e->nrec * sizeof(float),
                        cudaMemcpyDeviceToHost, e->stream));
-    CU(cudaStreamSynchronize(e->stream));
-    return e->check_status(true);
+    return e->check_status(true, e->stream);
 }
 
 int pam_read_wavefield(pam_engine* e, int shot, float* out) {

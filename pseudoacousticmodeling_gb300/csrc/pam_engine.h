@@ -46,12 +46,13 @@ struct pam_engine {
     // [0]: bit 0, a non-finite seismogram sample was recorded (of a run); [1]: a
     // block gave a barrier up (until it is reported)
     int* d_status = nullptr;
-    // after the stream has been waited for: PAM_E_CUDA for the second, PAM_E_NUMERIC
-    // (numeric) for the first, with a message
-    int check_status(bool numeric);
+    // waits for s; PAM_E_CUDA for the second, PAM_E_NUMERIC (numeric) for the
+    // first, with a message
+    int check_status(bool numeric, cudaStream_t s);
     int seis_own_shots = 0, seis_own_nrec = 0;
     std::vector<float> wavelet;
-    float* d_wavelet = nullptr;          // [nt], the persistent tiles' source samples
+    float* d_wavelet = nullptr;          // [nt], the persistent loops' source samples
+    bool wavelet_read = false;           // by a run since they were last set
 
     // step-level interface
     int step_shots = 0, next_step = 0;
